@@ -3,8 +3,8 @@
 // The code adjustment is a sequential coordinate descent in FP64 whose every
 // accepted move changes the running <o,o_a> and |o_a|^2 read by the next
 // dimension (caq_encoder.hpp:57-142); bit-exact codes need the reference's
-// exact FP64 operation sequence, so one thread owns one vector and walks its
-// dimensions in order.  In index construction the 32 lanes of a warp encode
+// exact FP64 sums, so one thread owns one vector and walks its dimensions in
+// order (caq_encode_one).  In index construction the 32 lanes of a warp encode
 // 32 vectors whose residuals and codes are interleaved by dimension, so every
 // step of the 32 chains is one coalesced access.  This file is compiled with
 // --fmad=false: no multiply is fused into an add unless written as fma().
@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <type_traits>
 #include <vector>
 
 #include "device_common.cuh"
@@ -58,40 +59,210 @@ __device__ float thread_eigen_sum(int n, F f) {
     return r;
 }
 
+// x as a double.  Normal floats take integer operations (widening the exponent,
+// shifting the mantissa): FP64 and its conversions run at 1/64 of the FP32 rate here.
+__device__ __forceinline__ double widen(float x) {
+    const uint32_t u = __float_as_uint(x);
+    if ((u & 0x7f800000u) - 0x00800000u >= 0x7f000000u) return (double)x;  // zero, denormal, inf, NaN
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+}
+
+// A double of magnitude in [2^-120, 2^120] truncated to float (within 2^-23 of it).
+__device__ __forceinline__ float narrow(double x) {
+    const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+    return __uint_as_float((hi & 0x80000000u) | (__funnelshift_l(lo, hi - 0x38000000u, 3) & 0x7fffffffu));
+}
+__device__ __forceinline__ bool in_range(double x, double lo, double hi) { return x >= lo && x <= hi; }
+
+__device__ __forceinline__ float rcp_approx(float x) {  // within 2^-23 of 1 / x
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// FP32 view of the adjustment's state (ip = <o, o_a>, oa2 = |o_a|^2).  A code's
+// value is oa = delta (m + 1/2) exactly, m = code - 2^(bits-1), so a move by one
+// code step is accepted (caq_encoder.hpp:93, 108) exactly when
+//   up:   g = a (a + 2) - Q (m + 1) - rho > 0
+//   down: g = a (a - 2) + Q m - rho > 0
+// with a = delta o_j / ip, Q = (1 + rho) 2 delta^2 / oa2, rho = re_eps / ip^2: both
+// sides of the reference's comparison divided by ip^2 oa2, their common part
+// taken off.  In FP32 g is within `margin` of its value: the factors are within
+// 2^-21.3 of theirs (truncation, reciprocal, up to three roundings), the sums add
+// three roundings, and 2^-19 (4 |a|max + Q (2^(bits-1) + 1) + |rho|) is over three
+// times that for |a| <= 2 (beyond, the margin is infinite); 1e-12 (1 + |rho|)
+// covers the rounding of the reference's own FP64 sides.  So a g outside the
+// margin has the FP64 comparison's outcome; within it (about one test in 10^5)
+// the FP64 comparison itself runs.
+//
+// init decides once whether the vector stays in float range: each |oa| lies in
+// [delta / 2, v_mx], which bounds oa2; an accepted move never lowers ip^2 / oa2,
+// so |ip| never falls below 2^-bits of its first value and stays below |o| |oa|.
+// Otherwise (or with a NaN) every test runs in FP64 (k* infinite or NaN).
+struct AdjView {
+    float A2, Q, rho, margin;
+    float df2, q1, ref, kv, kh;
+    __device__ __forceinline__ void init(double ip, double oa2, double re_eps, double v_mx, double delta, double l2max,
+                                         float half) {
+        const bool ok = in_range(fabs(ip), 0x1p-80, 0x1p80) && in_range(oa2, 0x1p-100, 0x1p100) &&
+                        in_range(v_mx, 0x1p-40, 0x1p40) && in_range(delta, 0x1p-44, 0x1p40) && l2max < 0x1p100 &&
+                        (re_eps == 0 || in_range(re_eps, 0x1p-100, 0x1p100));
+        const float vm = (float)v_mx, df = (float)delta;
+        df2 = 2.0f * df;
+        q1 = df2 * df;
+        ref = ok ? (float)re_eps : 0.0f;
+        kv = ok ? 3.8146973e-6f * vm : __int_as_float(0x7f800000);  // 2^-19 * 2 v_mx, on |A2| = 2 |A|
+        kh = 1.9073486e-6f * (half + 1.0f);
+        set(ip, oa2);
+    }
+    __device__ __forceinline__ void set(double ip, double oa2) {
+        const float ri = rcp_approx(narrow(ip)), ro = rcp_approx(narrow(oa2));
+        A2 = df2 * ri;
+        rho = ref * ri * ri;
+        Q = fmaf(rho, q1, q1) * ro;
+        const float am = fabsf(A2) * kv;  // 2^-19 * 4 |a|max
+        margin = am + fmaf(fabsf(Q), kh, fmaf(fabsf(rho), 1.9073496e-6f, 1e-12f));
+        if (!(am <= 1.5258789e-5f)) margin = __int_as_float(0x7f800000);  // |a|max > 2
+    }
+    // g of either direction, -inf where the code is at its end (top = 2^(bits-1) - 1)
+    __device__ __forceinline__ void test(float ov, float m, float top, float &gu, float &gd) const {
+        const float a2 = A2 * ov, a = 0.5f * a2, p = fmaf(a, a, -rho), w = fmaf(-Q, m, a2);
+        gu = m < top ? (p + w) - Q : __int_as_float(0xff800000);
+        gd = m > -top - 1.0f ? p - w : __int_as_float(0xff800000);
+    }
+    __device__ __forceinline__ float best(float ov, float m, float top) const {
+        float gu, gd;
+        test(ov, m, top, gu, gd);
+        return fmaxf(gu, gd);
+    }
+};
+
+// The reference's comparison (caq_encoder.hpp:93, 108): whether the move to
+// (ni, nl) is refused.  A call, so that its FP64 operations are not issued under a
+// false predicate on every visit.
+__device__ __noinline__ bool refused(double ip, double oa2, double re_eps, double ni, double nl) {
+    return __dmul_rn(__dadd_rn(__dmul_rn(ip, ip), re_eps), nl) >= __dmul_rn(__dmul_rn(ni, ni), oa2);
+}
+
+constexpr int kEncTableBits = 6;  // codes of at most this many bits keep their values in shared memory
+constexpr int kEncWin = 8;       // dimensions a warp visits together
+constexpr int kEncThreads = 32;  // one warp a CTA: the last wave fills evenly
+constexpr int kEncCtas = 21;     // resident CTAs per SM the register budget is sized for
+
+// Bytes of shared memory per warp: (oa, oa^2) of the codes above the middle (the
+// lower half mirrors them), one column per lane.
+__host__ __device__ constexpr size_t enc_table_bytes(int bits) {
+    return bits >= 1 && bits <= kEncTableBits ? (size_t)(1 << (bits - 1)) * 2 * 32 * 8 : 0;
+}
+
+// kN (4 or 8) consecutive dimensions of a vector, or of its codes.  STR = 1: a
+// row-major vector (16-byte accesses when `vec`); 32: a vector of a
+// warp-interleaved group.
+template <int STR, int kN>
+__device__ __forceinline__ void load_dims(const float *__restrict__ p, bool vec, float (&x)[kN]) {
+    if (STR == 1 && vec) {
+#pragma unroll
+        for (int k = 0; k < kN; k += 4) {
+            const float4 a = *reinterpret_cast<const float4 *>(p + k);
+            x[k] = a.x, x[k + 1] = a.y, x[k + 2] = a.z, x[k + 3] = a.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < kN; ++k) x[k] = p[k * STR];
+    }
+}
+template <int STR, int kN, class CodeT>
+__device__ __forceinline__ void load_codes(const CodeT *p, bool vec, int (&x)[kN]) {
+    if (STR == 1 && sizeof(CodeT) == 4 && vec) {
+#pragma unroll
+        for (int k = 0; k < kN; k += 4) {
+            const int4 a = *reinterpret_cast<const int4 *>(p + k);
+            x[k] = a.x, x[k + 1] = a.y, x[k + 2] = a.z, x[k + 3] = a.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < kN; ++k) x[k] = (int)p[k * STR];
+    }
+}
+
 // encode + code_adjustment + encode_and_fac (caq_encoder.hpp:57-247) for one
-// vector whose dimension j lies at o_[j * STR] (its code at code_[j * STR]):
-// STR = 1 for a row-major vector, 32 for a vector of a warp-interleaved group,
-// where the 32 lanes of a warp encode 32 vectors and every load and store of
-// the warp at dimension j is one contiguous 128-byte access.
-template <int STR>
+// vector of D dimensions (a multiple of 32), dimension j at o_[j * STR] (its code
+// at code_[j * STR]): STR = 1 for a row-major vector, 32 for a vector of a
+// warp-interleaved group, where the 32 lanes of a warp encode 32 vectors and
+// every load and store of the warp at dimension j is one contiguous line.
+//
+// The FP64 pipe bounds it (two lanes per SM and cycle).  With the adjustment as
+// the reference writes it, about 190 FP64 operations per dimension, 100,000 x 960
+// at 4 bits took 54 ms and 8,191 x 960 9.8 ms; now 5.6 and 1.7 ms, the FP64 pipe
+// active 70% of the time with about 23 operations per dimension.  What stays FP64
+// is what the codes and factors are made of, the running sums of accepted moves
+// and the correction sums:
+//   * the comparisons run in FP32 with a bound (AdjView): 54 to 12 ms;
+//   * the code values and their squares come from a table;
+//   * products that are exact in FP64 (24-bit operands: delta o_j, and oa o_j up to
+//     5 bits) are fused into their sums, which rounds the same;
+//   * the correction sums of a round accumulate while the round runs, since a
+//     dimension's code is final once its window is done;
+//   * a warp visits a window of kEncWin dimensions together, each lane at its own
+//     next move, so one pass of the FP64 operations serves every lane that still has
+//     a move: 3-4 passes per window instead of one or more per dimension (7.7 to
+//     5.6 ms).
+// Every sum rounds at the same places as the reference's.  kWidth: 0 up to 5 bits
+// (table, fused products), 1 for 6 (table), 2 for more.
+template <int STR, int kWidth, class CodeT>
 __device__ void caq_encode_one(const float *__restrict__ o_, int D, int bits, const float *__restrict__ cent, int rdlmt,
-                               float eps, int32_t *__restrict__ code_, float *__restrict__ fac) {
-    auto o = [&](int j) { return o_[(int64_t)j * STR]; };
-    auto code = [&](int j) -> int32_t & { return code_[(int64_t)j * STR]; };
+                               float eps, CodeT *code_, float *__restrict__ fac, bool vec, float *win, double *tab) {
+    auto code = [&](int j) -> CodeT & { return code_[(int64_t)j * STR]; };
+    // Eigen's 16-lane two-accumulator sum (thread_eigen_sum), four dimensions per load
+    auto eigen_sum = [&](auto f) {
+        float r[32];
+#pragma unroll
+        for (int l = 0; l < 32; ++l) r[l] = 0.0f;
+        for (int j = 0; j < D; j += 32)
+#pragma unroll
+            for (int h = 0; h < 32; h += 4) {
+                float x[4];
+                load_dims<STR>(o_ + (int64_t)(j + h) * STR, vec, x);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float t = f(j + h + k, x[k]);
+                    r[h + k] = j == 0 ? t : __fadd_rn(r[h + k], t);
+                }
+            }
+#pragma unroll
+        for (int l = 0; l < 16; ++l) r[l] = __fadd_rn(r[l], r[16 + l]);
+        return tree16(r);
+    };
     double v_mx = 0, v_mi = 0, delta = 0, ip = 0, oa2 = 0;
     if (bits > 0) {
         const int cmax = (1 << bits) - 1;
-        float mx = o(0), mn = o(0);
-        for (int j = 1; j < D; ++j) {
-            mx = fmaxf(mx, o(j));
-            mn = fminf(mn, o(j));
-        }
-        v_mx = (double)fmaxf(mx, -mn);
+        float mx = o_[0], mn = o_[0];
+        const double vec_sum = (double)eigen_sum([&](int, float x) {
+            mx = fmaxf(mx, x);
+            mn = fminf(mn, x);
+            return x;
+        });
+        const float vmx_f = fmaxf(mx, -mn);
+        v_mx = (double)vmx_f;
         v_mi = -v_mx;
         delta = __ddiv_rn(__dsub_rn(v_mx, v_mi), (double)(cmax + 1));
-        const double vec_sum = (double)thread_eigen_sum(D, [&](int i) { return o(i); });
         double ip_o_code = 0;
         uint64_t code_l2 = 0;
         uint32_t code_sum = 0;
         const float vmi_f = (float)v_mi, d_f = (float)delta;
-        for (int j = 0; j < D; ++j) {
-            float cf = 0.0f;
-            if (delta != 0) cf = fminf(floorf(__fdiv_rn(__fsub_rn(o(j), vmi_f), d_f)), (float)cmax);
-            ip_o_code = __dadd_rn(ip_o_code, (double)__fmul_rn(cf, o(j)));
-            const int c = (int)cf;
-            code(j) = c;
-            code_l2 += (uint64_t)(c * c);
-            code_sum += (uint32_t)c;
+        for (int j = 0; j < D; j += 4) {
+            float x[4];
+            load_dims<STR>(o_ + (int64_t)j * STR, vec, x);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                float cf = 0.0f;
+                if (delta != 0) cf = fminf(floorf(__fdiv_rn(__fsub_rn(x[k], vmi_f), d_f)), (float)cmax);
+                ip_o_code = __dadd_rn(ip_o_code, widen(__fmul_rn(cf, x[k])));
+                const int c = (int)cf;
+                code(j + k) = (CodeT)c;
+                code_l2 += (uint64_t)(c * c);
+                code_sum += (uint32_t)c;
+            }
         }
         ip = __dadd_rn(__dmul_rn(ip_o_code, delta), __dmul_rn(__dadd_rn(v_mi, __dmul_rn(0.5, delta)), vec_sum));
         const double dd = __dmul_rn(delta, delta);
@@ -102,55 +273,127 @@ __device__ void caq_encode_one(const float *__restrict__ o_, int D, int bits, co
         oa2 = __dadd_rn(oa2, __dmul_rn(k3, (double)D));
         if (rdlmt && oa2 != 0) {
             const double re_eps = __dmul_rn((double)eps, oa2);
+            const int half = 1 << (bits - 1);
+            const float bias = 8388608.0f + (float)half;
+            constexpr bool table = kWidth <= 1;
+            // m and its float: code - 2^(bits-1), by the mantissa of 2^23 + code
+            auto m_float = [&](int c) { return __int_as_float(0x4b000000 | c) - bias; };
+            auto m_int = [](float mf) { return __float_as_int(mf + 12582912.0f) - 0x4b400000; };
+            const float top = (float)(half - 1);
+            // oa and oa^2 of code half + m; entry i of the table holds those of m = i
+            // and, negated, of m = -i - 1
+            auto value = [&](int m, double &oa, double &sq) {
+                if (table) {
+                    const double2 t = *reinterpret_cast<const double2 *>(tab + (m ^ (m >> 31)) * 64);
+                    oa = __hiloint2double(__double2hiint(t.x) ^ (m & 0x80000000), __double2loint(t.x));
+                    sq = t.y;
+                } else {
+                    oa = __dadd_rn(__dmul_rn(widen((float)(m + half) + 0.5f), delta), v_mi);
+                    sq = __dmul_rn(oa, oa);
+                }
+            };
+            if (table)
+                for (int i = 0; i < half; ++i) {
+                    const double t = __dadd_rn(__dmul_rn((double)(half + i) + 0.5, delta), v_mi);
+                    *reinterpret_cast<double2 *>(tab + i * 64) = make_double2(t, __dmul_rn(t, t));
+                }
+            AdjView st;
+            st.init(ip, oa2, re_eps, v_mx, delta, (double)vmx_f * vmx_f * D, (float)half);
             for (int adj = 1, round = 1; adj; round++) {
                 adj = 0;
-                for (int j = 0; j < D; ++j) {
-                    int cur = 0;
-                    const float ov = o(j);
-                    double oa = __dadd_rn(__dmul_rn(__dadd_rn((double)code(j), 0.5), delta), v_mi);
-                    int c = code(j);
-                    const double tmp = __dsub_rn(oa2, __dmul_rn(oa, oa));
-                    const double ipd = __dmul_rn(delta, (double)ov);
-                    while (c < cmax) {
-                        const double nq = __dadd_rn(oa, delta), nl = __dadd_rn(tmp, __dmul_rn(nq, nq)),
-                                     ni = __dadd_rn(ip, ipd);
-                        if (__dmul_rn(__dadd_rn(__dmul_rn(ip, ip), re_eps), nl) >= __dmul_rn(__dmul_rn(ni, ni), oa2)) break;
-                        c++;
-                        ip = ni;
-                        oa = nq;
-                        oa2 = nl;
-                        cur++;
-                    }
-                    while (c > 0) {
-                        const double nq = __dsub_rn(oa, delta), nl = __dadd_rn(tmp, __dmul_rn(nq, nq)),
-                                     ni = __dsub_rn(ip, ipd);
-                        if (__dmul_rn(__dadd_rn(__dmul_rn(ip, ip), re_eps), nl) >= __dmul_rn(__dmul_rn(ni, ni), oa2)) break;
-                        c--;
-                        ip = ni;
-                        oa = nq;
-                        oa2 = nl;
-                        cur++;
-                    }
-                    if (code(j) != c) {
-                        code(j) = c;
-                        adj += cur;
-                    }
-                }
-                if (rdlmt && round >= rdlmt) break;
+                const bool last = round >= rdlmt;  // the reference leaves before this round's correction
                 double ci = 0, co = 0;
-                for (int j = 0; j < D; ++j) {
-                    const double qv = __dadd_rn(__dmul_rn(__dadd_rn((double)code(j), 0.5), delta), v_mi);
-                    ci = __dadd_rn(ci, __dmul_rn(qv, (double)o(j)));
-                    co = __dadd_rn(co, __dmul_rn(qv, qv));
+                float xn[kEncWin];
+                int cn[kEncWin];
+                load_dims<STR>(o_, vec, xn);
+                load_codes<STR>(code_, vec, cn);
+#pragma unroll 1
+                for (int j0 = 0; j0 < D; j0 += kEncWin) {
+                    float x[kEncWin];
+                    int c0[kEncWin];
+#pragma unroll
+                    for (int k = 0; k < kEncWin; ++k) {
+                        x[k] = xn[k];
+                        c0[k] = cn[k];
+                        win[k * 64] = x[k];
+                        win[k * 64 + 32] = m_float(c0[k]);
+                    }
+                    if (j0 + kEncWin < D) {  // the next window, in flight while this one is visited
+                        load_dims<STR>(o_ + (int64_t)(j0 + kEncWin) * STR, vec, xn);
+                        load_codes<STR>(code_ + (int64_t)(j0 + kEncWin) * STR, vec, cn);
+                    }
+                    // one code step of one dimension per trip: each lane takes its own next
+                    // dimension whose move is not surely refused, so the FP64 operations of a
+                    // trip serve every lane that still has one
+                    int k0 = 0, tj = -1;
+                    double tmp = 0;  // of dimension tj: oa2 less its oa^2, fixed while its steps last
+                    for (;;) {
+                        uint32_t cand = 0;
+#pragma unroll
+                        for (int k = 0; k < kEncWin; ++k) cand |= (uint32_t)(!(st.best(x[k], win[k * 64 + 32], top) < -st.margin)) << k;
+                        cand &= ~0u << k0;
+                        if (!cand) break;
+                        const int j = __ffs(cand) - 1;
+                        const float ov = win[j * 64], mf = win[j * 64 + 32];
+                        float gu, gd;
+                        st.test(ov, mf, top, gu, gd);
+                        int m = m_int(mf);
+                        const double od = widen(ov);
+                        double oa, sq, sqn;
+                        value(m, oa, sq);
+                        if (j != tj) tmp = __dsub_rn(oa2, sq);
+                        tj = j;
+                        const bool up = gu > st.margin;
+                        if (up || (gu < -st.margin && gd > st.margin)) {  // surely accepted; tested again next trip
+                            value(up ? m + 1 : m - 1, oa, sqn);
+                            ip = fma(up ? delta : -delta, od, ip);
+                            oa2 = __dadd_rn(tmp, sqn);
+                            win[j * 64 + 32] = up ? mf + 1.0f : mf - 1.0f;
+                            st.set(ip, oa2);
+                            k0 = j;
+                            continue;
+                        }
+                        // the reference's loops as written: upward steps until one is refused, then downward
+                        for (int d = 1; d >= -1; d -= 2)
+                            while (d > 0 ? m < half - 1 : m > -half) {
+                                value(m + d, oa, sqn);
+                                const double nl = __dadd_rn(tmp, sqn), ni = fma(d > 0 ? delta : -delta, od, ip);
+                                if (refused(ip, oa2, re_eps, ni, nl)) break;
+                                m += d;
+                                ip = ni;
+                                oa2 = nl;
+                            }
+                        win[j * 64 + 32] = (float)m;
+                        st.set(ip, oa2);
+                        k0 = j + 1;
+                    }
+#pragma unroll
+                    for (int k = 0; k < kEncWin; ++k) {
+                        const float mf = win[k * 64 + 32];
+                        const int m = m_int(mf);
+                        if (m + half != c0[k]) {
+                            code(j0 + k) = (CodeT)(m + half);
+                            adj = 1;
+                        }
+                        if (!last) {  // the correction sums over the round's final codes
+                            double oa, sq;
+                            value(m, oa, sq);
+                            const double od = widen(x[k]);
+                            ci = kWidth == 0 ? fma(oa, od, ci) : __dadd_rn(ci, __dmul_rn(oa, od));
+                            co = __dadd_rn(co, sq);
+                        }
+                    }
                 }
+                if (last) break;
                 oa2 = co;
                 ip = ci;
+                st.set(ip, oa2);
             }
         }
     } else {
         for (int j = 0; j < D; ++j) code(j) = 0;
     }
-    const double o_l2sqr = (double)thread_eigen_sum(D, [&](int i) { return __fmul_rn(o(i), o(i)); });
+    const double o_l2sqr = (double)eigen_sum([&](int, float x) { return __fmul_rn(x, x); });
     const double o_l2norm = __dsqrt_rn(o_l2sqr);
     double rescale = ip != 0 ? __ddiv_rn(o_l2sqr, ip) : 0.0;
     const double err = __dmul_rn(
@@ -165,7 +408,8 @@ __device__ void caq_encode_one(const float *__restrict__ o_, int D, int bits, co
     float ipc = 0.0f;
     if (bits > 1 && cent) {
         const float df = (float)delta, vf = (float)v_mi;
-        ipc = thread_eigen_sum(D, [&](int i) { return __fmul_rn(cent[i], __fadd_rn(__fmul_rn((float)code(i), df), vf)); });
+        ipc = thread_eigen_sum(
+            D, [&](int i) { return __fmul_rn(cent[i], __fadd_rn(__fmul_rn((float)(int)code(i), df), vf)); });
     }
     fac[0] = (float)o_l2norm;
     fac[1] = ipc;
@@ -173,11 +417,36 @@ __device__ void caq_encode_one(const float *__restrict__ o_, int D, int bits, co
     fac[3] = (float)err;
 }
 
-__global__ void k_caq_encode(const float *__restrict__ resid, int64_t n, int D, int bits, const float *__restrict__ cent,
-                             int rdlmt, float eps, int32_t *__restrict__ codes, float *__restrict__ facs) {
+// Shared memory of an encoding warp: its window (kEncWin dimensions and their
+// codes), then its table.
+__device__ __forceinline__ float *enc_window() {
+    extern __shared__ __align__(16) double enc_smem[];
+    return reinterpret_cast<float *>(enc_smem) + (threadIdx.x & 31);
+}
+__device__ __forceinline__ double *enc_table() {
+    extern __shared__ __align__(16) double enc_smem[];
+    return enc_smem + kEncWin * 32 + 2 * (threadIdx.x & 31);
+}
+
+template <int kWidth>
+__global__ void __launch_bounds__(kEncThreads, kEncCtas) k_caq_encode(const float *__restrict__ resid, int64_t n, int D, int bits,
+                                                            const float *__restrict__ cent, int rdlmt, float eps,
+                                                            int32_t *codes, float *__restrict__ facs, int vec) {
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= n) return;
-    caq_encode_one<1>(resid + v * D, D, bits, cent, rdlmt, eps, codes + v * D, facs + v * 4);
+    caq_encode_one<1, kWidth>(resid + v * D, D, bits, cent, rdlmt, eps, codes + v * D, facs + v * 4, vec != 0,
+                              enc_window(), enc_table());
+}
+
+// Shared memory of a CTA (one warp; at most 18 KB).
+size_t enc_smem_bytes(int bits) { return kEncWin * 32 * 8 + enc_table_bytes(bits); }
+
+// Calls f with the kernel's kWidth for codes of `bits` bits.
+template <class F>
+void by_width(int bits, F f) {
+    if (bits <= 5) f(std::integral_constant<int, 0>());
+    else if (bits <= kEncTableBits) f(std::integral_constant<int, 1>());
+    else f(std::integral_constant<int, 2>());
 }
 
 }  // namespace
@@ -203,8 +472,13 @@ void run_caq_encode(const float *resid, int64_t n, int64_t dim, int bits, const 
         dcodes = (int32_t *)(p + br + bc);
         dfacs = (float *)(p + br + bc + bo);
     }
-    const int tpb = 64;
-    k_caq_encode<<<(unsigned)((n + tpb - 1) / tpb), tpb, 0, st>>>(dr, n, (int)dim, bits, dc, rdlmt, eps, dcodes, dfacs);
+    // rows of a multiple of 32 floats: 16-byte accesses need only aligned bases
+    const int vec = ((uintptr_t)dr & 15) == 0 && ((uintptr_t)dcodes & 15) == 0;
+    by_width(bits, [&](auto w) {
+        k_caq_encode<decltype(w)::value>
+            <<<(unsigned)((n + kEncThreads - 1) / kEncThreads), kEncThreads, enc_smem_bytes(bits), st>>>(
+                dr, n, (int)dim, bits, dc, rdlmt, eps, dcodes, dfacs, vec);
+    });
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         if (buf) cudaFree(buf);
@@ -334,19 +608,22 @@ __global__ void k_centroid_slices(const float *__restrict__ cent, int64_t K, int
 // step of the 32 sequential FP64 chains reads one coalesced line.
 __device__ __forceinline__ int64_t inter_at(int64_t v, int D) { return (v >> 5) * (int64_t)D * 32 + (v & 31); }
 
-__global__ void k_caq_encode_clustered(const float *__restrict__ resid, int64_t n, int D, int bits,
-                                       const float *__restrict__ cslices, const int32_t *__restrict__ cid, int rdlmt,
-                                       float eps, int32_t *__restrict__ codes, float *__restrict__ facs) {
+template <int kWidth>
+__global__ void __launch_bounds__(kEncThreads, kEncCtas) k_caq_encode_clustered(const float *__restrict__ resid, int64_t n, int D,
+                                                                      int bits, const float *__restrict__ cslices,
+                                                                      const int32_t *__restrict__ cid, int rdlmt,
+                                                                      float eps, uint16_t *codes,
+                                                                      float *__restrict__ facs) {
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= n) return;
-    caq_encode_one<32>(resid + inter_at(v, D), D, bits, cslices + (int64_t)cid[v] * D, rdlmt, eps,
-                       codes + inter_at(v, D), facs + v * 4);
+    caq_encode_one<32, kWidth>(resid + inter_at(v, D), D, bits, cslices + (int64_t)cid[v] * D, rdlmt, eps,
+                       codes + inter_at(v, D), facs + v * 4, false, enc_window(), enc_table());
 }
 
 // CodeHelper<B>::compacted_code8/16 (code_helper.hpp) for one vector (code of
 // dimension d at v[d * STR]).
 template <int STR>
-__device__ void pack_bits8_dev(const int32_t *__restrict__ v, int D, int bits, int shift, int mask,
+__device__ void pack_bits8_dev(const uint16_t *__restrict__ v, int D, int bits, int shift, int mask,
                                uint8_t *__restrict__ y) {
     auto val = [&](int d) { return (uint32_t)((v[(int64_t)d * STR] >> shift) & mask); };
     switch (bits) {
@@ -405,7 +682,7 @@ __device__ void pack_bits8_dev(const int32_t *__restrict__ v, int D, int bits, i
 }
 
 template <int STR>
-__device__ void pack_excode_dev(const int32_t *__restrict__ code, int D, int exb, uint8_t *__restrict__ y) {
+__device__ void pack_excode_dev(const uint16_t *__restrict__ code, int D, int exb, uint8_t *__restrict__ y) {
     const int lowmask = (1 << exb) - 1;
     if (exb > 8) {  // compacted_code16: low bytes, then the remaining bits in their own layout
         for (int d = 0; d < D; ++d) y[d] = (uint8_t)(code[(int64_t)d * STR] & lowmask & 0xFF);
@@ -426,7 +703,7 @@ __device__ void pack_excode_dev(const int32_t *__restrict__ code, int D, int exb
 
 // ClusterPacker::store_and_pack + finalize_and_store (cluster_packer.hpp:59-116)
 // into the device layout (saqg_internal.h): one thread per vector.
-__global__ void k_pack(const int32_t *__restrict__ codes, const float *__restrict__ facs, int64_t n, int64_t vbase,
+__global__ void k_pack(const uint16_t *__restrict__ codes, const float *__restrict__ facs, int64_t n, int64_t vbase,
                        const int32_t *__restrict__ cid, const int64_t *__restrict__ blk_off,
                        const int64_t *__restrict__ vec_off, SegDev g) {
     const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -441,7 +718,7 @@ __global__ void k_pack(const int32_t *__restrict__ codes, const float *__restric
     if (g.bits == 0) return;
     g.ipcent[gb * 32 + lane] = f[1];
     g.exfac[gv] = make_float2(f[2], f[3]);
-    const int32_t *code = codes + inter_at(v, g.dim);  // warp-interleaved codes: dimension d at code[32 d]
+    const uint16_t *code = codes + inter_at(v, g.dim);  // warp-interleaved codes: dimension d at code[32 d]
     const int sb = 1 << (g.bits - 1);
     uint8_t *cb = reinterpret_cast<uint8_t *>(g.codes) + (size_t)gb * (g.dim / 8) * 32;
     for (int i = 0; i < g.dim / 8; ++i) {
@@ -493,6 +770,13 @@ void launch_check(const char *what) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) throw Error{SAQG_ERR_CUDA, std::string(what) + " launch failed: " + cudaGetErrorString(e)};
     count_launch(1);
+}
+
+int encoder_sms() {
+    int dev = 0, sms = 0;
+    SAQG_CUDA_TRY(cudaGetDevice(&dev));
+    SAQG_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    return std::max(1, sms);
 }
 
 struct DevBuf {
@@ -639,10 +923,15 @@ Index *construct_index(const float *data, int64_t n, int64_t dim, const float *c
     }
     int64_t maxd = 0;
     for (auto &sg : X.segs) maxd = std::max(maxd, sg.dim);
-    // chunks of whole 32-vector groups (residuals and codes are warp-interleaved)
-    const int64_t chunk = std::max<int64_t>(32, std::min<int64_t>(n, (int64_t)(1u << 30) / (8 * maxd)) / 32 * 32);
+    // equal chunks of whole 32-vector groups (residuals and codes are
+    // warp-interleaved), each no more than the encoder holds at once: a few warps left
+    // for a second wave would take as long as a full one
+    const int64_t at_once = std::max<int64_t>(
+        32, std::min<int64_t>((int64_t)(1u << 30) / (8 * maxd), (int64_t)encoder_sms() * kEncCtas * 32) / 32 * 32);
+    const int64_t nchunk = std::max<int64_t>(1, (n + at_once - 1) / at_once);
+    const int64_t chunk = std::max<int64_t>(32, ((n + nchunk - 1) / nchunk + 31) / 32 * 32);
     const int64_t chunk_pad = (std::min(chunk, n) + 31) / 32 * 32;
-    DevBuf resid(4 * (size_t)chunk_pad * maxd), codes(4 * (size_t)chunk_pad * maxd), facs(16 * (size_t)chunk_pad);
+    DevBuf resid(4 * (size_t)chunk_pad * maxd), codes(2 * (size_t)chunk_pad * maxd), facs(16 * (size_t)chunk_pad);
     DevBuf cslice(4 * (size_t)k * maxd);
     int off = 0;
     for (size_t s = 0; s < S; ++s) {
@@ -698,11 +987,14 @@ Index *construct_index(const float *data, int64_t n, int64_t dim, const float *c
             k_rotate<<<grid, 256>>>(ddata, (int)dim, drows.as<int64_t>() + v0, nv, off, (int)d,
                                     dP ? dP : idP->as<float>(), g.cent, dcid.as<int32_t>() + v0, resid.as<float>(), 1);
             launch_check("k_rotate");
-            k_caq_encode_clustered<<<(unsigned)((nv + 63) / 64), 64>>>(
-                resid.as<float>(), nv, (int)d, g.bits, cslice.as<float>(), dcid.as<int32_t>() + v0, cfg.caq_adj_rd_lmt,
-                cfg.caq_adj_eps, codes.as<int32_t>(), facs.as<float>());
+            by_width(g.bits, [&](auto w) {
+                k_caq_encode_clustered<decltype(w)::value>
+                    <<<(unsigned)((nv + kEncThreads - 1) / kEncThreads), kEncThreads, enc_smem_bytes(g.bits)>>>(
+                        resid.as<float>(), nv, (int)d, g.bits, cslice.as<float>(), dcid.as<int32_t>() + v0,
+                        cfg.caq_adj_rd_lmt, cfg.caq_adj_eps, codes.as<uint16_t>(), facs.as<float>());
+            });
             launch_check("k_caq_encode");
-            k_pack<<<(unsigned)((nv + 127) / 128), 128>>>(codes.as<int32_t>(), facs.as<float>(), nv, v0,
+            k_pack<<<(unsigned)((nv + 127) / 128), 128>>>(codes.as<uint16_t>(), facs.as<float>(), nv, v0,
                                                           dcid.as<int32_t>() + v0, dbo, dvo, g);
             launch_check("k_pack");
         }
