@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "device_common.cuh"
+#include "rotate.cuh"
 #include "saqg_internal.h"
 
 namespace saqg {
@@ -522,73 +523,54 @@ __global__ void k_colwise_var(const float *__restrict__ x, int64_t n, int D, flo
 }
 
 // Rotated residuals of one segment: out[v][i] = (x_v . P[:, i]) - rc[cid_v][i],
-// where x_v is rows[v]'s slice [off, off + dim) of the data, zero-padded past D,
-// and the dot product follows Eigen's GEMV order (one FMA chain per block of 16
-// inputs, or one chain when dim < 128, blocks added in order).  Tile: 64
-// vectors x 64 outputs per CTA, 4 x 4 per thread.
-constexpr int kRT = 64, kRK = 16;
-__global__ void __launch_bounds__(256) k_rotate(const float *__restrict__ data, int D, const int64_t *__restrict__ rows,
-                                                int64_t nv, int off, int dim, const float *__restrict__ P,
-                                                const float *__restrict__ rc, const int32_t *__restrict__ cid,
-                                                float *__restrict__ out, int interleaved) {
-    __shared__ float xs[kRK][kRT + 1];
-    __shared__ float ps[kRK][kRT];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int64_t v0 = (int64_t)blockIdx.y * kRT;
-    const int o0 = blockIdx.x * kRT;
-    const int fold = dim < 128 ? dim : 16;
-    float res[4][4], c[4][4];
+// where x_v is rows[v]'s slice [off, off + dim) of the data, zero-padded past D
+// (rotate_tile; rc null: no centroid taken off).  `vec`: the data are 16-byte
+// aligned (rows and slices start at multiples of 64 floats).  Output
+// warp-interleaved ([v / 32][dim][v % 32], padded to whole groups) or row-major.
+// 100,000 x 960 (184 GFLOP): 6.8 ms with 64 x 64
+// tiles of scalar FMAs, 3.6 ms now (51 TFLOP/s; FMA pipe 70%, shared memory 73%).
+__global__ void __launch_bounds__(kRotThreads, 2) k_rotate(const float *__restrict__ data, int D,
+                                                           const int64_t *__restrict__ rows, int64_t nv, int off,
+                                                           int dim, const float *__restrict__ P,
+                                                           const float *__restrict__ rc,
+                                                           const int32_t *__restrict__ cid, float *__restrict__ out,
+                                                           int interleaved, int vec) {
+    rotate_tile(
+        dim, P, (int64_t)blockIdx.y * kRotM, blockIdx.x * kRotN,
+        [&](int64_t v, int j) {
+            float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (v < nv && off + j < D) {  // D is a multiple of 64: four inputs at once are in or out
+                const float *x = data + rows[v] * D + off + j;
+                if (vec) r = *reinterpret_cast<const float4 *>(x);
+                else r = make_float4(x[0], x[1], x[2], x[3]);
+            }
+            return r;
+        },
+        [&](int64_t v, int o, float (&r)[8][4]) {
+            if (v >= nv) return;
+            if (rc)
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) res[a][b] = c[a][b] = 0.0f;
-    for (int j0 = 0; j0 < dim; j0 += kRK) {
-        for (int t = threadIdx.x; t < kRT * kRK; t += 256) {
-            const int r = t / kRK, k = t % kRK;
-            const int64_t v = v0 + r;
-            const int gj = off + j0 + k;
-            float val = 0.0f;
-            if (v < nv && gj < D) val = data[rows[v] * D + gj];
-            xs[k][r] = val;
-            const int rr = t / kRT, cc = t % kRT;
-            ps[rr][cc] = (o0 + cc < dim) ? P[(int64_t)(j0 + rr) * dim + o0 + cc] : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kRK; ++k) {
-            float xv[4], pv[4];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) xv[a] = xs[k][ty * 4 + a];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) pv[b] = ps[k][tx * 4 + b];
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int b = 0; b < 4; ++b) c[a][b] = fmaf(pv[b], xv[a], c[a][b]);
-        }
-        if ((j0 + kRK) % fold == 0) {
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
+                for (int i = 0; i < 8; ++i) {
+                    const float4 c = *reinterpret_cast<const float4 *>(rc + (int64_t)cid[min(v + i, nv - 1)] * dim + o);
+                    r[i][0] = __fsub_rn(r[i][0], c.x);
+                    r[i][1] = __fsub_rn(r[i][1], c.y);
+                    r[i][2] = __fsub_rn(r[i][2], c.z);
+                    r[i][3] = __fsub_rn(r[i][3], c.w);
+                }
+            if (interleaved) {
 #pragma unroll
                 for (int b = 0; b < 4; ++b) {
-                    res[a][b] = fmaf(c[a][b], 1.0f, res[a][b]);
-                    c[a][b] = 0.0f;
+                    float4 *d = reinterpret_cast<float4 *>(out + (v >> 5) * (int64_t)dim * 32 + (int64_t)(o + b) * 32 + (v & 31));
+                    d[0] = make_float4(r[0][b], r[1][b], r[2][b], r[3][b]);
+                    d[1] = make_float4(r[4][b], r[5][b], r[6][b], r[7][b]);
                 }
-        }
-        __syncthreads();
-    }
+            } else {
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int64_t v = v0 + ty * 4 + a;
-        if (v >= nv) continue;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int o = o0 + tx * 4 + b;
-            if (o >= dim) continue;
-            const float r = rc ? __fsub_rn(res[a][b], rc[(int64_t)cid[v] * dim + o]) : res[a][b];
-            out[interleaved ? (v >> 5) * (int64_t)dim * 32 + (int64_t)o * 32 + (v & 31) : v * dim + o] = r;
-        }
-    }
+                for (int i = 0; i < 8; ++i)
+                    if (v + i < nv)
+                        *reinterpret_cast<float4 *>(out + (v + i) * dim + o) = make_float4(r[i][0], r[i][1], r[i][2], r[i][3]);
+            }
+        });
 }
 
 // Un-rotated centroid slice (zero-padded) of cluster c, as the reference passes
@@ -960,10 +942,10 @@ Index *construct_index(const float *data, int64_t n, int64_t dim, const float *c
         SAQG_CUDA_TRY(cudaMemset(g.exfac, 0, 8 * (size_t)n));
         // rotated centroids: clus.centroid() = centroid * P (quantizer.hpp:46)
         {
-            dim3 grid((unsigned)((d + kRT - 1) / kRT), (unsigned)((k + kRT - 1) / kRT));
+            dim3 grid((unsigned)(d / kRotN), (unsigned)((k + kRotM - 1) / kRotM));
             if (dP) {
-                k_rotate<<<grid, 256>>>(dcent, (int)dim, didx.as<int64_t>(), k, off, (int)d, dP, nullptr, nullptr, g.cent,
-                                        0);
+                k_rotate<<<grid, kRotThreads>>>(dcent, (int)dim, didx.as<int64_t>(), k, off, (int)d, dP, nullptr, nullptr,
+                                                g.cent, 0, 1);
                 launch_check("k_rotate(centroids)");
             }
             k_centroid_slices<<<(unsigned)((k * d + 255) / 256), 256>>>(dcent, k, (int)dim, off, (int)d,
@@ -983,9 +965,10 @@ Index *construct_index(const float *data, int64_t n, int64_t dim, const float *c
         }
         for (int64_t v0 = 0; v0 < n; v0 += chunk) {
             const int64_t nv = std::min(chunk, n - v0);
-            dim3 grid((unsigned)((d + kRT - 1) / kRT), (unsigned)((nv + kRT - 1) / kRT));
-            k_rotate<<<grid, 256>>>(ddata, (int)dim, drows.as<int64_t>() + v0, nv, off, (int)d,
-                                    dP ? dP : idP->as<float>(), g.cent, dcid.as<int32_t>() + v0, resid.as<float>(), 1);
+            dim3 grid((unsigned)(d / kRotN), (unsigned)((nv + kRotM - 1) / kRotM));
+            k_rotate<<<grid, kRotThreads>>>(ddata, (int)dim, drows.as<int64_t>() + v0, nv, off, (int)d,
+                                            dP ? dP : idP->as<float>(), g.cent, dcid.as<int32_t>() + v0,
+                                            resid.as<float>(), 1, ((uintptr_t)ddata & 15) == 0);
             launch_check("k_rotate");
             by_width(g.bits, [&](auto w) {
                 k_caq_encode_clustered<decltype(w)::value>

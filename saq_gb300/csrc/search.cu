@@ -6,7 +6,8 @@
 //                  (FlatInitializer::centroids_distances, initializer.hpp:52-76)
 //   k_probe_select the nprobe nearest in std::partial_sort order: radix select
 //                  + sort; on any tie the exact libstdc++ heap algorithm runs
-//   k_qprep        per segment: zero-padded query slice, prune bound
+//   k_qprep_few / k_qprep_tiled + k_prune_bounds
+//                  per segment: zero-padded query slice, prune bound
 //                  sqrt(sum var*q^2)*m and the rotated query q_s*P_s in Eigen's
 //                  GEMV order (saq_estimator.hpp:28-48, caq_estimator.hpp:56-68)
 //   k_scan         one CTA per query walks its probes in order.  Per cluster:
@@ -29,6 +30,7 @@
 #include <tuple>
 
 #include "device_common.cuh"
+#include "rotate.cuh"
 #include "saqg_internal.h"
 
 namespace saqg {
@@ -615,40 +617,16 @@ __global__ void k_probe_dist_list(DevIndexView ix, const float *__restrict__ q, 
 }
 
 // ------------------------------------------------------------------ query prep
-__global__ void k_qprep(DevIndexView ix, const float *__restrict__ q, float m, float *__restrict__ qrot,
-                        float *__restrict__ prune) {
-    extern __shared__ float cq[];
-    const int s = blockIdx.x, qi = blockIdx.y;
-    const SegDev &g = ix.seg[s];
-    const int dim = g.dim, qoff = g.qoff;
-    for (int i = threadIdx.x; i < dim; i += blockDim.x) {
-        const int gi = qoff + i;
-        cq[i] = gi < ix.D ? q[(size_t)qi * ix.D + gi] : 0.0f;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const float *var = ix.var + qoff;
-        const float v2 = warp_eigen_sum(dim, [&](int i) { return __fmul_rn(var[i], __fmul_rn(cq[i], cq[i])); });
-        if (threadIdx.x == 0) prune[(size_t)qi * ix.S + s] = __fmul_rn(sqrtf(v2), m);
-    }
-    float *out = qrot + (size_t)qi * ix.Dtot + qoff;
-    if (!g.P) {
-        for (int i = threadIdx.x; i < dim; i += blockDim.x) out[i] = cq[i];
-        return;
-    }
-    // Eigen general_matrix_vector_product<ColMajor> (GeneralMatrixVector.h:108-300):
-    // per output, FMA chains over blocks of 16 inputs (one block if dim < 128).
-    const int bc = dim < 128 ? dim : 16;
-    for (int i = threadIdx.x; i < dim; i += blockDim.x) {
-        float res = 0.0f;
-        for (int j2 = 0; j2 < dim; j2 += bc) {
-            float c = 0.0f;
-            const int je = min(j2 + bc, dim);
-            for (int j = j2; j < je; ++j) c = fmaf(g.P[(size_t)j * dim + i], cq[j], c);
-            res = fmaf(c, 1.0f, res);
-        }
-        out[i] = res;
-    }
+// Prune bound sqrt(sum var * q^2) * m of segment s and query slice cq (zero-padded
+// past the dimension), by one warp; valid in every lane.
+template <class Q>
+__device__ __forceinline__ float prune_bound(const DevIndexView &ix, const SegDev &g, float m, Q cq) {
+    const float *var = ix.var + g.qoff;
+    const float v2 = warp_eigen_sum(g.dim, [&](int i) {
+        const float q = cq(i);
+        return __fmul_rn(var[i], __fmul_rn(q, q));
+    });
+    return __fmul_rn(sqrtf(v2), m);
 }
 
 // ------------------------------------------------------------------ LUT
@@ -721,138 +699,136 @@ __device__ __forceinline__ void pool_insert(uint32_t *ids, float *d, int &size, 
     size += (size < cap);
 }
 
-// k_qprep for a few queries, spread for latency: in Eigen's GEMV order the
-// 16-input block sums c_b of an output are independent (only their fold
-// res = fma(c_b, 1, res) runs in block order), so a CTA takes 32 outputs of
-// one (segment, query), its warps compute the block sums (lane = output, a
-// 16-step chain each), and warp 0 folds them in order.  Bit-identical to
-// k_qprep; the prune bound comes from the CTA holding the first 32 outputs.
+// Prune bounds and rotated queries (saq_estimator.hpp:28-48, caq_estimator.hpp:56-68)
+// of a few queries, spread for latency: in Eigen's GEMV order the 16-input block
+// sums of an output are independent (only their fold runs in block order), so a
+// CTA takes 32 outputs of one segment for up to kQprepFewQ queries, its warps
+// compute the block sums (lane = output; the block's 16 matrix elements are loaded
+// at once and serve every query), and the sums are folded in order.  The prune
+// bounds come from the CTA of the first 32 outputs.  Bound by one pass of load
+// latency: one query of 960 dimensions 11.6 us (62 us with the block's elements
+// loaded one after the other), 37 of segments (64, 320, 640) 11.2 us (88 us).
 constexpr int kQprepOut = 32;
-__global__ void __launch_bounds__(256) k_qprep_small(DevIndexView ix, const float *__restrict__ q, float m,
-                                                     float *__restrict__ qrot, float *__restrict__ prune) {
-    extern __shared__ __align__(16) float qsm[];  // [dim] query slice, then [dim / 16][32] block sums
-    const int s = blockIdx.x, qi = blockIdx.y, o0 = blockIdx.z * kQprepOut;
+constexpr int kQprepFewQ = 8;
+constexpr int kQprepFewThreads = 512;
+__host__ __device__ inline size_t qprep_few_smem(int dim, int nq) {
+    const int blocks = dim < 128 ? 1 : dim / 16;
+    return 4 * (size_t)nq * (dim + (size_t)blocks * kQprepOut);
+}
+__global__ void __launch_bounds__(kQprepFewThreads) k_qprep_few(DevIndexView ix, const float *__restrict__ q, int nq,
+                                                                float m, float *__restrict__ qrot,
+                                                                float *__restrict__ prune) {
+    extern __shared__ __align__(16) float qsm[];  // [queries][dim], then [block][queries][32] block sums
+    const int s = blockIdx.y, q0 = blockIdx.z * kQprepFewQ, nqt = min(kQprepFewQ, nq - q0);
     const SegDev &g = ix.seg[s];
-    const int dim = g.dim, qoff = g.qoff;
+    const int dim = g.dim, qoff = g.qoff, o0 = blockIdx.x * kQprepOut;
     if (o0 >= dim) return;
-    float *cq = qsm, *part = qsm + dim;
-    for (int i = threadIdx.x; i < dim; i += blockDim.x) {
-        const int gi = qoff + i;
-        cq[i] = gi < ix.D ? q[(size_t)qi * ix.D + gi] : 0.0f;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = kQprepFewThreads / 32, i = o0 + lane;
+    const int nbk = dim < 128 ? 1 : dim / 16;
+    float *cq = qsm, *part = qsm + nqt * dim;
+    for (int e = threadIdx.x; e < nqt * dim; e += kQprepFewThreads) {
+        const int t = e / dim, gi = qoff + e - t * dim;
+        cq[e] = gi < ix.D ? q[(size_t)(q0 + t) * ix.D + gi] : 0.0f;
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i = o0 + lane;
-    if (blockIdx.z == 0 && warp == 1) {
-        const float *var = ix.var + qoff;
-        const float v2 = warp_eigen_sum(dim, [&](int e) { return __fmul_rn(var[e], __fmul_rn(cq[e], cq[e])); });
-        if (lane == 0) prune[(size_t)qi * ix.S + s] = __fmul_rn(sqrtf(v2), m);
+    if (g.P) {
+        if (dim < 128) {  // one chain of `dim` inputs: a warp per query
+            for (int t = warp; t < nqt; t += nw) {
+                float c = 0.0f;
+#pragma unroll 16
+                for (int j = 0; j < dim; ++j) c = fmaf(g.P[(size_t)j * dim + i], cq[t * dim + j], c);
+                part[t * kQprepOut + lane] = c;
+            }
+        } else {
+            for (int b = warp; b < nbk; b += nw) {
+                float p[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) p[j] = g.P[(size_t)(16 * b + j) * dim + i];
+#pragma unroll 2
+                for (int t = 0; t < nqt; ++t) {
+                    const float4 *x = reinterpret_cast<const float4 *>(cq + t * dim + 16 * b);
+                    float c = 0.0f;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float4 v = x[j];
+                        c = fmaf(p[4 * j], v.x, c);
+                        c = fmaf(p[4 * j + 1], v.y, c);
+                        c = fmaf(p[4 * j + 2], v.z, c);
+                        c = fmaf(p[4 * j + 3], v.w, c);
+                    }
+                    part[(b * nqt + t) * kQprepOut + lane] = c;
+                }
+            }
+        }
     }
-    float *out = qrot + (size_t)qi * ix.Dtot + qoff;
-    if (!g.P) {
-        if (warp == 0 && i < dim) out[i] = cq[i];
-        return;
-    }
-    const int bc = dim < 128 ? dim : 16, nbk = (dim + bc - 1) / bc;
-    for (int b = warp; b < nbk; b += blockDim.x >> 5) {
-        float c = 0.0f;
-        const int j2 = b * bc, je = min(j2 + bc, dim);
-        if (i < dim)
-            for (int j = j2; j < je; ++j) c = fmaf(g.P[(size_t)j * dim + i], cq[j], c);
-        part[b * kQprepOut + lane] = c;
-    }
+    if (blockIdx.x == 0)
+        for (int t = warp; t < nqt; t += nw) {
+            const float v = prune_bound(ix, g, m, [&](int e) { return cq[t * dim + e]; });
+            if (lane == 0) prune[(size_t)(q0 + t) * ix.S + s] = v;
+        }
     __syncthreads();
-    if (warp == 0 && i < dim) {
+    for (int t = warp; t < nqt; t += nw) {
         float res = 0.0f;
-        for (int b = 0; b < nbk; ++b) res = fmaf(part[b * kQprepOut + lane], 1.0f, res);
-        out[i] = res;
+        if (g.P) {
+#pragma unroll 8
+            for (int b = 0; b < nbk; ++b) res = __fadd_rn(part[(b * nqt + t) * kQprepOut + lane], res);
+        } else {
+            res = cq[t * dim + i];
+        }
+        qrot[(size_t)(q0 + t) * ix.Dtot + qoff + i] = res;
     }
 }
 
-// k_qprep for a tile of kQprepQT queries per CTA: each P element is read once
-// for the whole tile and drives kQprepQT independent chains, each in exactly
-// k_qprep's order (so the outputs are bit-identical); L2 traffic for the
-// rotations drops by the tile size.  A CTA computes kQprepSlice outputs (one
-// per thread; blockIdx.z picks the slice), and the P column of the next
-// 16-input block is loaded while the current block's chains run.
-constexpr int kQprepQT = 16;
-constexpr int kQprepSlice = 256;
-__global__ void __launch_bounds__(kQprepSlice) k_qprep_tiled(DevIndexView ix, const float *__restrict__ q, int nq,
-                                                             float m, float *__restrict__ qrot,
-                                                             float *__restrict__ prune) {
-    extern __shared__ __align__(16) float cqs[];  // [kQprepQT][dim]
-    const int s = blockIdx.x, q0 = blockIdx.y * kQprepQT, nqt = min(kQprepQT, nq - q0);
-    const SegDev &g = ix.seg[s];
+// The same for a batch: tiles of 128 queries x 64 outputs (rotate_tile), grid
+// (outputs, segment, queries); the prune bounds in a kernel of their own (a warp
+// per query and segment).  2,048 queries of 1,536 dimensions: 615 us with 16
+// queries x 256 outputs per CTA, one thread per output; 226 us
+// now, 16 us the bounds.
+__global__ void __launch_bounds__(kRotThreads, 2) k_qprep_tiled(DevIndexView ix, const float *__restrict__ q, int nq,
+                                                                int vec, float *__restrict__ qrot) {
+    const SegDev &g = ix.seg[blockIdx.y];
     const int dim = g.dim, qoff = g.qoff;
-    const int i = blockIdx.z * kQprepSlice + threadIdx.x;
-    if (blockIdx.z * kQprepSlice >= dim) return;
-    for (int e = threadIdx.x; e < kQprepQT * dim; e += blockDim.x) {
-        const int t = e / dim, ii = e - t * dim, gi = qoff + ii;
-        cqs[e] = (t < nqt && gi < ix.D) ? q[(size_t)(q0 + t) * ix.D + gi] : 0.0f;
-    }
-    __syncthreads();
-    const int warp = threadIdx.x >> 5;
-    if (blockIdx.z == 0)
-        for (int t = warp; t < nqt; t += blockDim.x >> 5) {
-            const float *cq = cqs + t * dim, *var = ix.var + qoff;
-            const float v2 = warp_eigen_sum(dim, [&](int k) { return __fmul_rn(var[k], __fmul_rn(cq[k], cq[k])); });
-            if ((threadIdx.x & 31) == 0) prune[(size_t)(q0 + t) * ix.S + s] = __fmul_rn(sqrtf(v2), m);
+    if ((int)blockIdx.x * kRotN >= dim) return;
+    auto load4 = [&](int64_t v, int j) {
+        float4 r = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const int gi = qoff + j;
+        if (v < nq) {
+            const float *x = q + (size_t)v * ix.D + gi;
+            if (vec && gi + 3 < ix.D) r = *reinterpret_cast<const float4 *>(x);
+            else r = make_float4(gi < ix.D ? x[0] : 0.0f, gi + 1 < ix.D ? x[1] : 0.0f, gi + 2 < ix.D ? x[2] : 0.0f,
+                                 gi + 3 < ix.D ? x[3] : 0.0f);
         }
-    if (i >= dim) return;
-    if (!g.P) {
-        for (int t = 0; t < nqt; ++t) qrot[(size_t)(q0 + t) * ix.Dtot + qoff + i] = cqs[t * dim + i];
+        return r;
+    };
+    if (!g.P) {  // no rotation: the padded slice itself
+        const int64_t v0 = (int64_t)blockIdx.z * kRotM;
+        for (int e = threadIdx.x; e < kRotM * kRotN / 4; e += kRotThreads) {
+            const int64_t v = v0 + e / (kRotN / 4);
+            const int j = blockIdx.x * kRotN + e % (kRotN / 4) * 4;
+            if (v < nq) *reinterpret_cast<float4 *>(qrot + v * ix.Dtot + qoff + j) = load4(v, j);
+        }
         return;
     }
-    float res[kQprepQT], c[kQprepQT];
+    rotate_tile(dim, g.P, (int64_t)blockIdx.z * kRotM, blockIdx.x * kRotN, load4,
+                [&](int64_t v, int o, float (&r)[8][4]) {
 #pragma unroll
-    for (int t = 0; t < kQprepQT; ++t) res[t] = 0.0f;
-    if (dim < 128) {  // one block of `dim` inputs (dims are multiples of 64)
-#pragma unroll
-        for (int t = 0; t < kQprepQT; ++t) c[t] = 0.0f;
-        for (int j = 0; j < dim; j += 4) {
-            const float p0 = g.P[(size_t)j * dim + i], p1 = g.P[(size_t)(j + 1) * dim + i];
-            const float p2 = g.P[(size_t)(j + 2) * dim + i], p3 = g.P[(size_t)(j + 3) * dim + i];
-#pragma unroll
-            for (int t = 0; t < kQprepQT; ++t) {
-                const float4 v = *reinterpret_cast<const float4 *>(cqs + t * dim + j);
-                c[t] = fmaf(p0, v.x, c[t]);
-                c[t] = fmaf(p1, v.y, c[t]);
-                c[t] = fmaf(p2, v.z, c[t]);
-                c[t] = fmaf(p3, v.w, c[t]);
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < kQprepQT; ++t) res[t] = fmaf(c[t], 1.0f, res[t]);
-    } else {  // blocks of 16 inputs, the next block's P column in flight
-        float pc[16], pn[16];
-#pragma unroll
-        for (int jj = 0; jj < 16; ++jj) pc[jj] = g.P[(size_t)jj * dim + i];
-        for (int j2 = 0; j2 < dim; j2 += 16) {
-            if (j2 + 16 < dim) {
-#pragma unroll
-                for (int jj = 0; jj < 16; ++jj) pn[jj] = g.P[(size_t)(j2 + 16 + jj) * dim + i];
-            }
-#pragma unroll
-            for (int t = 0; t < kQprepQT; ++t) c[t] = 0.0f;
-#pragma unroll
-            for (int jj = 0; jj < 16; jj += 4) {
-#pragma unroll
-                for (int t = 0; t < kQprepQT; ++t) {
-                    const float4 v = *reinterpret_cast<const float4 *>(cqs + t * dim + j2 + jj);
-                    c[t] = fmaf(pc[jj], v.x, c[t]);
-                    c[t] = fmaf(pc[jj + 1], v.y, c[t]);
-                    c[t] = fmaf(pc[jj + 2], v.z, c[t]);
-                    c[t] = fmaf(pc[jj + 3], v.w, c[t]);
-                }
-            }
-#pragma unroll
-            for (int t = 0; t < kQprepQT; ++t) res[t] = fmaf(c[t], 1.0f, res[t]);
-#pragma unroll
-            for (int jj = 0; jj < 16; ++jj) pc[jj] = pn[jj];
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < kQprepQT; ++t)
-        if (t < nqt) qrot[(size_t)(q0 + t) * ix.Dtot + qoff + i] = res[t];
+                    for (int i = 0; i < 8; ++i)
+                        if (v + i < nq)
+                            *reinterpret_cast<float4 *>(qrot + (v + i) * ix.Dtot + qoff + o) =
+                                make_float4(r[i][0], r[i][1], r[i][2], r[i][3]);
+                });
+}
+__global__ void __launch_bounds__(256) k_prune_bounds(DevIndexView ix, const float *__restrict__ q, int nq, float m,
+                                                      float *__restrict__ prune) {
+    const int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (w >= (int64_t)nq * ix.S) return;
+    const int64_t qi = w / ix.S;
+    const int s = (int)(w - qi * ix.S);
+    const SegDev &g = ix.seg[s];
+    const float *x = q + qi * ix.D + g.qoff;
+    const int n = ix.D - g.qoff;
+    const float v = prune_bound(ix, g, m, [&](int i) { return i < n ? x[i] : 0.0f; });
+    if ((threadIdx.x & 31) == 0) prune[w] = v;
 }
 
 // ------------------------------------------------------------------ scan
@@ -3051,6 +3027,39 @@ int full_grid(const void *fn, int threads, size_t smem) {
     return g;
 }
 
+// Prune bounds and rotated queries of a call on `st`.  k_qprep_few spreads over the
+// GPU but reads the matrices once per 8 queries, k_qprep_tiled reads them once per
+// 128 and needs a chain of the longest segment's length: up to kQprepFewWork
+// query-matrix elements the former is faster.  Segments (64, 320, 640): 64 queries
+// 12 against 49 us, 512: 45 against 50, 1,024: 80 against 75; one of 1,536: 128
+// queries 68 against 106 us, 256: 124 against 108.
+constexpr int64_t kQprepFewWork = 400000000;
+void launch_qprep(const DevIndexView &ix, const float *q, int64_t nq, float m, float *qrot, float *prune,
+                  cudaStream_t st) {
+    int dmax = 0;
+    int64_t elems = 0;
+    for (int s = 0; s < ix.S; ++s) {
+        dmax = std::max(dmax, ix.seg[s].dim);
+        elems += (int64_t)ix.seg[s].dim * ix.seg[s].dim;
+    }
+    const int few = (int)std::min<int64_t>(nq, kQprepFewQ);
+    const size_t smem = qprep_few_smem(dmax, few);
+    if (nq <= kQprepFewWork / elems && smem <= 200 * 1024) {
+        ensure_smem((const void *)k_qprep_few, smem);
+        k_qprep_few<<<dim3((unsigned)(dmax / kQprepOut), (unsigned)ix.S, (unsigned)((nq + kQprepFewQ - 1) / kQprepFewQ)),
+                      kQprepFewThreads, smem, st>>>(ix, q, (int)nq, m, qrot, prune);
+        check_launch("k_qprep_few");
+        return;
+    }
+    const int vec = ((uintptr_t)q & 15) == 0 && ix.D % 4 == 0;
+    k_qprep_tiled<<<dim3((unsigned)(dmax / kRotN), (unsigned)ix.S, (unsigned)((nq + kRotM - 1) / kRotM)), kRotThreads, 0,
+                    st>>>(ix, q, (int)nq, vec, qrot);
+    check_launch("k_qprep_tiled");
+    k_prune_bounds<<<(unsigned)((nq * ix.S + 7) / 8), 256, 0, st>>>(ix, q, (int)nq, m, prune);
+    check_launch("k_prune_bounds");
+    count_launch(1);
+}
+
 }  // namespace
 
 int64_t tune_bucket(int64_t nq) {
@@ -3271,34 +3280,19 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
         // (beside the shortlist and its select when the GEMM ranks the centroids:
         // the GEMM wants whole SMs; those two then run at the greatest priority,
         // so their CTAs go first)
-        auto launch_qprep = [&]() {
+        auto fork_qprep = [&]() {
             cudaStream_t qs = C.low_stream();
             SAQG_CUDA_TRY(cudaEventRecord(C.qfork_event(), st));
             SAQG_CUDA_TRY(cudaStreamWaitEvent(qs, C.qfork_event(), 0));
-            size_t qsm = 0;
-            for (int s = 0; s < ix.S; ++s) qsm = std::max(qsm, (size_t)4 * ix.seg[s].dim);
-            if (nq >= kQprepQT && kQprepQT * qsm <= 200 * 1024) {
-                ensure_smem((const void *)k_qprep_tiled, (size_t)(kQprepQT * qsm));
-                k_qprep_tiled<<<dim3((unsigned)ix.S, (unsigned)((nq + kQprepQT - 1) / kQprepQT),
-                                     (unsigned)((qsm / 4 + kQprepSlice - 1) / kQprepSlice)),
-                                kQprepSlice, kQprepQT * qsm, qs>>>(ix, qin, (int)nq, m, qrot, prune);
-                check_launch("k_qprep_tiled");
-            } else {
-                int dmax = 0;
-                for (int s = 0; s < ix.S; ++s) dmax = std::max(dmax, ix.seg[s].dim);
-                const size_t sm_small = 4 * ((size_t)dmax + (size_t)(dmax / 16 + 1) * kQprepOut);
-                k_qprep_small<<<dim3((unsigned)ix.S, (unsigned)nq, (unsigned)((dmax + kQprepOut - 1) / kQprepOut)),
-                                256, sm_small, qs>>>(ix, qin, m, qrot, prune);
-                check_launch("k_qprep_small");
-            }
+            launch_qprep(ix, qin, nq, m, qrot, prune, qs);
             SAQG_CUDA_TRY(cudaEventRecord(C.qjoin_event(), qs));
         };
         const char *pm = std::getenv("SAQG_PROBE");
         shortlist = nq >= kGemmMinQueries && nprobe <= kShortCap && !(pm && std::string(pm) == "exact");
-        if (!shortlist) launch_qprep();
+        if (!shortlist) fork_qprep();
         if (shortlist) {
             probe_shortlist(I, C, qin, nq, nprobe, qsh.np, dist, probe, full, fb_list, flags, work,
-                            stats ? counters : nullptr, qbf, st, launch_qprep);
+                            stats ? counters : nullptr, qbf, st, fork_qprep);
         } else if (nq >= 8 && I.D % 32 == 0 && I.D <= 32 * kProbeRegs) {
             const size_t qsm = 4 * (size_t)kProbeQT * I.D;
             ensure_smem((const void *)k_probe_dist_tiled, (size_t)qsm);
@@ -3560,10 +3554,7 @@ int64_t run_estimate(const Index &I, const float *q_host, int64_t nprobe, float 
     check_launch("k_probe_dist");
     k_probe_select<<<1, kSelThreads, 0, st>>>(dist, (int)I.K, (int)nprobe, probe, work, flags);
     check_launch("k_probe_select");
-    size_t qsm = 0;
-    for (int s = 0; s < ix.S; ++s) qsm = std::max(qsm, (size_t)4 * ix.seg[s].dim);
-    k_qprep<<<dim3((unsigned)ix.S, 1), 256, qsm, st>>>(ix, dq, m, qrot, prune);
-    check_launch("k_qprep");
+    launch_qprep(ix, dq, 1, m, qrot, prune, st);
     std::vector<uint32_t> hprobe(nprobe);
     SAQG_CUDA_TRY(cudaMemcpy(hprobe.data(), probe, 4 * nprobe, cudaMemcpyDeviceToHost));
     std::vector<int64_t> off(nprobe + 1, 0);
@@ -3710,10 +3701,7 @@ void run_search_static(const Index &I, const float *q, int64_t nq, int64_t topk,
     }
     k_probe_select<<<(unsigned)nq, kSelThreads, 0, st>>>(dist, (int)I.K, (int)nprobe, probe, work, flags);
     check_launch("k_probe_select");
-    size_t qsm = 0;
-    for (int s = 0; s < ix.S; ++s) qsm = std::max(qsm, (size_t)4 * ix.seg[s].dim);
-    k_qprep<<<dim3((unsigned)ix.S, (unsigned)nq), 256, qsm, st>>>(ix, q, m, qrot, prune);
-    check_launch("k_qprep");
+    launch_qprep(ix, q, nq, m, qrot, prune, st);
     const size_t smem_k = scan_smem_bytes(ix.Dtot, ix.S, (int)topk, xstride_of(ix));
     SAQG_REQUIRE(smem_k <= 200 * 1024, "dimension / topk too large for the scan kernel's shared memory");
     ensure_smem((const void *)k_scan, (size_t)smem_k);
@@ -3914,18 +3902,7 @@ void tc_rank_rotate(const Index &I, SearchCtx &C, const float *q, int64_t nq, in
                                                               qnp);
         check_launch("k_probe_select");
     }
-    size_t qsm = 0;
-    for (int s = 0; s < ix.S; ++s) qsm = std::max(qsm, (size_t)4 * ix.seg[s].dim);
-    if (nq >= kQprepQT && kQprepQT * qsm <= 200 * 1024) {
-        ensure_smem((const void *)k_qprep_tiled, (size_t)(kQprepQT * qsm));
-        k_qprep_tiled<<<dim3((unsigned)ix.S, (unsigned)((nq + kQprepQT - 1) / kQprepQT),
-                             (unsigned)((qsm / 4 + kQprepSlice - 1) / kQprepSlice)),
-                        kQprepSlice, kQprepQT * qsm, st>>>(ix, q, (int)nq, m, qrot, prune);
-        check_launch("k_qprep_tiled");
-    } else {
-        k_qprep<<<dim3((unsigned)ix.S, (unsigned)nq), 256, qsm, st>>>(ix, q, m, qrot, prune);
-        check_launch("k_qprep");
-    }
+    launch_qprep(ix, q, nq, m, qrot, prune, st);
     count_launch(4);
 }
 
