@@ -500,26 +500,106 @@ namespace {
 // SaqDataMaker::compute_variance (saq_data.hpp:95-100): column means by Eigen's
 // packetwise reduction (PartialReduxEvaluator.h:102-128), variances of the
 // rowwise() difference by a sequential column sum (that expression has no
-// packet access); both divided by the row count.  One thread per column.
-__global__ void k_colwise_var(const float *__restrict__ x, int64_t n, int D, float *__restrict__ var) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= D) return;
-    float p = x[c];
-    const int64_t size4 = (n - 1) & ~int64_t(3);
-    int64_t i = 1;
-    for (; i < size4; i += 4) {
-        const float a = __fadd_rn(x[i * D + c], x[(i + 1) * D + c]);
-        const float b = __fadd_rn(x[(i + 2) * D + c], x[(i + 3) * D + c]);
-        p = __fadd_rn(p, __fadd_rn(a, b));
-    }
-    for (; i < n; ++i) p = __fadd_rn(p, x[i * D + c]);
+// packet access); both divided by the row count.
+//
+// The order of the sums leaves one chain of n / 4 and one of n FP32 adds per
+// column, so a column belongs to one thread and its time is the adds' latency if
+// the rows arrive in time.  A CTA has 16 columns (64 bytes of a row; more CTAs than
+// with 32 share the loading): warp 1 keeps 14 stages of 64 rows in flight by
+// asynchronous copies while warp 0 adds one up.  Row 0 is taken apart, so that the
+// groups of four rows of the mean start at a stage.  250,007 x 1,024: 36 ms with a
+// thread per column loading its own rows (each group waited for memory), 3.4 with
+// one warp copying and adding, 2.0 now.
+constexpr int kVarCols = 16, kVarRows = 64, kVarStages = 16, kVarThreads = 64;
+__global__ void __launch_bounds__(kVarThreads) k_colwise_var(const float *__restrict__ x, int64_t n, int D, int vec,
+                                                             float *__restrict__ var) {
+    extern __shared__ __align__(16) float var_ring[];  // [stage][row][kVarCols]
+    const int lane = threadIdx.x & 31, c0 = blockIdx.x * kVarCols, col = lane & (kVarCols - 1);
+    const bool copier = threadIdx.x >= 32;
+    const int64_t rest = n - 1, nst = (rest + kVarRows - 1) / kVarRows;  // rows 1 .. n - 1 in stages
+    auto issue = [&](int64_t st) {
+        if (st < nst) {
+            float *dst = var_ring + (int)(st & (kVarStages - 1)) * (kVarRows * kVarCols);
+            const int rows = (int)min((int64_t)kVarRows, rest - st * kVarRows);
+            const float *src = x + (1 + st * kVarRows) * D + c0;
+            if (vec) {
+                const int k = lane % (kVarCols / 4) * 4;
+#pragma unroll
+                for (int r = lane / (kVarCols / 4); r < kVarRows; r += 128 / kVarCols)
+                    if (r < rows)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                         (unsigned)__cvta_generic_to_shared(dst + r * kVarCols + k)),
+                                     "l"(src + (int64_t)r * D + k)
+                                     : "memory");
+            } else {
+                for (int e = lane; e < rows * kVarCols; e += 32) {
+                    const int r = e / kVarCols, k = e % kVarCols;
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                                     (unsigned)__cvta_generic_to_shared(dst + r * kVarCols + k)),
+                                 "l"(src + (int64_t)r * D + k)
+                                 : "memory");
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // f(rows of the stage, its column) of warp 0: the stages in order.  While it adds
+    // stage st up, warp 1 refills the stage read before it and waits for the next.
+    auto stream = [&](auto f) {
+        if (copier) {
+            for (int st = 0; st < kVarStages - 1; ++st) issue(st);
+            asm volatile("cp.async.wait_group %0;" ::"n"(kVarStages - 2) : "memory");
+        }
+        __syncthreads();
+        for (int64_t st = 0; st < nst; ++st) {
+            if (copier) {
+                issue(st + kVarStages - 1);
+                asm volatile("cp.async.wait_group %0;" ::"n"(kVarStages - 2) : "memory");
+            } else {
+                f((int)min((int64_t)kVarRows, rest - st * kVarRows),
+                  var_ring + (int)(st & (kVarStages - 1)) * (kVarRows * kVarCols) + col);
+            }
+            __syncthreads();
+        }
+    };
+    const float first = x[c0 + col];
+    float p = first;
+    stream([&](int rows, const float *s) {
+        if (rows == kVarRows) {
+#pragma unroll
+            for (int r = 0; r < kVarRows; r += 4) {
+                const float a = __fadd_rn(s[r * kVarCols], s[(r + 1) * kVarCols]);
+                const float b = __fadd_rn(s[(r + 2) * kVarCols], s[(r + 3) * kVarCols]);
+                p = __fadd_rn(p, __fadd_rn(a, b));
+            }
+        } else {  // the last stage: groups of four while they fit, then single rows
+            int r = 0;
+            for (; r + 4 <= rows; r += 4) {
+                const float a = __fadd_rn(s[r * kVarCols], s[(r + 1) * kVarCols]);
+                const float b = __fadd_rn(s[(r + 2) * kVarCols], s[(r + 3) * kVarCols]);
+                p = __fadd_rn(p, __fadd_rn(a, b));
+            }
+            for (; r < rows; ++r) p = __fadd_rn(p, s[r * kVarCols]);
+        }
+    });
     const float mean = __fdiv_rn(p, (float)n);
-    float v = 0.0f;
-    for (int64_t r = 0; r < n; ++r) {
-        const float d = __fsub_rn(x[r * D + c], mean);
-        v = r == 0 ? __fmul_rn(d, d) : __fadd_rn(v, __fmul_rn(d, d));
-    }
-    var[c] = __fdiv_rn(v, (float)n);
+    const float d0 = __fsub_rn(first, mean);
+    float v = __fmul_rn(d0, d0);
+    stream([&](int rows, const float *s) {
+        if (rows == kVarRows) {
+#pragma unroll
+            for (int r = 0; r < kVarRows; ++r) {
+                const float d = __fsub_rn(s[r * kVarCols], mean);
+                v = __fadd_rn(v, __fmul_rn(d, d));
+            }
+        } else {
+            for (int r = 0; r < rows; ++r) {
+                const float d = __fsub_rn(s[r * kVarCols], mean);
+                v = __fadd_rn(v, __fmul_rn(d, d));
+            }
+        }
+    });
+    if (threadIdx.x < kVarCols) var[c0 + col] = __fdiv_rn(v, (float)n);
 }
 
 // Rotated residuals of one segment: out[v][i] = (x_v . P[:, i]) - rc[cid_v][i],
@@ -824,7 +904,10 @@ Index *construct_index(const float *data, int64_t n, int64_t dim, const float *c
         plan = make_plan_gpu(variance, dim, cfg.avg_bits, cfg.enable_segmentation != 0, cfg.seg_eqseg, false, 0);
     } else {
         DevBuf dv(4 * dim);
-        k_colwise_var<<<(unsigned)((dim + 127) / 128), 128>>>(ddata, n, (int)dim, dv.as<float>());
+        constexpr int ring = 4 * kVarStages * kVarRows * kVarCols;
+        SAQG_CUDA_TRY(cudaFuncSetAttribute(k_colwise_var, cudaFuncAttributeMaxDynamicSharedMemorySize, ring));
+        k_colwise_var<<<(unsigned)(dim / kVarCols), kVarThreads, ring>>>(ddata, n, (int)dim, ((uintptr_t)ddata & 15) == 0,
+                                                               dv.as<float>());
         launch_check("k_colwise_var");
         plan = make_plan_gpu(dv.as<float>(), dim, cfg.avg_bits, cfg.enable_segmentation != 0, cfg.seg_eqseg, true, 0);
         SAQG_CUDA_TRY(cudaMemcpy(I->var.data(), dv.p, 4 * dim, cudaMemcpyDeviceToHost));
