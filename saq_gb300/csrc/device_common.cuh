@@ -83,150 +83,149 @@ __device__ __forceinline__ float warp_min_tree(float x) {
 }
 
 // --------------------------------------------------------------- ex-codes
-// One 16-lane chain of CodeHelper<B>::compute_ip, lane l of a half-warp
-// accumulating dims l, l+16, l+32, ... in increasing order.  The reference's
-// compacted layouts were designed for 16-lane SIMD, so lane l reads the same
-// byte positions in every group of dims; the chains read them straight from
-// global memory (L1/L2), 16 consecutive bytes per half-warp load.
+// CodeHelper<B>::compute_ip (code_helper.hpp) by a half-warp: lane l accumulates
+// dims l, l+16, l+32, ... in increasing order, as SIMD lane l does, reading the
+// bytes that the reference's compacted layouts give that lane (the same positions
+// in every 64 dims) straight from global memory, 16 consecutive bytes per half-warp
+// load.  The query is in ex order: within every 64 dims, lane l's four values (dims
+// l, 16+l, 32+l, 48+l) lie together at 4l, one 16-byte load.
+__device__ __forceinline__ int ex_order(int d) { return (d & ~63) | ((d & 15) << 2) | ((d >> 4) & 3); }
+
+// The integer in the bits of `field` at position SH and up, as a float: set under
+// the mantissa of 2^(23-SH), whose last place then counts 2^-SH; the difference is
+// exact.  No shift and no conversion instruction.
+template <int SH>
+__device__ __forceinline__ float bits_float(uint32_t field) {
+    return __fsub_rn(__uint_as_float(field | (0x4b000000u - ((uint32_t)SH << 23))), __uint_as_float(0x4b000000u - ((uint32_t)SH << 23)));
+}
+
+// What lane l reads of 64 dims of a B-bit code, and its four values from that.
 template <int B>
-__device__ __forceinline__ float chain_bits(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int l);
-
-template <>
-__device__ __forceinline__ float chain_bits<1>(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int l) {
-    // CodeHelper<1>: bit d of the little-endian bit string; masked adds
-    float acc = 0.0f;
-    for (int g = 0; g < D; g += 16) {
-        const uint32_t m = (uint32_t)y[g / 8] | ((uint32_t)y[g / 8 + 1] << 8);
-        acc = __fadd_rn(acc, ((m >> l) & 1u) ? q[g + l] : 0.0f);
-    }
-    return acc;
-}
-
-template <>
-__device__ __forceinline__ float chain_bits<2>(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int l) {
-    float acc = 0.0f;
-    for (int g = 0; g < D; g += 64) {
-        const uint32_t b = y[(g / 64) * 16 + l];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) acc = fmaf((float)((b >> (2 * k)) & 3u), q[g + 16 * k + l], acc);
-    }
-    return acc;
-}
-
-template <>
-__device__ __forceinline__ float chain_bits<3>(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int l) {
-    float acc = 0.0f;
-    for (int g = 0; g < D; g += 64) {
-        const uint8_t *gp = y + (g / 64) * 24;
-        const uint32_t b = gp[l];
-        // top bit of dim (16k + l) sits in byte 16 + (l & 7), bit 2k + (l >> 3)
-        const uint32_t t = gp[16 + (l & 7)];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const uint32_t v = ((b >> (2 * k)) & 3u) | (((t >> (2 * k + (l >> 3))) & 1u) << 2);
-            acc = fmaf((float)v, q[g + 16 * k + l], acc);
+struct Ex64 {
+    static constexpr int kLoads = B <= 2 ? 1 : B == 3 || B == 4 ? 2 : B == 6 ? 3 : 4;
+    uint32_t r[kLoads];
+    __device__ __forceinline__ void load(const uint8_t *__restrict__ g, int l) {
+        if (B == 1) {  // bit d of the little-endian string: this lane's bits in the words' places
+            const uint2 w = *reinterpret_cast<const uint2 *>(g);
+            r[0] = ((w.x >> l) & 1u) | (((w.x >> (16 + l)) & 1u) << 1) | (((w.y >> l) & 1u) << 2) |
+                   (((w.y >> (16 + l)) & 1u) << 3);
+        } else {
+            r[0] = g[l];
+            if (B == 3) r[1] = g[16 + (l & 7)];  // top bit of dim 16k + l: bit 2k + (l >> 3)
+            if (B >= 4) r[1] = g[16 + l];
+            if (B >= 6) r[2] = g[32 + l];
+            if (B == 7) r[3] = g[48 + (l & 7)];  // as for 3 bits
+            if (B == 8) r[3] = g[48 + l];
         }
     }
-    return acc;
-}
-
-template <>
-__device__ __forceinline__ float chain_bits<4>(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int l) {
-    float acc = 0.0f;
-    for (int g = 0; g < D; g += 32) {
-        const uint32_t b = y[(g / 32) * 16 + l];
-        acc = fmaf((float)(b & 15u), q[g + l], acc);
-        acc = fmaf((float)(b >> 4), q[g + 16 + l], acc);
-    }
-    return acc;
-}
-
-template <int B>  // 6 or 7
-__device__ __forceinline__ float chain_67(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int l) {
-    float acc = 0.0f;
-    for (int g = 0; g < D; g += 64) {
-        const uint8_t *gp = y + (g / 64) * (B == 6 ? 48 : 56);
-        const uint32_t b0 = gp[l], b1 = gp[16 + l], b2 = gp[32 + l];
-        uint32_t v0 = b0 & 63u, v1 = b1 & 63u;
-        uint32_t v2 = ((b0 >> 6) << 4) | (b2 & 15u), v3 = ((b1 >> 6) << 4) | (b2 >> 4);
-        if (B == 7) {
-            const uint32_t t = gp[48 + (l & 7)];
-            const int sh = l >> 3;
-            v0 |= ((t >> (0 + sh)) & 1u) << 6;
-            v1 |= ((t >> (2 + sh)) & 1u) << 6;
-            v2 |= ((t >> (4 + sh)) & 1u) << 6;
-            v3 |= ((t >> (6 + sh)) & 1u) << 6;
+    __device__ __forceinline__ void values(int l, float (&v)[4]) const {
+        if (B == 2 || B == 3) {
+            const uint32_t t = B == 3 ? (r[kLoads - 1] >> (l >> 3)) << 2 : 0u;
+            v[0] = bits_float<0>((r[0] & 0x03u) | (t & 0x04u));
+            v[1] = bits_float<2>((r[0] & 0x0cu) | (t & 0x10u));
+            v[2] = bits_float<4>((r[0] & 0x30u) | (t & 0x40u));
+            v[3] = bits_float<6>((r[0] & 0xc0u) | (t & 0x100u));
+        } else if (B == 4) {
+            v[0] = bits_float<0>(r[0] & 0x0fu);
+            v[1] = bits_float<4>(r[0] & 0xf0u);
+            v[2] = bits_float<0>(r[kLoads - 1] & 0x0fu);
+            v[3] = bits_float<4>(r[kLoads - 1] & 0xf0u);
+        } else if (B == 6 || B == 7) {
+            const uint32_t b0 = r[0], b1 = r[1 % kLoads], b2 = r[2 % kLoads];
+            const uint32_t t = B == 7 ? r[kLoads - 1] >> (l >> 3) : 0u;
+            v[0] = bits_float<0>((b0 & 0x3fu) | ((t << 6) & 0x40u));
+            v[1] = bits_float<0>((b1 & 0x3fu) | ((t << 4) & 0x40u));
+            v[2] = bits_float<0>(((b0 >> 2) & 0x30u) | (b2 & 0x0fu) | ((t << 2) & 0x40u));
+            v[3] = bits_float<4>((b2 & 0xf0u) | ((b1 << 2) & 0x300u) | ((t << 4) & 0x400u));
+        } else if (B == 8) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) v[k] = bits_float<0>(r[k % kLoads]);
         }
-        acc = fmaf((float)v0, q[g + l], acc);
-        acc = fmaf((float)v1, q[g + 16 + l], acc);
-        acc = fmaf((float)v2, q[g + 32 + l], acc);
-        acc = fmaf((float)v3, q[g + 48 + l], acc);
     }
-    return acc;
-}
+    __device__ __forceinline__ void add(int l, const float4 &q, float &acc) const {
+        if (B == 1) {  // masked adds
+            acc = __fadd_rn(acc, (r[0] & 1u) ? q.x : 0.0f);
+            acc = __fadd_rn(acc, (r[0] & 2u) ? q.y : 0.0f);
+            acc = __fadd_rn(acc, (r[0] & 4u) ? q.z : 0.0f);
+            acc = __fadd_rn(acc, (r[0] & 8u) ? q.w : 0.0f);
+        } else {
+            float v[4];
+            values(l, v);
+            acc = fmaf(v[0], q.x, acc);
+            acc = fmaf(v[1], q.y, acc);
+            acc = fmaf(v[2], q.z, acc);
+            acc = fmaf(v[3], q.w, acc);
+        }
+    }
+};
 
-template <>
-__device__ __forceinline__ float chain_bits<6>(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int l) {
-    return chain_67<6>(q, y, D, l);
-}
-template <>
-__device__ __forceinline__ float chain_bits<7>(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int l) {
-    return chain_67<7>(q, y, D, l);
-}
-
-template <>
-__device__ __forceinline__ float chain_bits<8>(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int l) {
+// Every lane of the warp takes part (both halves with the same D); the half's
+// result is valid in its lane 0.  Four groups' codes are loaded ahead of their
+// chain: the chain of a lane is D / 16 FMAs, and a load per step would wait D / 64
+// times.
+template <int B>
+__device__ __forceinline__ float ip16_bits(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int l) {
+    const float4 *q4 = reinterpret_cast<const float4 *>(q) + l;
+    const int G = D / 64;
     float acc = 0.0f;
-    for (int d = l; d < D; d += 16) acc = fmaf((float)y[d], q[d], acc);
-    return acc;
+    int g = 0;
+    for (; g + 4 <= G; g += 4) {
+        Ex64<B> e[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) e[u].load(y + (g + u) * 8 * B, l);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) e[u].add(l, q4[(g + u) * 16], acc);
+    }
+    for (; g < G; ++g) {
+        Ex64<B> e;
+        e.load(y + g * 8 * B, l);
+        e.add(l, q4[g * 16], acc);
+    }
+    return half_reduce16(acc, kFull);
 }
 
-// IP of a code of at most 8 bits, reduced over the half-warp (valid in lane 0).
-__device__ __forceinline__ float ip8_half(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int bits,
-                                          int l, unsigned mask) {
+__device__ __forceinline__ float ip16_8(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int bits, int l) {
     switch (bits) {
     case 1:
-        return half_reduce16(chain_bits<1>(q, y, D, l), mask);
+        return ip16_bits<1>(q, y, D, l);
     case 2:
-        return half_reduce16(chain_bits<2>(q, y, D, l), mask);
+        return ip16_bits<2>(q, y, D, l);
     case 3:
-        return half_reduce16(chain_bits<3>(q, y, D, l), mask);
+        return ip16_bits<3>(q, y, D, l);
     case 4:
-        return half_reduce16(chain_bits<4>(q, y, D, l), mask);
+        return ip16_bits<4>(q, y, D, l);
     case 5: {  // CodeHelper<5>::compute_ip = 2 * IP4(top 4 bits) + IP1(low bit)
-        const float a = half_reduce16(chain_bits<4>(q, y, D, l), mask);
-        const float b = half_reduce16(chain_bits<1>(q, y + D / 2, D, l), mask);
+        const float a = ip16_bits<4>(q, y, D, l);
+        const float b = ip16_bits<1>(q, y + D / 2, D, l);
         return __fadd_rn(2.0f * a, b);
     }
     case 6:
-        return half_reduce16(chain_bits<6>(q, y, D, l), mask);
+        return ip16_bits<6>(q, y, D, l);
     case 7:
-        return half_reduce16(chain_bits<7>(q, y, D, l), mask);
+        return ip16_bits<7>(q, y, D, l);
     case 8:
-        return half_reduce16(chain_bits<8>(q, y, D, l), mask);
+        return ip16_bits<8>(q, y, D, l);
     default:
         return 0.0f;
     }
 }
 
-// get_IP_FUNC(ex_bits)(q, y, D) (code_helper.hpp:599-640) computed by a
-// half-warp; result valid in the half's lane 0.
-__device__ __forceinline__ float excode_ip_half(const float *__restrict__ q, const uint8_t *__restrict__ y, int D,
-                                                int exb, int l, unsigned mask) {
-    if (exb == 0) return 0.0f;
-    if (exb > 8) {  // CodeHelper<B>::compute_ip, B > 8: IP8(low bytes) + 256 * IP(rest)
-        const float lo = ip8_half(q, y, D, 8, l, mask);
-        const float hi = ip8_half(q, y + D, D, exb - 8, l, mask);
-        return __fadd_rn(lo, 256.0f * hi);
-    }
-    return ip8_half(q, y, D, exb, l, mask);
+// get_IP_FUNC(ex_bits)(q, y, D) (code_helper.hpp:599-640) by half-warps, q in ex
+// order.  One copy per kernel: the callers' loops are short beside it.
+static __device__ __noinline__ float excode_ip16(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int exb) {
+    const int l = threadIdx.x & 15;
+    if (exb > 8)  // CodeHelper<B>::compute_ip, B > 8: IP8(low bytes) + 256 * IP(rest)
+        return __fadd_rn(ip16_bits<8>(q, y, D, l), 256.0f * ip16_8(q, y + D, D, exb - 8, l));
+    return ip16_8(q, y, D, exb, l);
 }
 
 // ---- the same inner products computed by ONE thread: the 16 SIMD lanes of
 // CodeHelper<B>::compute_ip become 16 independent accumulators (lane l takes
 // dims l, l+16, ... in increasing order), reduced with the same 16->1 tree.
-// Bit-identical to the half-warp form; used where many candidate vectors are
-// re-ranked at once (one thread per vector and segment).
+// Bit-identical to the half-warp form, about half its instructions per vector (no
+// reduction across lanes) but its whole length in one thread: used where many
+// candidate vectors are re-ranked at once (one thread per vector and segment).
+// The query is in ex order here too.
 __device__ __forceinline__ float tree16(const float *a) {
     float x[8], y[4];
 #pragma unroll
@@ -241,78 +240,48 @@ __device__ __forceinline__ float ip_thread_bits(const float *__restrict__ q, con
     float acc[16];
 #pragma unroll
     for (int l = 0; l < 16; ++l) acc[l] = 0.0f;
-    if (B == 1) {
-        for (int g = 0; g < D; g += 16) {
-            const uint32_t m = (uint32_t)y[g / 8] | ((uint32_t)y[g / 8 + 1] << 8);
+    uint32_t nxt[2 * B];  // a group's 8 B bytes (groups of odd widths are 8-byte aligned)
+    auto fetch = [&](int g) {
+        const uint8_t *gp = y + g * 8 * B;
+        if (B % 2 == 0) {
 #pragma unroll
-            for (int l = 0; l < 16; ++l) acc[l] = __fadd_rn(acc[l], ((m >> l) & 1u) ? q[g + l] : 0.0f);
-        }
-    } else if (B == 2 || B == 3) {
-        for (int g = 0; g < D; g += 64) {
-            const uint8_t *gp = y + (g / 64) * (B == 2 ? 16 : 24);
-            // 16 low-bit bytes; 3-bit groups are 24 bytes, so only 8-byte alignment is guaranteed
-            const uint2 w0 = *reinterpret_cast<const uint2 *>(gp), w1 = *reinterpret_cast<const uint2 *>(gp + 8);
-            const uint32_t wv[4] = {w0.x, w0.y, w1.x, w1.y};
-            uint2 tt = make_uint2(0, 0);
-            if (B == 3) tt = *reinterpret_cast<const uint2 *>(gp + 16);
-            const uint32_t tv[2] = {tt.x, tt.y};
+            for (int i = 0; i < B / 2; ++i) {
+                const uint4 v = reinterpret_cast<const uint4 *>(gp)[i];
+                nxt[4 * i] = v.x, nxt[4 * i + 1] = v.y, nxt[4 * i + 2] = v.z, nxt[4 * i + 3] = v.w;
+            }
+        } else {
 #pragma unroll
-            for (int l = 0; l < 16; ++l) {
-                const uint32_t b = (wv[l >> 2] >> (8 * (l & 3))) & 255u;
-                const uint32_t t = (tv[(l & 7) >> 2] >> (8 * (l & 3))) & 255u;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    uint32_t v = (b >> (2 * k)) & 3u;
-                    if (B == 3) v |= ((t >> (2 * k + (l >> 3))) & 1u) << 2;
-                    acc[l] = fmaf((float)v, q[g + 16 * k + l], acc[l]);
-                }
+            for (int i = 0; i < B; ++i) {
+                const uint2 v = reinterpret_cast<const uint2 *>(gp)[i];
+                nxt[2 * i] = v.x, nxt[2 * i + 1] = v.y;
             }
         }
-    } else if (B == 4) {
-        for (int g = 0; g < D; g += 32) {
-            const uint4 w = *reinterpret_cast<const uint4 *>(y + (g / 32) * 16);
-            const uint32_t wv[4] = {w.x, w.y, w.z, w.w};
+    };
+    constexpr bool kAhead = B <= 4;  // the next group's words in flight (wider codes: too many registers)
+    if (kAhead) fetch(0);
+    for (int g = 0; g < D / 64; ++g) {
+        if (!kAhead) fetch(g);
+        uint32_t w[2 * B];
 #pragma unroll
-            for (int l = 0; l < 16; ++l) {
-                const uint32_t b = (wv[l >> 2] >> (8 * (l & 3))) & 255u;
-                acc[l] = fmaf((float)(b & 15u), q[g + l], acc[l]);
-                acc[l] = fmaf((float)(b >> 4), q[g + 16 + l], acc[l]);
-            }
-        }
-    } else if (B == 6 || B == 7) {
-        for (int g = 0; g < D; g += 64) {
-            const uint8_t *gp = y + (g / 64) * (B == 6 ? 48 : 56);
-            uint32_t tv[2] = {0, 0};
-            if (B == 7) {
-                const uint2 tt = *reinterpret_cast<const uint2 *>(gp + 48);
-                tv[0] = tt.x;
-                tv[1] = tt.y;
-            }
+        for (int i = 0; i < 2 * B; ++i) w[i] = nxt[i];
+        if (kAhead && g + 1 < D / 64) fetch(g + 1);
+        auto byte = [&](int i) { return __byte_perm(w[(i >> 2) % (2 * B)], 0u, 0x4440u | (i & 3)); };
+        const float4 *q4 = reinterpret_cast<const float4 *>(q + 64 * g);
 #pragma unroll
-            for (int l = 0; l < 16; ++l) {
-                const uint32_t b0 = gp[l], b1 = gp[16 + l], b2 = gp[32 + l];
-                uint32_t v0 = b0 & 63u, v1 = b1 & 63u;
-                uint32_t v2 = ((b0 >> 6) << 4) | (b2 & 15u), v3 = ((b1 >> 6) << 4) | (b2 >> 4);
-                if (B == 7) {
-                    const uint32_t t = (tv[(l & 7) >> 2] >> (8 * (l & 3))) & 255u;
-                    const int sh = l >> 3;
-                    v0 |= ((t >> (0 + sh)) & 1u) << 6;
-                    v1 |= ((t >> (2 + sh)) & 1u) << 6;
-                    v2 |= ((t >> (4 + sh)) & 1u) << 6;
-                    v3 |= ((t >> (6 + sh)) & 1u) << 6;
-                }
-                acc[l] = fmaf((float)v0, q[g + l], acc[l]);
-                acc[l] = fmaf((float)v1, q[g + 16 + l], acc[l]);
-                acc[l] = fmaf((float)v2, q[g + 32 + l], acc[l]);
-                acc[l] = fmaf((float)v3, q[g + 48 + l], acc[l]);
+        for (int l = 0; l < 16; ++l) {  // what SIMD lane l reads, as Ex64::load
+            Ex64<B> e;
+            if (B == 1) {
+                e.r[0] = ((w[0] >> l) & 1u) | (((w[0] >> (16 + l)) & 1u) << 1) | (((w[1] >> l) & 1u) << 2) |
+                         (((w[1] >> (16 + l)) & 1u) << 3);
+            } else {
+                e.r[0] = byte(l);
+                if (B == 3) e.r[1] = byte(16 + (l & 7));
+                if (B >= 4) e.r[1] = byte(16 + l);
+                if (B >= 6) e.r[2] = byte(32 + l);
+                if (B == 7) e.r[3] = byte(48 + (l & 7));
+                if (B == 8) e.r[3] = byte(48 + l);
             }
-        }
-    } else {  // 8
-        for (int g = 0; g < D; g += 16) {
-            const uint4 w = *reinterpret_cast<const uint4 *>(y + g);
-            const uint32_t wv[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-            for (int l = 0; l < 16; ++l) acc[l] = fmaf((float)((wv[l >> 2] >> (8 * (l & 3))) & 255u), q[g + l], acc[l]);
+            e.add(l, q4[l], acc[l]);
         }
     }
     return tree16(acc);
@@ -342,146 +311,11 @@ __device__ __forceinline__ float ip8_thread(const float *__restrict__ q, const u
 }
 
 // get_IP_FUNC(ex_bits)(q, y, D) by one thread.
-__device__ __forceinline__ float excode_ip_thread(const float *__restrict__ q, const uint8_t *__restrict__ y, int D,
-                                                  int exb) {
+static __device__ __noinline__ float excode_ip_thread(const float *__restrict__ q, const uint8_t *__restrict__ y, int D,
+                                                      int exb) {
     if (exb == 0) return 0.0f;
     if (exb > 8) return __fadd_rn(ip8_thread(q, y, D, 8), 256.0f * ip8_thread(q, y + D, D, exb - 8));
     return ip8_thread(q, y, D, exb);
-}
-
-// ---- the same inner products by four lanes: lane j of an aligned group of
-// four keeps the SIMD accumulators 4j .. 4j+3 of ip_thread_bits, reading the
-// same words, and the group combines them with tree16's pairing (i with i + 8
-// and i + 4 across lanes, then (0 + 2) + (1 + 3) in lane 0).  Bit-identical to
-// the one-thread form, a quarter of its chain; valid in the group's lane 0.
-__device__ __forceinline__ uint32_t pick4(uint32_t a, uint32_t b, uint32_t c, uint32_t d, int j) {
-    return j == 0 ? a : j == 1 ? b : j == 2 ? c : d;
-}
-
-template <int B>
-__device__ __forceinline__ float ip_quad_bits(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int j) {
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    const int l0 = 4 * j;
-    if (B == 1) {
-        for (int g = 0; g < D; g += 16) {
-            const uint32_t m = (uint32_t)y[g / 8] | ((uint32_t)y[g / 8 + 1] << 8);
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-                const int l = l0 + jj;
-                acc[jj] = __fadd_rn(acc[jj], ((m >> l) & 1u) ? q[g + l] : 0.0f);
-            }
-        }
-    } else if (B == 2 || B == 3) {
-        for (int g = 0; g < D; g += 64) {
-            const uint8_t *gp = y + (g / 64) * (B == 2 ? 16 : 24);
-            const uint2 w0 = *reinterpret_cast<const uint2 *>(gp), w1 = *reinterpret_cast<const uint2 *>(gp + 8);
-            const uint32_t w = pick4(w0.x, w0.y, w1.x, w1.y, j);
-            uint32_t tw = 0;
-            if (B == 3) {
-                const uint2 tt = *reinterpret_cast<const uint2 *>(gp + 16);
-                tw = (j & 1) ? tt.y : tt.x;  // word (l & 7) >> 2 of the top bits
-            }
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-                const int l = l0 + jj;
-                const uint32_t b = (w >> (8 * jj)) & 255u;
-                const uint32_t t = (tw >> (8 * jj)) & 255u;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    uint32_t v = (b >> (2 * k)) & 3u;
-                    if (B == 3) v |= ((t >> (2 * k + (l >> 3))) & 1u) << 2;
-                    acc[jj] = fmaf((float)v, q[g + 16 * k + l], acc[jj]);
-                }
-            }
-        }
-    } else if (B == 4) {
-        for (int g = 0; g < D; g += 32) {
-            const uint4 w4 = *reinterpret_cast<const uint4 *>(y + (g / 32) * 16);
-            const uint32_t w = pick4(w4.x, w4.y, w4.z, w4.w, j);
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-                const int l = l0 + jj;
-                const uint32_t b = (w >> (8 * jj)) & 255u;
-                acc[jj] = fmaf((float)(b & 15u), q[g + l], acc[jj]);
-                acc[jj] = fmaf((float)(b >> 4), q[g + 16 + l], acc[jj]);
-            }
-        }
-    } else if (B == 6 || B == 7) {
-        for (int g = 0; g < D; g += 64) {
-            const uint8_t *gp = y + (g / 64) * (B == 6 ? 48 : 56);
-            uint32_t tw = 0;
-            if (B == 7) {
-                const uint2 tt = *reinterpret_cast<const uint2 *>(gp + 48);
-                tw = (j & 1) ? tt.y : tt.x;
-            }
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-                const int l = l0 + jj;
-                const uint32_t b0 = gp[l], b1 = gp[16 + l], b2 = gp[32 + l];
-                uint32_t v0 = b0 & 63u, v1 = b1 & 63u;
-                uint32_t v2 = ((b0 >> 6) << 4) | (b2 & 15u), v3 = ((b1 >> 6) << 4) | (b2 >> 4);
-                if (B == 7) {
-                    const uint32_t t = (tw >> (8 * jj)) & 255u;
-                    const int sh = l >> 3;
-                    v0 |= ((t >> (0 + sh)) & 1u) << 6;
-                    v1 |= ((t >> (2 + sh)) & 1u) << 6;
-                    v2 |= ((t >> (4 + sh)) & 1u) << 6;
-                    v3 |= ((t >> (6 + sh)) & 1u) << 6;
-                }
-                acc[jj] = fmaf((float)v0, q[g + l], acc[jj]);
-                acc[jj] = fmaf((float)v1, q[g + 16 + l], acc[jj]);
-                acc[jj] = fmaf((float)v2, q[g + 32 + l], acc[jj]);
-                acc[jj] = fmaf((float)v3, q[g + 48 + l], acc[jj]);
-            }
-        }
-    } else {  // 8
-        for (int g = 0; g < D; g += 16) {
-            const uint4 w4 = *reinterpret_cast<const uint4 *>(y + g);
-            const uint32_t w = pick4(w4.x, w4.y, w4.z, w4.w, j);
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) acc[jj] = fmaf((float)((w >> (8 * jj)) & 255u), q[g + l0 + jj], acc[jj]);
-        }
-    }
-    // tree16: x[i] = a[i] + a[i + 8] (lanes 0, 1 with lanes 2, 3), y[i] = x[i] + x[i + 4]
-    // (lane 0 with lane 1), then (y0 + y2) + (y1 + y3)
-#pragma unroll
-    for (int jj = 0; jj < 4; ++jj) acc[jj] = __fadd_rn(acc[jj], __shfl_down_sync(kFull, acc[jj], 2, 4));
-#pragma unroll
-    for (int jj = 0; jj < 4; ++jj) acc[jj] = __fadd_rn(acc[jj], __shfl_down_sync(kFull, acc[jj], 1, 4));
-    return __fadd_rn(__fadd_rn(acc[0], acc[2]), __fadd_rn(acc[1], acc[3]));
-}
-
-__device__ __forceinline__ float ip8_quad(const float *__restrict__ q, const uint8_t *__restrict__ y, int D, int bits,
-                                          int j) {
-    switch (bits) {
-    case 1:
-        return ip_quad_bits<1>(q, y, D, j);
-    case 2:
-        return ip_quad_bits<2>(q, y, D, j);
-    case 3:
-        return ip_quad_bits<3>(q, y, D, j);
-    case 4:
-        return ip_quad_bits<4>(q, y, D, j);
-    case 5:  // CodeHelper<5>::compute_ip = 2 * IP4(top 4 bits) + IP1(low bit)
-        return __fadd_rn(2.0f * ip_quad_bits<4>(q, y, D, j), ip_quad_bits<1>(q, y + D / 2, D, j));
-    case 6:
-        return ip_quad_bits<6>(q, y, D, j);
-    case 7:
-        return ip_quad_bits<7>(q, y, D, j);
-    case 8:
-        return ip_quad_bits<8>(q, y, D, j);
-    default:
-        return 0.0f;
-    }
-}
-
-// get_IP_FUNC(ex_bits)(q, y, D) by an aligned group of four lanes (j = lane & 3;
-// every lane of the warp takes part); valid in the group's lane 0.
-__device__ __forceinline__ float excode_ip_quad(const float *__restrict__ q, const uint8_t *__restrict__ y, int D,
-                                                int exb, int j) {
-    if (exb == 0) return 0.0f;
-    if (exb > 8) return __fadd_rn(ip8_quad(q, y, D, 8, j), 256.0f * ip8_quad(q, y + D, D, exb - 8, j));
-    return ip8_quad(q, y, D, exb, j);
 }
 
 // CaqCluEstimator::compAccurateDist + Lut::getExtIP, L2 (caq_estimator.hpp:190-217, lut.hpp:121-126)

@@ -10,13 +10,14 @@
 //                  per segment: zero-padded query slice, prune bound
 //                  sqrt(sum var*q^2)*m and the rotated query q_s*P_s in Eigen's
 //                  GEMV order (saq_estimator.hpp:28-48, caq_estimator.hpp:56-68)
-//   k_scan         one CTA per query walks its probes in order.  Per cluster:
-//                  LUTs (Lut::prepare, lut.hpp:60-87); per tile of blocks
-//                  (one warp = one 32-vector block): FastScan sums and fast /
+//   k_scan         one CTA per query walks its probes in order: 128 blocks at a
+//                  time are filtered by the first pruning stage; of the rest, per
+//                  cluster the LUTs (Lut::prepare, lut.hpp:60-87) and per tile of
+//                  blocks (one warp = one 32-vector block) FastScan sums and fast /
 //                  variance estimates, the block's pruning stages, accurate
 //                  distances of every lane that can pass under the tile-start
 //                  distk (distk only shrinks, so this is a superset), then one
-//                  thread replays SAQSearcher::searchCluster / scanCluster
+//                  warp replays SAQSearcher::searchCluster / scanCluster
 //                  (saq_searcher.hpp:68-214) and the ResultPool inserts
 //                  (utils/pool.hpp:17-30) exactly in the reference's order.
 #include <cfloat>
@@ -42,6 +43,7 @@ constexpr int kScanThreads = kScanWarps * 32;
 constexpr int kBlocksPerWarp = 2;
 constexpr int kTileB = kScanWarps * kBlocksPerWarp;  // blocks per tile
 constexpr int kMaxTopK = 4096;
+constexpr int kItemCands = 16;  // candidates of a tile up to which half-warps take the accurate distances
 constexpr int kScanMinCtas = 4;  // resident scan CTAs per SM the register budget is sized for
 
 struct SegScal {
@@ -840,6 +842,7 @@ struct ScanSmem {
     float *cd, *ipx, *part, *cur, *stage;
     uint32_t *cmask;
     int *nstage;
+    int *sblk;        // block of the cluster in each slot of the tile
     uint32_t *pool_id;
     float *pool_d;
     uint32_t *mm;     // per segment LUT min / max keys
@@ -860,7 +863,7 @@ __host__ __device__ inline size_t scan_smem_bytes(int Dtot, int S, int topk, int
     b += align16(sizeof(float) * kTileB * 32);          // cur
     b += align16(sizeof(float) * kTileB * (S + 1));     // stage minima
     b += align16(sizeof(uint32_t) * kTileB);
-    b += align16(sizeof(int) * kTileB);
+    b += 2 * align16(sizeof(int) * kTileB);             // nstage, sblk
     b += align16(sizeof(uint32_t) * (topk + 1));
     b += align16(sizeof(float) * (topk + 1));
     return b;
@@ -896,6 +899,8 @@ __device__ ScanSmem scan_smem_layout(char *base, int Dtot, int S, int topk, int 
     s.cmask = (uint32_t *)(base + o);
     o += align16(sizeof(uint32_t) * kTileB);
     s.nstage = (int *)(base + o);
+    o += align16(sizeof(int) * kTileB);
+    s.sblk = (int *)(base + o);
     o += align16(sizeof(int) * kTileB);
     s.pool_id = (uint32_t *)(base + o);
     o += align16(sizeof(uint32_t) * (topk + 1));
@@ -976,10 +981,21 @@ __device__ __forceinline__ void codebook_keys(const float *qq, uint32_t &kmin, u
     kmax = fkey(hi);
 }
 
+// One group of 64 residuals into ex order, by a whole warp.
+__device__ __forceinline__ void ex_reorder(float *x) {
+    const int lane = threadIdx.x & 31;
+    const float a = x[lane], b = x[lane + 32];
+    __syncwarp();
+    x[ex_order(lane)] = a;
+    x[ex_order(lane + 32)] = b;
+    __syncwarp();
+}
+
 // Lut::prepare (lut.hpp:60-87) for every segment of cluster c, spread over the
 // whole CTA: residual query, its Eigen-order sum and squared norm, the float
 // LUT's min / max, delta = (max-min)/(65536-0.01) in double, the u16 LUT
 // trunc((entry-min)/delta), and the epilogue constants of compFastIP.
+// Leaves the residual query in ex order (see excode_ip16).
 // t_first > 0: only threads [t_first, blockDim.x) take part (whole warps),
 // synchronising on named barrier `bar` instead of __syncthreads.
 __device__ void prepare_cluster(const DevIndexView &ix, const float *__restrict__ qrot, const float *__restrict__ prune,
@@ -1043,6 +1059,8 @@ __device__ void prepare_cluster(const DevIndexView &ix, const float *__restrict_
         const SegScal &sc = sm.scal[s];
         quant_codebook(sm.qres + cb * 4, sc.vl, sc.delta, sc.rdelta, sm.lut + cb * 16);
     }
+    sync();
+    for (int g = warp; g < ix.Dtot / 64; g += nt / 32) ex_reorder(sm.qres + 64 * g);
     sync();
 }
 
@@ -1138,7 +1156,7 @@ __global__ void __launch_bounds__(kLutWarps * 32) k_lut(DevIndexView ix, const u
 }
 
 // The prepared state of cluster c from k_lut's output (lut / scal: this
-// pair's), and the residual query, into the CTA's shared memory.
+// pair's), and the residual query in ex order, into the CTA's shared memory.
 __device__ void load_cluster(const DevIndexView &ix, const float *__restrict__ qrot, const uint16_t *__restrict__ lut,
                              const SegScal *__restrict__ scal, int c, ScanSmem &sm) {
     const int tid = threadIdx.x, nt = blockDim.x;
@@ -1149,7 +1167,7 @@ __device__ void load_cluster(const DevIndexView &ix, const float *__restrict__ q
     for (int s = 0; s < ix.S; ++s) {
         const SegDev &g = ix.seg[s];
         const float *cent = g.cent + (size_t)c * g.dim;
-        for (int i = tid; i < g.dim; i += nt) sm.qres[g.qoff + i] = __fsub_rn(qrot[g.qoff + i], cent[i]);
+        for (int i = tid; i < g.dim; i += nt) sm.qres[g.qoff + ex_order(i)] = __fsub_rn(qrot[g.qoff + i], cent[i]);
     }
     __syncthreads();
 }
@@ -1164,19 +1182,64 @@ __device__ __forceinline__ float block_min(float cur) {
     return warp_min_tree(cur);
 }
 
-// Pulls cluster c's rotated centroid rows (every segment, 4 * Dtot bytes) into
-// L2 ahead of its prepare_cluster: thread tid of nt takes the 128-byte lines
-// tid, tid + nt, ... of the rows laid end to end.
-__device__ __forceinline__ void prefetch_centroid(const DevIndexView &ix, int c, int tid, int nt) {
-    for (int s = 0, first = 0; s < ix.S; ++s) {
-        const SegDev &g = ix.seg[s];
-        const char *row = reinterpret_cast<const char *>(g.cent + (size_t)c * g.dim);
-        const int lines = (4 * g.dim + 127) / 128;
-        int l = tid - first;  // first line of this row that is the thread's
-        if (l < 0) l += (-l + nt - 1) / nt * nt;
-        for (; l < lines; l += nt) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + 128 * l));
-        first += lines;
+// Stage 0 of SAQSearcher::searchCluster (saq_searcher.hpp:87-97) for four
+// consecutive blocks at once, by a warp: lane l takes vectors 4 (l & 7) .. + 3 of
+// block l >> 3, whose variance bounds sum in the same order as block_estimates'.
+// A block whose smallest bound exceeds `tau` (>= every distk it will meet) stops at
+// this stage and has no effect; the others come back as four bits.  Most blocks of a
+// probed cluster stop here (88% of those a 10M batch probes, 60% at nprobe up to 256),
+// and 16 bytes per lane and segment decide four of them, so the scans look at 128
+// blocks ahead and spend their tiles, LUT copies and barriers on the rest.
+// gb: first block of the four (global); nvalid: blocks of them that exist; vf: the
+// segments' q_l2sqr - 2 prune.  A block with a NaN bound stays (its minimum depends
+// on the reference's reduction order).  U groups of four at a time, for more loads in
+// flight.
+constexpr int kQuad = 4;
+template <int U>
+__device__ __forceinline__ void quad_filter(const DevIndexView &ix, const float *const (&vf)[U], const int64_t (&gb)[U],
+                                            const int (&nvalid)[U], float tau, uint32_t (&left)[U]) {
+    const int lane = threadIdx.x & 31;
+    float4 cur[U];
+#pragma unroll
+    for (int i = 0; i < U; ++i) cur[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+    for (int s = 0; s < ix.S; ++s)
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            float4 on = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if ((lane >> 3) < nvalid[i]) on = *reinterpret_cast<const float4 *>(ix.seg[s].onorm + gb[i] * 32 + 4 * lane);
+            const float v = vf[i][s];
+            cur[i].x = __fadd_rn(cur[i].x, maxps(0.0f, __fadd_rn(__fmul_rn(on.x, on.x), v)));
+            cur[i].y = __fadd_rn(cur[i].y, maxps(0.0f, __fadd_rn(__fmul_rn(on.y, on.y), v)));
+            cur[i].z = __fadd_rn(cur[i].z, maxps(0.0f, __fadd_rn(__fmul_rn(on.z, on.z), v)));
+            cur[i].w = __fadd_rn(cur[i].w, maxps(0.0f, __fadd_rn(__fmul_rn(on.w, on.w), v)));
+        }
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+        // left: some vector's bound is not above tau (or is a NaN)
+        const bool keep = (lane >> 3) < nvalid[i] &&
+                          !(cur[i].x > tau && cur[i].y > tau && cur[i].z > tau && cur[i].w > tau);
+        const uint32_t b = __ballot_sync(kFull, keep);
+        left[i] = ((b & 0xffu) ? 1u : 0u) | ((b & 0xff00u) ? 2u : 0u) | ((b & 0xff0000u) ? 4u : 0u) | ((b >> 24) ? 8u : 0u);
     }
+}
+
+// q_l2sqr - 2 prune of segment s and cluster c (seg_epilogue_scalars' vfac), by a warp.
+__device__ __forceinline__ float stage0_scalar(const DevIndexView &ix, int s, int c, const float *__restrict__ qrot,
+                                               const float *__restrict__ prune) {
+    const SegDev &g = ix.seg[s];
+    const float *cent = g.cent + (size_t)c * g.dim, *q = qrot + g.qoff;
+    const float q2 = warp_eigen_sum(g.dim, [&](int i) {
+        const float r = __fsub_rn(q[i], cent[i]);
+        return __fmul_rn(r, r);
+    });
+    return __fsub_rn(q2, __fmul_rn(2.0f, prune[s]));
+}
+
+// Position of the n-th (from 0) set bit of a warp-uniform mask.
+__device__ __forceinline__ int nth_bit(uint32_t m, int n) {
+    const int lane = threadIdx.x & 31;
+    return __ffs(__ballot_sync(kFull, ((m >> lane) & 1u) && __popc(m & ((1u << lane) - 1u)) == n)) - 1;
 }
 
 // Estimates of one block (this warp, lane = vector).  Fills cd/ipx for every
@@ -1241,117 +1304,169 @@ __device__ __forceinline__ bool stages_pass(const float *st, int n, float tau) {
     return true;
 }
 
-// Steps 1-3 of a tile of up to kTileB blocks (warp w <-> blocks t0 + w + k * nwarps
-// of the cluster): estimates, candidate masks under `tau`, and the accurate
-// distances (multi-segment: accurate - estimate per segment) of every
-// candidate lane.  Ends with the partials in sm.part and the masks in sm.cmask.
-// The threads [tbase, tbase + nthr) take part (whole warps; a tile then has
-// nthr / 32 * kBlocksPerWarp slots); they synchronise on __syncthreads when
+// Steps 1-3 of a tile of ng blocks of one cluster (at most kTileB): estimates,
+// candidate masks under `tau`, and the accurate distances (multi-segment: accurate
+// - estimate per segment) of every candidate lane.  Slot i holds block blk(i) of the
+// cluster (called by whole warps, blk ascending; also left in sm.sblk).  Ends with the
+// partials in sm.part and the masks in sm.cmask.
+// The threads [tbase, tbase + nthr) take part (whole warps; a tile then has at
+// most nthr / 32 * kBlocksPerWarp slots); they synchronise on __syncthreads when
 // barid is 0, else on the named barrier barid.
-__device__ void tile_candidates(const DevIndexView &ix, ScanSmem &sm, int64_t b0, int64_t v0, int nb, int n, int t0,
-                                int t_end, float tau, int tbase = 0, int nthr = kScanThreads, int barid = 0) {
+template <class Blk>
+__device__ __forceinline__ void tile_candidates(const DevIndexView &ix, ScanSmem &sm, int64_t b0, int64_t v0, int nb, int n, int ng,
+                                Blk blk, float tau, int tbase = 0, int nthr = kScanThreads, int barid = 0) {
     const int S = ix.S, tid = (int)threadIdx.x - tbase, w = tid >> 5, lane = tid & 31;
     const int nwarps = nthr >> 5, nslots = nwarps * kBlocksPerWarp;
     auto sync = [&]() {
         if (barid) asm volatile("bar.sync %0, %1;" ::"r"(barid), "r"(nthr) : "memory");
         else __syncthreads();
     };
-#pragma unroll
-    for (int k = 0; k < kBlocksPerWarp; ++k) {
-        const int slot = w + k * nwarps, b = t0 + slot;
-        if (b < t_end) block_estimates(ix, b0 + b, sm, slot, lane, tau);
-    }
-    // a slot's mask reads only what the same warp's estimates wrote (its cd,
-    // cur, stage and nstage rows): a warp barrier orders them
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < kBlocksPerWarp; ++k) {
-        const int slot = w + k * nwarps, b = t0 + slot;
-        if (b < t_end) {
-            bool cand;
-            if (S == 1) {
-                const int cnp = (b == nb - 1) ? (n % 32) : 32;  // scanCluster's last-block count (saq_searcher.hpp:186)
-                cand = lane < cnp && sm.cd[slot * 32 + lane] < tau;
-            } else {
-                cand = stages_pass(sm.stage + slot * (S + 1), sm.nstage[slot], tau) && sm.cur[slot * 32 + lane] < tau &&
-                       (b * 32 + lane) < n;
+    // pull a block's codes into L1, a line of 128 bytes per lane at a time
+    auto pull_codes = [&](int b) {
+        for (int s = 0; s < S; ++s) {
+            const SegDev &g = ix.seg[s];
+            const int lines = g.bits ? g.dim / 64 * 2 : 0;
+            const char *p = reinterpret_cast<const char *>(g.codes) + (size_t)(b0 + b) * lines * 128;
+            for (int l = lane; l < lines; l += 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(p + l * 128));
+        }
+    };
+    if (w < ng) pull_codes(blk(w));
+#pragma unroll 1
+    for (int slot = w; slot < nslots; slot += nwarps) {
+        if (slot >= ng) {
+            if (lane == 0) sm.cmask[slot] = 0;
+            continue;
+        }
+        const int b = blk(slot);
+        if (slot + nwarps < ng) pull_codes(blk(slot + nwarps));
+        block_estimates(ix, b0 + b, sm, slot, lane, tau);
+        // the mask reads only what this warp's estimates wrote (the slot's cd, cur,
+        // stage and nstage rows): a warp barrier orders them
+        __syncwarp();
+        bool cand;
+        if (S == 1) {
+            const int cnp = (b == nb - 1) ? (n % 32) : 32;  // scanCluster's last-block count (saq_searcher.hpp:186)
+            cand = lane < cnp && sm.cd[slot * 32 + lane] < tau;
+        } else {
+            cand = stages_pass(sm.stage + slot * (S + 1), sm.nstage[slot], tau) && sm.cur[slot * 32 + lane] < tau &&
+                   (b * 32 + lane) < n;
+        }
+        const uint32_t m = __ballot_sync(kFull, cand);
+        if (lane == 0) {
+            sm.cmask[slot] = m;
+            sm.sblk[slot] = b;
+        }
+        if (cand) {  // pull the candidate's ex-code rows, factors and id into L1 ahead of their use
+            const int64_t gv = v0 + (int64_t)b * 32 + lane;
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(ix.ids + gv));
+            for (int s = 0; s < S; ++s) {
+                const SegDev &g = ix.seg[s];
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(g.exfac + gv));
+                if (g.bits > 1) {
+                    const uint8_t *row = g.lcode + (size_t)gv * g.lstride;
+                    for (int o = 0; o < g.lstride; o += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(row + o));
+                }
             }
-            const uint32_t m = __ballot_sync(kFull, cand);
-            if (lane == 0) sm.cmask[slot] = m;
-        } else if (lane == 0) {
-            sm.cmask[slot] = 0;
         }
     }
     sync();
-    // accurate distances: one thread per (candidate vector, segment); the
-    // tasks of a segment start on a warp boundary, so a warp's lanes run the
-    // same code (one ex-code width and length) instead of diverging over all
-    int ncand = 0;
-    for (int i = 0; i < nslots; ++i) ncand += __popc(sm.cmask[i]);
-    const int P = (ncand + 31) & ~31;
-    const int total = S * P;
-    auto decode = [&](int r, int &ww, int &j) {
-        ww = 0;
-        while (r >= __popc(sm.cmask[ww])) {
-            r -= __popc(sm.cmask[ww]);
-            ++ww;
-        }
-        uint32_t mk = sm.cmask[ww];
-        for (int i = 0; i < r; ++i) mk &= mk - 1;
-        j = __ffs(mk) - 1;
-    };
-    // first pull every task's ex-code row into L1, so the chains below do not
-    // wait on memory group by group
-    for (int t = tid; t < total; t += nthr) {
-        const int s = t / P, r = t - s * P;
-        if (r >= ncand) continue;
-        int ww, j;
-        decode(r, ww, j);
-        const SegDev &g = ix.seg[s];
-        if (g.bits > 1) {
-            const uint8_t *row = g.lcode + (size_t)(v0 + (int64_t)(t0 + ww) * 32 + j) * g.lstride;
-            for (int o = 0; o < g.lstride; o += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(row + o));
-        }
+    // Accurate distances.  Few candidates (at most kItemCands): work items of two
+    // candidates of one segment, a half-warp each (excode_ip16), the widest segments
+    // first; a warp takes every nwarps-th.  More: one thread per (candidate, segment)
+    // (excode_ip_thread), the tasks of a segment from a warp boundary on, which takes
+    // half the instructions.  The line lies where the two
+    // cross: 256 queries of 1,536 dimensions (about 13 candidates a tile) take 1.67 ms
+    // with half-warps up to 16 candidates and 2.51 without, 37 queries with k = 100
+    // (about 75) 4.04 ms without and 4.65 with half-warps up to 96.
+    // The FP64 step of the distance (accurate_dist) would cost a warp's issue for two
+    // lanes, so lane 2i, 2i + 1 keep the products of the warp's i-th item and up to 32
+    // of them take that step together.
+    const uint32_t my_mask = lane < nslots ? sm.cmask[lane] : 0u;  // lane i: slot i
+    int incl = __popc(my_mask);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += y;
     }
-    auto finish = [&](int s, int ww, int j, float ex) {
-        const int64_t gb = b0 + t0 + ww, gv = v0 + (int64_t)(t0 + ww) * 32 + j;
-        const SegDev &g = ix.seg[s];
-        const SegScal &sc = sm.scal[s];
-        const float acc = accurate_dist(g.onorm[gb * 32 + j], sm.ipx[(ww * S + s) * 32 + j], ex, g.exfac[gv].x, g.bits,
-                                        sc.sum_q, sc.q_l2sqr);
-        sm.part[(ww * S + s) * 32 + j] = S == 1 ? acc : __fsub_rn(acc, sm.cd[(ww * S + s) * 32 + j]);
+    const int ncand = __shfl_sync(kFull, incl, 31);
+    // the r-th candidate of the tile, as slot * 32 + lane of its block
+    auto locate = [&](int r) {
+        const int slot = __popc(__ballot_sync(kFull, incl <= r));  // lanes past the last slot hold ncand > r
+        const uint32_t m = __shfl_sync(kFull, my_mask, slot);
+        const int nth = r - (__shfl_sync(kFull, incl, slot) - __popc(m));
+        const uint32_t hit = __ballot_sync(kFull, ((m >> lane) & 1u) && __popc(m & ((1u << lane) - 1u)) == nth);
+        return slot * 32 + __ffs(hit) - 1;
     };
-    // few tasks: four lanes per task (excode_ip_quad), a quarter of the chain;
-    // else one thread per task
-    const int P4 = (ncand + 7) & ~7;
-    if (S * P4 * 4 <= nthr) {
-        // a warp holds 8 tasks of one segment (each segment's tasks padded to a
-        // multiple of 8); padding tasks compute on candidate 0 and are discarded
-        for (int gl = tid; gl < S * P4 * 4; gl += nthr) {  // warp-uniform: a multiple of 32 lanes
-            const int t = gl >> 2, q4 = gl & 3, s = t / P4, r = t - s * P4;
-            const bool valid = r < ncand;
-            int ww, j;
-            decode(valid ? r : 0, ww, j);
-            const SegDev &g = ix.seg[s];
-            const int64_t gv = v0 + (int64_t)(t0 + ww) * 32 + j;
-            const float ex = g.bits > 1 ? excode_ip_quad(sm.qres + g.qoff, g.lcode + (size_t)gv * g.lstride, g.dim,
-                                                         g.bits - 1, q4)
-                                        : 0.0f;
-            if (valid && q4 == 0) finish(s, ww, j, ex);
+    if (ncand == 0 && !barid) return;  // the callers' next barrier orders the rest
+    auto vec_of = [&](int c) { return v0 + (int64_t)sm.sblk[c >> 5] * 32 + (c & 31); };
+    int held = 0, my_seg = -1, my_cand = 0;
+    float my_ex = 0.0f;
+    auto finish = [&]() {
+        if (my_seg >= 0) {
+            const int ww = my_cand >> 5, j = my_cand & 31;
+            const int64_t gb = b0 + sm.sblk[ww], gv = vec_of(my_cand);
+            const SegDev &g = ix.seg[my_seg];
+            const SegScal &sc = sm.scal[my_seg];
+            const int at = (ww * S + my_seg) * 32 + j;
+            const float acc = accurate_dist(g.onorm[gb * 32 + j], sm.ipx[at], my_ex, g.exfac[gv].x, g.bits, sc.sum_q,
+                                            sc.q_l2sqr);
+            sm.part[at] = S == 1 ? acc : __fsub_rn(acc, sm.cd[at]);
         }
-    } else {
-        for (int t = tid; t < total; t += nthr) {
-            const int s = t / P, r = t - s * P;
-            if (r >= ncand) continue;
-            int ww, j;
-            decode(r, ww, j);
-            const SegDev &g = ix.seg[s];
-            const int64_t gv = v0 + (int64_t)(t0 + ww) * 32 + j;
-            finish(s, ww, j,
-                   g.bits > 1 ? excode_ip_thread(sm.qres + g.qoff, g.lcode + (size_t)gv * g.lstride, g.dim, g.bits - 1)
-                              : 0.0f);
+        my_seg = -1;
+        held = 0;
+        __syncwarp();
+    };
+    if (ncand > kItemCands) {
+        const int P = (ncand + 31) >> 5;  // warps' worth of tasks per segment
+        for (int t = w; t < S * P; t += nwarps) {
+            const int si = t / P, r0 = (t - si * P) * 32, s = S - 1 - si;
+            // the candidates [r0, r0 + 32) of the tile, one per lane: from the slots they span
+            int c = 0;
+            {
+                const int r = min(r0 + lane, ncand - 1);
+                int slot = 0;
+#pragma unroll
+                for (int o = 8; o; o >>= 1) {  // slot: how many have incl <= r (incl ascends)
+                    const int v = __shfl_sync(kFull, incl, slot + o - 1);
+                    if (v <= r) slot += o;
+                }
+                uint32_t m = __shfl_sync(kFull, my_mask, slot);
+                for (int i = r - (__shfl_sync(kFull, incl, slot) - __popc(m)); i > 0; --i) m &= m - 1;
+                c = slot * 32 + __ffs(m) - 1;
+            }
+            if (r0 + lane < ncand) {
+                const SegDev &g = ix.seg[s];
+                my_seg = s;
+                my_cand = c;
+                my_ex = g.bits > 1 ? excode_ip_thread(sm.qres + g.qoff, g.lcode + (size_t)vec_of(c) * g.lstride, g.dim, g.bits - 1)
+                                   : 0.0f;
+            }
+            finish();
         }
+        sync();
+        return;
     }
+    const int pairs = (ncand + 1) >> 1;
+    for (int it = w; it < S * pairs; it += nwarps) {
+        const int si = it / pairs, r0 = 2 * (it - si * pairs), s = S - 1 - si;
+        const int c0 = locate(r0), c1 = locate(min(r0 + 1, ncand - 1)), c = lane < 16 ? c0 : c1;
+        const SegDev &g = ix.seg[s];
+        float ex = 0.0f;
+        if (g.bits > 1)
+            ex = excode_ip16(sm.qres + g.qoff, g.lcode + (size_t)vec_of(c) * g.lstride, g.dim, g.bits - 1);
+        const float e0 = __shfl_sync(kFull, ex, 0), e1 = __shfl_sync(kFull, ex, 16);
+        if (lane == 2 * held) {
+            my_seg = s;
+            my_cand = c0;
+            my_ex = e0;
+        } else if (lane == 2 * held + 1 && r0 + 1 < ncand) {
+            my_seg = s;
+            my_cand = c1;
+            my_ex = e1;
+        }
+        if (++held == 16) finish();
+    }
+    if (held) finish();
     sync();
 }
 
@@ -1498,16 +1613,157 @@ __device__ __forceinline__ void replay_block_warp(int S, int bb, const float *cu
     }
 }
 
+// ResultPool (utils/pool.hpp:17-49) of at most 32 kRows entries in a warp's
+// registers, entry 32 r + lane in d[r] / u[r].  An insert costs a ballot per 32
+// entries and a few shuffles, where the pool in shared memory (pool_insert_warp)
+// takes a chain of loads, stores and warp barriers.
+constexpr int kRegPool = 128;  // largest k whose pool is held so
+template <int kRows>
+struct RegPool {
+    float d[kRows], dk;
+    uint32_t u[kRows];
+    int sz, cap;
+    bool nan;  // an entry is NaN: the order is not total, replay_block_warp takes over
+    __device__ __forceinline__ void load(const uint32_t *pid, const float *pd, int size, int topk, float distk) {
+        const int lane = threadIdx.x & 31;
+        sz = size;
+        cap = topk;
+        dk = distk;
+        bool n = false;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            const int e = 32 * r + lane;
+            d[r] = e < sz ? pd[e] : 0.0f;
+            u[r] = e < sz ? pid[e] : 0u;
+            n |= d[r] != d[r];
+        }
+        nan = __any_sync(kFull, n);
+    }
+    __device__ __forceinline__ void store(uint32_t *pid, float *pd) const {
+        const int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            const int e = 32 * r + lane;
+            if (e < sz) {
+                pd[e] = d[r];
+                pid[e] = u[r];
+            }
+        }
+        __syncwarp();
+    }
+    // Inserts `dist` (uniform, no NaN, accepted under dk) and updates dk.
+    __device__ __forceinline__ void insert(uint32_t id, float dist) {
+        const int lane = threadIdx.x & 31;
+        int lo = 0;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r)
+            if (r == 0 || 32 * r < sz) lo += __popc(__ballot_sync(kFull, 32 * r + lane < sz && d[r] < dist));
+#pragma unroll
+        for (int r = kRows - 1; r >= 0; --r) {
+            if (r > 0 && (32 * r >= cap || 32 * r + 31 < lo)) continue;
+            float v = __shfl_up_sync(kFull, d[r], 1);
+            uint32_t x = __shfl_up_sync(kFull, u[r], 1);
+            if (r > 0) {
+                const float pv = __shfl_sync(kFull, d[r > 0 ? r - 1 : 0], 31);
+                const uint32_t px = __shfl_sync(kFull, u[r > 0 ? r - 1 : 0], 31);
+                if (lane == 0) {
+                    v = pv;
+                    x = px;
+                }
+            }
+            const int e = 32 * r + lane;
+            d[r] = e > lo ? v : e == lo ? dist : d[r];
+            u[r] = e > lo ? x : e == lo ? id : u[r];
+        }
+        sz += sz < cap;
+        float last = d[0];
+#pragma unroll
+        for (int r = 1; r < kRows; ++r)
+            if (r == (cap - 1) >> 5) last = d[r];
+        last = __shfl_sync(kFull, last, (cap - 1) & 31);
+        dk = sz == cap ? last : FLT_MAX;
+    }
+};
+
+// replay_block_warp on a pool in registers, for at most kRegSegs segments (ids: the
+// block's 32 ids).  A lane's running sums are formed once and stay in registers: while
+// the largest is below dk the reference's loop runs to the last one, which is
+// inserted; otherwise it ends at the first sum >= dk, which is refused under a full
+// pool unless it equals dk.  Returns false, nothing changed, when a NaN is met.
+constexpr int kRegSegs = 4;
+template <int kRows>
+__device__ __forceinline__ bool replay_block_regs(int S, const float *cur, float smax, const float *part, uint32_t cm,
+                                                  const uint32_t *ids, RegPool<kRows> &P, unsigned long long &c_rr) {
+    const int lane = threadIdx.x & 31;
+    if (!cm || (S > 1 && smax > P.dk)) return true;
+    const bool in = (cm >> lane) & 1u;
+    const uint32_t id = in ? ids[lane] : 0u;
+    const float c = in ? cur[lane] : FLT_MAX;
+    float x[kRegSegs];
+#pragma unroll
+    for (int s = 0; s < kRegSegs; ++s) x[s] = in && s < S ? part[s * 32 + lane] : 0.0f;
+    if (S == 1) {
+        const float a = in ? x[0] : FLT_MAX;
+        if (P.nan || __any_sync(kFull, a != a)) return false;
+        uint32_t rest = __ballot_sync(kFull, in && c < P.dk);  // the mask, at the block's start
+        c_rr += __popc(rest);
+        while (rest) {
+            const uint32_t ok = rest & __ballot_sync(kFull, !(P.sz == P.cap && a > P.dk));
+            if (!ok) break;
+            const int j = __ffs(ok) - 1;
+            P.insert(__shfl_sync(kFull, id, j), __shfl_sync(kFull, a, j));
+            rest &= ~((2u << j) - 1u);
+        }
+        return true;
+    }
+    float sum[kRegSegs], top, last = c;
+#pragma unroll
+    for (int s = 0; s < kRegSegs; ++s) {
+        if (s < S) last = __fadd_rn(last, x[s]);
+        sum[s] = last;  // past the last segment: the last sum again
+        top = s == 0 ? last : fmaxf(top, last);
+    }
+    bool nan = false;  // a NaN stays one in the later sums
+    nan = last != last;
+    if (P.nan || __any_sync(kFull, in && nan)) return false;
+    uint32_t rest = cm;
+    do {
+        const float dk = P.dk;
+        const bool full = P.sz == P.cap;
+        const uint32_t pass = rest & __ballot_sync(kFull, c < dk);
+        // the value the lane inserts: the last sum, or the first at or above dk
+        float acc = last;
+        bool taken = top < dk;
+        if (!taken) {
+#pragma unroll
+            for (int s = kRegSegs - 1; s >= 0; --s)
+                if (sum[s] >= dk) acc = sum[s];
+            taken = !(full && acc > dk);
+        }
+        const uint32_t ok = pass & __ballot_sync(kFull, taken);
+        if (!ok) {
+            c_rr += __popc(pass);
+            break;
+        }
+        const int j = __ffs(ok) - 1;
+        c_rr += __popc(pass & ((2u << j) - 1u));
+        P.insert(__shfl_sync(kFull, id, j), __shfl_sync(kFull, acc, j));
+        rest &= ~((2u << j) - 1u);
+    } while (rest);
+    return true;
+}
+
 // The reference's decisions for the nblk (<= 32) blocks of a tile, in order, by
 // one warp: lane i first reads block i's candidate mask and (several segments)
 // the largest of its stage minima, and a ballot keeps the blocks that can
 // change the pool under the distk at the tile's start.  distk only decreases,
 // so a block dropped here (no candidate lane, or a stage minimum above distk)
-// would be skipped by replay_block_warp as well; the rest are replayed in order.
+// would be skipped by the replay as well; the rest are replayed in order.  Slot i is
+// block sblk[i] of the cluster (sblk null: block t0 + i).
 // Returns the tile's candidate lanes (for the tally).
-__device__ __forceinline__ unsigned replay_tile_warp(int S, int t0, int nblk, const ScanSmem &v, const uint32_t *ids_v0,
-                                                     uint32_t *pid, float *pd, int &sz, int topk, float &dk,
-                                                     unsigned long long &c_rr) {
+__device__ __forceinline__ unsigned replay_tile_warp(int S, int t0, const int *sblk, int nblk, const ScanSmem &v,
+                                                     const uint32_t *ids_v0, uint32_t *pid, float *pd, int &sz, int topk,
+                                                     float &dk, unsigned long long &c_rr) {
     const int lane = threadIdx.x & 31;
     uint32_t cm = 0;
     float smax = 0.0f;
@@ -1516,12 +1772,32 @@ __device__ __forceinline__ unsigned replay_tile_warp(int S, int t0, int nblk, co
         if (S > 1 && cm) smax = stage_max(v.stage + lane * (S + 1), v.nstage[lane]);
     }
     uint32_t live = __ballot_sync(kFull, cm != 0 && !(S > 1 && smax > dk));
-    while (live) {
+    if (!live) return __reduce_add_sync(kFull, __popc(cm));
+    auto in_regs = [&](auto &P) {
+        P.load(pid, pd, sz, topk, dk);
+        while (live) {
+            const int ww = __ffs(live) - 1, bb = sblk ? sblk[ww] : t0 + ww;
+            if (!replay_block_regs(S, v.cur + ww * 32, __shfl_sync(kFull, smax, ww), v.part + ww * S * 32,
+                                   __shfl_sync(kFull, cm, ww), ids_v0 + (int64_t)bb * 32, P, c_rr))
+                break;
+            live &= live - 1;
+        }
+        P.store(pid, pd);
+        sz = P.sz;
+        dk = P.dk;
+    };
+    if (S > kRegSegs) {
+    } else if (topk <= 32) {
+        RegPool<1> P;
+        in_regs(P);
+    } else if (topk <= kRegPool) {
+        RegPool<kRegPool / 32> P;
+        in_regs(P);
+    }
+    for (; live; live &= live - 1) {  // more segments, a longer pool, or a NaN met
         const int ww = __ffs(live) - 1;
-        live &= live - 1;
-        replay_block_warp(S, t0 + ww, v.cur + ww * 32, __shfl_sync(kFull, smax, ww),
-                          S == 1 ? v.part + ww * 32 : v.part + ww * S * 32, __shfl_sync(kFull, cm, ww), ids_v0, pid, pd,
-                          sz, topk, dk, c_rr);
+        replay_block_warp(S, sblk ? sblk[ww] : t0 + ww, v.cur + ww * 32, __shfl_sync(kFull, smax, ww), v.part + ww * S * 32,
+                          __shfl_sync(kFull, cm, ww), ids_v0, pid, pd, sz, topk, dk, c_rr);
     }
     return __reduce_add_sync(kFull, __popc(cm));
 }
@@ -1530,40 +1806,143 @@ struct ScanTally {
     unsigned long long blocks = 0, vecs = 0, rr = 0, spec = 0;
 };
 
-// Exact sequential scan of probes [p_begin, p_end) of one query, continuing
-// the pool held in shared memory (pool_size / distk in shared memory).  Each
-// nonempty probed cluster's LUT comes from the batched preparation when `lut`
-// is set (this query's pairs: probe p's at lut + p * 4 * Dtot, scal + p * S),
-// else it is built here.
-__device__ void scan_probes(const DevIndexView &ix, const uint32_t *__restrict__ probe, int p_begin, int p_end,
+// Exact sequential scan of the np probes of one query, continuing the pool held
+// in shared memory (pool_size / distk in shared memory).  A probed cluster's LUT comes
+// from the batched preparation when `lut` is set (this query's pairs: probe p's at
+// lut + p * 4 * Dtot, scal + p * S), else it is built here, when a block first needs it.
+//
+// The blocks of up to kHdrProbes probes form one sequence of groups of four, in scan order.  A pass looks at kPassQuads groups (one or
+// a few until the pool is full and bounds distk: their every vector is a candidate): several segments, all warps filter them
+// by stage 0 (quad_filter) under the pass's distk, then the blocks left are taken in
+// order, up to kTileB of one cluster per tile; a probe with none left is not touched
+// any further, nor its LUT.
+constexpr int kHdrProbes = 32, kPassQuads = 32;
+struct ProbeHdr {
+    int c, nb, n, quads;
+    int64_t b0, v0;
+};
+__device__ void scan_probes(const DevIndexView &ix, const uint32_t *__restrict__ probe, int np,
                             const float *__restrict__ qrot, const float *__restrict__ prune, int topk, ScanSmem &sm,
                             int &pool_size, float &distk, ScanTally &tl, const uint16_t *__restrict__ lut,
                             const SegScal *__restrict__ scal) {
-    const int S = ix.S, tid = threadIdx.x;
-    for (int p = p_begin; p < p_end; ++p) {
-        const int c = (int)probe[p];
-        const int64_t b0 = ix.blk_off[c], v0 = ix.vec_off[c];
-        const int nb = (int)(ix.blk_off[c + 1] - b0), n = (int)(ix.vec_off[c + 1] - v0);
-        tl.blocks += nb;
-        tl.vecs += n;
-        if (nb == 0) continue;
-        if (lut) load_cluster(ix, qrot, lut + (size_t)p * 4 * ix.Dtot, scal + (size_t)p * S, c, sm);
-        else prepare_cluster(ix, qrot, prune, c, sm);
-        if (p + 1 < p_end) prefetch_centroid(ix, (int)probe[p + 1], tid, blockDim.x);
-        for (int t0 = 0; t0 < nb; t0 += kTileB) {
-            tile_candidates(ix, sm, b0, v0, nb, n, t0, nb, distk);
-            if (tid < 32) {
-                float dk = distk;
-                int sz = pool_size;
-                const unsigned nc = replay_tile_warp(S, t0, min(kTileB, nb - t0), sm, ix.ids + v0, sm.pool_id, sm.pool_d,
-                                                     sz, topk, dk, tl.rr);
-                if (tid == 0) {
-                    tl.spec += nc;
-                    distk = dk;
-                    pool_size = sz;
+    __shared__ ProbeHdr hdr[kHdrProbes];
+    __shared__ float vf[kHdrProbes * kMaxSeg];
+    __shared__ uint8_t nib[2][kPassQuads];  // blocks of each group left by the filter (two passes' worth)
+    const int S = ix.S, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    int par = 0;
+    for (int p0 = 0; p0 < np; p0 += kHdrProbes) {
+        const int m = min(kHdrProbes, np - p0);
+        __syncthreads();  // every thread is done with the headers
+        if (tid < kHdrProbes) {
+            ProbeHdr h{0, 0, 0, 0, 0, 0};
+            if (lane < m) {
+                h.c = (int)probe[p0 + lane];
+                h.b0 = ix.blk_off[h.c];
+                h.v0 = ix.vec_off[h.c];
+                h.nb = (int)(ix.blk_off[h.c + 1] - h.b0);
+                h.n = (int)(ix.vec_off[h.c + 1] - h.v0);
+                h.quads = (h.nb + kQuad - 1) / kQuad;
+            }
+            hdr[lane] = h;
+            tl.blocks += __reduce_add_sync(kFull, (unsigned)h.nb);
+            tl.vecs += __reduce_add_sync(kFull, (unsigned)h.n);
+        }
+        __syncthreads();
+        if (S > 1) {  // stage 0's scalars of every probe (Lut::prepare's q_l2sqr, in its order), a warp per probe
+            for (int i = w; i < m; i += kScanWarps)
+                if (hdr[i].nb)
+                    for (int s = 0; s < S; ++s) {
+                        const float v = stage0_scalar(ix, s, hdr[i].c, qrot, prune);
+                        if (lane == 0) vf[i * S + s] = v;
+                    }
+            __syncthreads();
+        }
+        int loaded = -1;  // probe whose LUT is in place
+        // lane i: groups of probes 0 .. i
+        int qincl = hdr[lane].quads;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, qincl, o);
+            if (lane >= o) qincl += y;
+        }
+        const int total = __shfl_sync(kFull, qincl, 31);
+        for (int q0 = 0; q0 < total;) {
+            const float tau = distk;
+            const int nqd = min(pool_size == topk ? kPassQuads : min(4, (topk + 63) >> 6), total - q0);
+            for (int qd = w; qd < nqd; qd += 2 * kScanWarps) {  // this warp's groups, two at a time
+                const float *fv[2];
+                int64_t gb[2];
+                int nv[2];
+                uint32_t left[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int q = min(qd + i * kScanWarps, nqd - 1);
+                    const int pi = __popc(__ballot_sync(kFull, qincl <= q0 + q));
+                    const ProbeHdr &h = hdr[pi];
+                    const int bq = kQuad * (q0 + q - (__shfl_sync(kFull, qincl, pi) - h.quads));
+                    nv[i] = min(kQuad, h.nb - bq);
+                    gb[i] = h.b0 + bq;
+                    fv[i] = vf + pi * S;
+                    left[i] = (1u << nv[i]) - 1u;
+                }
+                if (S > 1) quad_filter(ix, fv, gb, nv, tau, left);
+                if (lane == 0) {
+                    nib[par][qd] = (uint8_t)left[0];
+                    if (qd + kScanWarps < nqd) nib[par][qd + kScanWarps] = (uint8_t)left[1];
                 }
             }
             __syncthreads();
+            // lane i: the pass's i-th group, its probe, and the blocks left up to it
+            const uint32_t mine = lane < nqd ? nib[par][lane] : 0u;
+            par ^= 1;
+            int my_pi = 0;
+            {
+                const int x = q0 + min(lane, nqd - 1);
+#pragma unroll
+                for (int o = 16; o; o >>= 1) {
+                    const int v = __shfl_sync(kFull, qincl, my_pi + o - 1);
+                    if (v <= x) my_pi += o;
+                }
+            }
+            int sincl = __popc(mine);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(kFull, sincl, o);
+                if (lane >= o) sincl += y;
+            }
+            const int nleft = __shfl_sync(kFull, sincl, 31);
+            for (int k = 0; k < nleft;) {
+                const int pi = __shfl_sync(kFull, my_pi, __popc(__ballot_sync(kFull, sincl <= k)));
+                const int same = 31 - __clz(__ballot_sync(kFull, lane < nqd && my_pi == pi));  // its last group
+                const int ng = min(kTileB, __shfl_sync(kFull, sincl, same) - k);
+                const ProbeHdr h = hdr[pi];
+                if (loaded != pi) {
+                    if (lut) load_cluster(ix, qrot, lut + (size_t)(p0 + pi) * 4 * ix.Dtot, scal + (size_t)(p0 + pi) * S, h.c, sm);
+                    else prepare_cluster(ix, qrot, prune, h.c, sm);
+                    loaded = pi;
+                }
+                const int first = q0 - (__shfl_sync(kFull, qincl, pi) - h.quads);  // group of the probe at lane 0
+                auto blk = [&](int slot) {
+                    const int r = k + slot, g = __popc(__ballot_sync(kFull, sincl <= r));
+                    const uint32_t gm = __shfl_sync(kFull, mine, g);
+                    return kQuad * (first + g) + nth_bit(gm, r - (__shfl_sync(kFull, sincl, g) - __popc(gm)));
+                };
+                tile_candidates(ix, sm, h.b0, h.v0, h.nb, h.n, ng, blk, distk);
+                if (tid < 32) {
+                    float dk = distk;
+                    int sz = pool_size;
+                    const unsigned nc = replay_tile_warp(S, 0, sm.sblk, ng, sm, ix.ids + h.v0, sm.pool_id, sm.pool_d, sz,
+                                                         topk, dk, tl.rr);
+                    if (tid == 0) {
+                        tl.spec += nc;
+                        distk = dk;
+                        pool_size = sz;
+                    }
+                }
+                __syncthreads();
+                k += ng;
+            }
+            q0 += nqd;
         }
     }
 }
@@ -1619,7 +1998,7 @@ struct WsTile {
 __host__ __device__ inline size_t ws_tile_bytes(int S) {
     return 3 * align16(sizeof(float) * kTileB * S * 32) + align16(sizeof(float) * kTileB * 32) +
            align16(sizeof(float) * kTileB * (S + 1)) + align16(sizeof(uint32_t) * kTileB) +
-           align16(sizeof(int) * kTileB);
+           2 * align16(sizeof(int) * kTileB);
 }
 
 __host__ __device__ inline size_t ws_smem_bytes(int Dtot, int S, int topk, int xstride) {
@@ -1645,6 +2024,8 @@ __device__ __forceinline__ ScanSmem ws_view(const ScanSmem &sm, char *extra, int
     v.cmask = (uint32_t *)(extra + o);
     o += align16(sizeof(uint32_t) * kTileB);
     v.nstage = (int *)(extra + o);
+    o += align16(sizeof(int) * kTileB);
+    v.sblk = (int *)(extra + o);
     return v;
 }
 
@@ -1691,7 +2072,8 @@ __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan_ws(DevIndex
                 ScanSmem v = ws_view(sm, extra, S, b);
                 if (tid == 32) meta[b] = WsTile{v0, t0};
                 const float tau = __shfl_sync(kFull, *vdistk, 0);  // warp-uniform, as block_estimates wants
-                tile_candidates(ix, v, b0, v0, nb, n, t0, min(nb, t0 + kWsSlots), tau, 32, kWsWorkers, 1);
+                tile_candidates(ix, v, b0, v0, nb, n, min(kWsSlots, nb - t0), [&](int slot) { return t0 + slot; }, tau, 32,
+                                kWsWorkers, 1);
                 __threadfence_block();
                 named_arrive(2 + b, kScanThreads);
             }
@@ -1714,7 +2096,7 @@ __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan_ws(DevIndex
                 named_sync(2 + b, kScanThreads);  // tile ntiles written
                 const ScanSmem v = ws_view(sm, extra, S, b);
                 const WsTile mt = meta[b];
-                const unsigned nc = replay_tile_warp(S, mt.t0, min(kWsSlots, nb - mt.t0), v, ix.ids + mt.v0,
+                const unsigned nc = replay_tile_warp(S, mt.t0, nullptr, min(kWsSlots, nb - mt.t0), v, ix.ids + mt.v0,
                                                      sm.pool_id, sm.pool_d, sz, topk, dk, rr);
                 if (tid == 0) {
                     spec += nc;
@@ -1849,6 +2231,7 @@ __device__ void prepare_cluster_warp(const DevIndexView &ix, const float *__rest
         }
     }
     __syncwarp();
+    for (int g = 0; g < ix.Dtot / 64; ++g) ex_reorder(ws.qres + 64 * g);
 }
 
 __global__ void __launch_bounds__(kWarpsPerCta * 32) k_scan_warp(DevIndexView ix, const uint32_t *__restrict__ probe,
@@ -1975,8 +2358,6 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) k_scan_warp(DevIndexView ix
 // reference's decisions on the records.  Blocks without a record cannot insert
 // anything (none of their lanes is below tau1 >= distk), so the replay is exact.
 constexpr int kTileBlocks = 16;
-constexpr int kSpecChunk = 8;          // speculative tiles per work chunk of k_scan_spec
-constexpr int kSpecChunkPrepared = 2;  // ... when the LUTs come from the batched preparation
 constexpr int kFirstBlocks = 16;  // exact prefix of a deferred query (its distk bounds the first level)
 // Levels of the speculation for deferred queries, in tiles after the split
 // point: [0, 8), [8, 64), [64, end) by default; the autotuner may pick another
@@ -1991,8 +2372,12 @@ constexpr int kSpecLevelSets[][kMaxSpecLevels] = {
     {0, 64, -1, -1, -1},
 };
 constexpr int kNumSpecLevelSets = (int)(sizeof(kSpecLevelSets) / sizeof(kSpecLevelSets[0]));
-constexpr int kDeferBlocks = 1024;  // a query scanning more blocks than this takes the split pass
-                                     // (SAQG_DEFER_BLOCKS overrides it; 0 disables deferral)
+// A query probing more blocks than this takes the split pass (SAQG_DEFER_BLOCKS
+// overrides it; 0 disables deferral).  The longest query on a single CTA ends the
+// CTA scan, so the line lies low: 37 queries of 1,800 blocks 4.23 ms with 1,024
+// and 1.73 with 256, 256 queries of 560 blocks 1.72 and 1.22, 4,096 queries over
+// 10M vectors 2.90 and 2.15 (384: 2.13, 192: 2.21).
+constexpr int kDeferBlocks = 256;
 
 struct SplitState {
     int *nlist;          // number of queries on the list (device)
@@ -2089,11 +2474,11 @@ __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan_first(DevIn
                 const int te = min(nb, t0 + kTileB);
                 tl.blocks += te - t0;
                 tl.vecs += min(n, te * 32) - t0 * 32;
-                tile_candidates(ix, sm, b0, v0, nb, n, t0, nb, distk);
+                tile_candidates(ix, sm, b0, v0, nb, n, te - t0, [&](int slot) { return t0 + slot; }, distk);
                 if (tid < 32) {
                     float dk = distk;
                     int sz = pool_size;
-                    const unsigned nc = replay_tile_warp(S, t0, te - t0, sm, ix.ids + v0, sm.pool_id, sm.pool_d, sz, topk, dk,
+                    const unsigned nc = replay_tile_warp(S, t0, nullptr, te - t0, sm, ix.ids + v0, sm.pool_id, sm.pool_d, sz, topk, dk,
                                                          tl.rr);
                     if (tid == 0) {
                         tl.spec += nc;
@@ -2177,128 +2562,170 @@ __global__ void __launch_bounds__(kPrefixThreads) k_tile_prefix(SplitState st) {
     }
 }
 
+// Last index i of a[0, n) (ascending, a[0] <= x) with a[i] <= x, by a warp.
+__device__ __forceinline__ int warp_last_le(const int *__restrict__ a, int n, int x) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0;
+    while (n > 1) {
+        const int step = (n + 31) >> 5, i = lane * step;
+        const int hit = __popc(__ballot_sync(kFull, i < n && a[lo + min(i, n - 1)] <= x)) - 1;  // a prefix of the lanes
+        lo += hit * step;
+        n = min(step, n - hit * step);
+    }
+    return lo;
+}
+
+// One tile of a chunk of k_scan_spec.
+struct SpecTile {
+    int slot, q, p, c, n, nb, first, blocks;  // blocks [first, first + blocks) of cluster c, probe p of query q
+    int64_t b0, v0, pos;                      // pos: record position of block 0 of the cluster (in the slot's)
+    float tau;
+    uint32_t left;  // its blocks that stage 0 leaves
+};
+
 __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan_spec(DevIndexView ix, const uint32_t *__restrict__ probe,
                                                             int nprobe, const float *__restrict__ qrot_all,
                                                             const float *__restrict__ prune_all, SplitState st,
                                                             unsigned long long *__restrict__ counters, int xstride,
                                                             Prepared prep) {
     extern __shared__ __align__(16) char smem_raw[];
-    const int S = ix.S, tid = threadIdx.x;
+    __shared__ SpecTile tiles[kScanWarps];
+    __shared__ float vf[kScanWarps * kMaxSeg];
+    const int S = ix.S, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     ScanSmem sm = scan_smem_layout(smem_raw, ix.Dtot, S, 1, xstride);
     ScanTally tl;
     const int nl = list_len(st);
     const int total = st.q_tile_off[nl];
-    // chunks of consecutive tiles (mostly of one cluster: one LUT) taken from a
-    // shared counter: tiles differ widely in cost (candidates, pruning stages),
-    // so equal shares per CTA leave a long tail.  When every listed query has
-    // prepared LUTs a cluster switch is a copy, and chunks are short.
-    // at least about four chunks per CTA, so that a small level (few queries)
-    // still spreads over the whole grid
-    const bool all_prepared = prep.lut && prep.slots >= nl;
-    const int ct = max(1, min(all_prepared ? kSpecChunkPrepared : kSpecChunk, total / (4 * (int)gridDim.x)));
+    // chunks of consecutive tiles taken from a shared counter: tiles differ widely in
+    // cost (candidates, pruning stages), so equal shares per CTA leave a long tail.  A
+    // chunk has up to a tile per warp: each warp finds its tile and filters its blocks
+    // by stage 0 when the LUT's scalars are prepared, then the CTA takes the tiles with
+    // blocks left in order.  At least about four chunks per CTA, so that a small level
+    // (few queries) still spreads over the whole grid.
+    const int ct = max(1, min(kScanWarps, total / (4 * (int)gridDim.x)));
     __shared__ int chunk;
     int last_slot = -1, last_c = -1;
     for (;;) {
         if (tid == 0) chunk = atomicAdd(st.work_next, 1);
         __syncthreads();
-        const int w_begin = chunk * ct, w_end = min(total, w_begin + ct);
-        __syncthreads();  // every thread has read `chunk` before thread 0 takes the next
-        if (w_begin >= total) break;
-        for (int wi = w_begin; wi < w_end; ++wi) {
-            int lo = 0, hi = nl;  // slot: last with q_tile_off[slot] <= wi
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (st.q_tile_off[mid] <= wi) lo = mid;
-                else hi = mid;
-            }
-            const int slot = lo, q = st.qlist[slot];
+        const int w_begin = chunk * ct, nt = min(total - w_begin, ct);
+        if (nt <= 0) break;
+        if (w < nt) {
+            const int wi = w_begin + w, slot = warp_last_le(st.q_tile_off, nl, wi);
             const int local = st.t_lo + (wi - st.q_tile_off[slot]);
             const int *to = st.tile_off + (size_t)slot * (nprobe + 1);
-            int plo = 0, phi = nprobe;  // probe: last p with to[p] <= local
-            while (phi - plo > 1) {
-                const int mid = (plo + phi) >> 1;
-                if (to[mid] <= local) plo = mid;
-                else phi = mid;
-            }
-            const int p = plo, tile = local - to[p];
-            const int c = (int)probe[(size_t)q * nprobe + p];
-            if (slot != last_slot || c != last_c) {  // LUTs survive across tiles of one cluster
-                if (prep.has(slot)) load_cluster(ix, qrot_all + (size_t)q * ix.Dtot, prep.lut_of(slot, p, ix.Dtot),
-                                                 prep.scal_of(slot, p, S), c, sm);
-                else prepare_cluster(ix, qrot_all + (size_t)q * ix.Dtot, prune_all + (size_t)q * S, c, sm);
-                last_slot = slot;
-                last_c = c;
-            }
-            const int64_t b0 = ix.blk_off[c], v0 = ix.vec_off[c];
-            const int nb = (int)(ix.blk_off[c + 1] - b0), n = (int)(ix.vec_off[c + 1] - v0);
-            const int first = p == st.split_p[slot] ? st.split_b[slot] : 0;
-            const int bstart = first + tile * kTileBlocks, bend = min(nb, bstart + kTileBlocks);
-            if (tid == 0) {
-                tl.blocks += bend - bstart;
-                tl.vecs += min(n, bend * 32) - bstart * 32;
-            }
-            const float tau = st.tau[slot];
-            const int64_t base = st.blk_base[(size_t)slot * nprobe + p];
-            for (int t0 = bstart; t0 < bend; t0 += kTileB) {
-                tile_candidates(ix, sm, b0, v0, nb, n, t0, bend, tau);
-                const int lane = tid & 31;
-                for (int k = 0; k < kBlocksPerWarp; ++k) {
-                    const int w = (tid >> 5) + k * kScanWarps, b = t0 + w;
-                    if (b < bend) {
-                        const uint32_t cm = sm.cmask[w];
-                        const int64_t pos = base + b;
-                        if (cm && pos < st.npos[slot]) {
-                            float *r = st.rec + (size_t)(st.pos_off[slot] + pos) * st.rec_words;
-                            uint32_t *ri = reinterpret_cast<uint32_t *>(r);
-                            // summary: a later distk below the minimum estimate, or below a stage minimum,
-                            // leaves the block without effect
-                            const bool in = (cm >> lane) & 1u;
-                            float mn = in ? sm.cur[w * 32 + lane] : __int_as_float(0x7fffffff);
-                            float mx = (S > 1 && lane < sm.nstage[w]) ? sm.stage[w * (S + 1) + lane] : __int_as_float(0x7fffffff);
-                            // ... and a later distk below every value the lane's accept test can
-                            // compare (replay_block_warp: the accurate distance, or each running sum)
-                            float mz = __int_as_float(0x7f800000);
-                            if (in) {
-                                if (S == 1) {
-                                    mz = sm.part[w * 32 + lane];
-                                } else {
-                                    float acc = sm.cur[w * 32 + lane];
-                                    for (int s2 = 0; s2 < S; ++s2) {
-                                        acc = __fadd_rn(acc, sm.part[(w * S + s2) * 32 + lane]);
-                                        mz = fminf(mz, acc);
-                                        if (acc != acc) mz = -__int_as_float(0x7f800000);
-                                    }
-                                }
-                                if (mz != mz) mz = -__int_as_float(0x7f800000);
-                            }
-    #pragma unroll
-                            for (int o = 16; o; o >>= 1) {
-                                mn = fminf(mn, __shfl_xor_sync(kFull, mn, o));
-                                mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
-                                mz = fminf(mz, __shfl_xor_sync(kFull, mz, o));
-                            }
-                            if (lane == 0) {
-                                ri[0] = (uint32_t)pos;
-                                ri[1] = cm;
-                                ri[2] = (uint32_t)(S == 1 ? 0 : sm.nstage[w]);
-                                ri[3] = (uint32_t)c;
-                                ri[4] = (uint32_t)b;
-                                ri[5] = (uint32_t)(uint64_t)v0;
-                                ri[6] = (uint32_t)((uint64_t)v0 >> 32);
-                                ri[7] = __float_as_uint(mx);
-                                st.summ[st.pos_off[slot] + pos] = make_float4(mn, mx, mz, 0.0f);
-                                if (counters) atomicAdd(counters + 3, (unsigned long long)__popc(cm));
-                            }
-                            if (S > 1 && lane <= S) r[8 + lane] = sm.stage[w * (S + 1) + lane];
-                            r[8 + (S + 1) + lane] = sm.cur[w * 32 + lane];
-                            for (int s = 0; s < S; ++s)
-                                r[8 + (S + 1) + 32 + s * 32 + lane] = sm.part[(w * S + s) * 32 + lane];
-                        }
+            const int p = warp_last_le(to, nprobe, local), q = st.qlist[slot];
+            SpecTile t;
+            t.slot = slot;
+            t.q = q;
+            t.p = p;
+            t.c = (int)probe[(size_t)q * nprobe + p];
+            t.b0 = ix.blk_off[t.c];
+            t.v0 = ix.vec_off[t.c];
+            t.nb = (int)(ix.blk_off[t.c + 1] - t.b0);
+            t.n = (int)(ix.vec_off[t.c + 1] - t.v0);
+            t.first = (p == st.split_p[slot] ? st.split_b[slot] : 0) + (local - to[p]) * kTileBlocks;
+            t.blocks = min(kTileBlocks, t.nb - t.first);
+            t.tau = st.tau[slot];
+            t.pos = st.blk_base[(size_t)slot * nprobe + p];
+            t.left = (1u << t.blocks) - 1u;
+            if (S > 1) {
+                float *fv = vf + w * kMaxSeg;
+                if (prep.has(slot)) {
+                    if (lane < S) fv[lane] = prep.scal_of(slot, p, S)[lane].vfac;
+                } else {
+                    for (int s = 0; s < S; ++s) {
+                        const float v = stage0_scalar(ix, s, t.c, qrot_all + (size_t)q * ix.Dtot, prune_all + (size_t)q * S);
+                        if (lane == 0) fv[s] = v;
                     }
                 }
-                __syncthreads();
+                __syncwarp();
+                uint32_t left = 0;
+                for (int g = 0; g < kTileBlocks / kQuad; g += 2) {
+                    const float *const fvs[2] = {fv, fv};
+                    const int64_t gb[2] = {t.b0 + t.first + kQuad * g, t.b0 + t.first + kQuad * g + kQuad};
+                    const int nv[2] = {t.blocks - kQuad * g, t.blocks - kQuad * g - kQuad};  // past the tile: none
+                    uint32_t l2[2];
+                    const int nvc[2] = {min(kQuad, nv[0]), min(kQuad, nv[1])};
+                    quad_filter(ix, fvs, gb, nvc, t.tau, l2);
+                    left |= (l2[0] | l2[1] << kQuad) << (kQuad * g);
+                }
+                t.left = left;
             }
+            if (lane == 0) tiles[w] = t;
         }
+        __syncthreads();
+        for (int i = 0; i < nt; ++i) {
+            const SpecTile &t = tiles[i];
+            if (tid == 0) {
+                tl.blocks += t.blocks;
+                tl.vecs += min(t.n, (t.first + t.blocks) * 32) - t.first * 32;
+            }
+            const uint32_t left = t.left;
+            const int ng = __popc(left), slot = t.slot;
+            if (ng == 0) continue;
+            if (slot != last_slot || t.c != last_c) {  // LUTs survive across tiles of one cluster
+                if (prep.has(slot)) load_cluster(ix, qrot_all + (size_t)t.q * ix.Dtot, prep.lut_of(slot, t.p, ix.Dtot),
+                                                 prep.scal_of(slot, t.p, S), t.c, sm);
+                else prepare_cluster(ix, qrot_all + (size_t)t.q * ix.Dtot, prune_all + (size_t)t.q * S, t.c, sm);
+                last_slot = slot;
+                last_c = t.c;
+            }
+            tile_candidates(ix, sm, t.b0, t.v0, t.nb, t.n, ng, [&](int sl) { return t.first + nth_bit(left, sl); }, t.tau);
+            for (int wslot = w; wslot < ng; wslot += kScanWarps) {
+                const uint32_t cm = sm.cmask[wslot];
+                const int b = sm.sblk[wslot];
+                const int64_t pos = t.pos + b;
+                if (cm && pos < st.npos[slot]) {
+                    float *r = st.rec + (size_t)(st.pos_off[slot] + pos) * st.rec_words;
+                    uint32_t *ri = reinterpret_cast<uint32_t *>(r);
+                    // summary: a later distk below the minimum estimate, or below a stage minimum,
+                    // leaves the block without effect
+                    const bool in = (cm >> lane) & 1u;
+                    float mn = in ? sm.cur[wslot * 32 + lane] : __int_as_float(0x7fffffff);
+                    float mx = (S > 1 && lane < sm.nstage[wslot]) ? sm.stage[wslot * (S + 1) + lane] : __int_as_float(0x7fffffff);
+                    // ... and a later distk below every value the lane's accept test can
+                    // compare (replay_block_warp: the accurate distance, or each running sum)
+                    float mz = __int_as_float(0x7f800000);
+                    if (in) {
+                        if (S == 1) {
+                            mz = sm.part[wslot * 32 + lane];
+                        } else {
+                            float acc = sm.cur[wslot * 32 + lane];
+                            for (int s2 = 0; s2 < S; ++s2) {
+                                acc = __fadd_rn(acc, sm.part[(wslot * S + s2) * 32 + lane]);
+                                mz = fminf(mz, acc);
+                                if (acc != acc) mz = -__int_as_float(0x7f800000);
+                            }
+                        }
+                        if (mz != mz) mz = -__int_as_float(0x7f800000);
+                    }
+#pragma unroll
+                    for (int o = 16; o; o >>= 1) {
+                        mn = fminf(mn, __shfl_xor_sync(kFull, mn, o));
+                        mx = fmaxf(mx, __shfl_xor_sync(kFull, mx, o));
+                        mz = fminf(mz, __shfl_xor_sync(kFull, mz, o));
+                    }
+                    if (lane == 0) {
+                        ri[0] = (uint32_t)pos;
+                        ri[1] = cm;
+                        ri[2] = (uint32_t)(S == 1 ? 0 : sm.nstage[wslot]);
+                        ri[3] = (uint32_t)t.c;
+                        ri[4] = (uint32_t)b;
+                        ri[5] = (uint32_t)(uint64_t)t.v0;
+                        ri[6] = (uint32_t)((uint64_t)t.v0 >> 32);
+                        ri[7] = __float_as_uint(mx);
+                        st.summ[st.pos_off[slot] + pos] = make_float4(mn, mx, mz, 0.0f);
+                        if (counters) atomicAdd(counters + 3, (unsigned long long)__popc(cm));
+                    }
+                    if (S > 1 && lane <= S) r[8 + lane] = sm.stage[wslot * (S + 1) + lane];
+                    r[8 + (S + 1) + lane] = sm.cur[wslot * 32 + lane];
+                    for (int s = 0; s < S; ++s) r[8 + (S + 1) + 32 + s * 32 + lane] = sm.part[(wslot * S + s) * 32 + lane];
+                }
+            }
+            __syncthreads();
+        }
+        __syncthreads();  // every thread is done with the chunk's tiles
     }
     if (tid == 0 && counters) {
         atomicAdd(counters + 0, tl.blocks);
@@ -2355,6 +2782,10 @@ constexpr int kReplayPer = 4;    // scan positions per thread in a window
 // every warp evaluates records under the current distk; the first record with
 // an accepted insert is replayed exactly by warp 0 (the records before it
 // change nothing and only add their counts), and evaluation resumes after it.
+// kRows > 0 (no counters kept, k at most 32 kRows, at most kRegSegs segments): warp 0 holds the pool in registers,
+// and a chunk is evaluated once: the records marked under the distk at its start are
+// replayed one after the other, without a barrier per record.
+template <int kRows>
 __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, SplitState st,
                                                               uint32_t *__restrict__ out_ids, float *__restrict__ out_d,
                                                               unsigned long long *__restrict__ counters, int xstride) {
@@ -2391,6 +2822,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
         const int RW = st.rec_words, R16 = RW / 4;
         unsigned long long rr = 0;
         __syncthreads();
+        RegPool<kRows ? kRows : 1> P;
+        if (kRows && w == 0) P.load(sm.pool_id, sm.pool_d, pool_size, topk, distk);
         const int pos_end = min(np, s_phi);
         for (int base = s_plo; base < pos_end; base += kScanThreads * kReplayPer) {
             // thread t tests positions base + kReplayPer t .. + kReplayPer - 1; a
@@ -2480,6 +2913,47 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
                 __syncthreads();
                 const float *buf = stage_buf + (size_t)(k & 1) * kReplayRecs * RW;
                 const int c0 = k * kReplayRecs, cn = min(kReplayRecs, total - c0);
+                if (kRows) {
+                    // every warp marks the records with an accepted insert under the distk at the
+                    // chunk's start (a superset of those that have one at their turn)
+                    const float dk = distk;
+                    const int sz = pool_size;
+                    for (int r = w; r < cn; r += kScanWarps) {
+                        int c;
+                        const float *rec = buf + (size_t)r * RW;
+                        const bool e = record_effect(S, rec, dk, sz, topk, c);
+                        if (lane == 0) {
+                            eff[r] = e;
+                            const uint32_t *ri = reinterpret_cast<const uint32_t *>(rec);
+                            const int64_t v0 = (int64_t)(((uint64_t)ri[6] << 32) | ri[5]);
+                            if (e) asm volatile("prefetch.global.L1 [%0];" ::"l"(ix.ids + v0 + (int64_t)ri[4] * 32));
+                        }
+                    }
+                    __syncthreads();
+                    if (w == 0) {
+                        uint32_t live = __ballot_sync(kFull, lane < cn && eff[lane]);
+                        for (; live; live &= live - 1) {
+                            const float *rec = buf + (size_t)(__ffs(live) - 1) * RW;
+                            const uint32_t *ri = reinterpret_cast<const uint32_t *>(rec);
+                            const uint32_t *rid = ix.ids + (int64_t)(((uint64_t)ri[6] << 32) | ri[5]) + (int64_t)ri[4] * 32;
+                            if (!replay_block_regs(S, rec + 8 + (S + 1), __uint_as_float(ri[7]), rec + 8 + (S + 1) + 32,
+                                                   ri[1], rid, P, rr)) {  // a NaN: on the pool in shared memory
+                                P.store(sm.pool_id, sm.pool_d);
+                                float dkw = P.dk;
+                                int szw = P.sz;
+                                replay_block_warp(S, 0, rec + 8 + (S + 1), __uint_as_float(ri[7]), rec + 8 + (S + 1) + 32,
+                                                  ri[1], rid, sm.pool_id, sm.pool_d, szw, topk, dkw, rr);
+                                P.load(sm.pool_id, sm.pool_d, szw, topk, dkw);
+                            }
+                        }
+                        if (lane == 0) {
+                            distk = P.dk;
+                            pool_size = P.sz;
+                        }
+                    }
+                    __syncthreads();
+                    continue;
+                }
                 if (tid == 0) {  // read by warp 0 (thread 0 first) and, after the chunk, by count_dropped
                     c_dk0 = distk;
                     n_eff = 0;
@@ -2532,6 +3006,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
                 }
             }
         }
+        if (kRows && w == 0) P.store(sm.pool_id, sm.pool_d);
         __syncthreads();
         if (tid == 0 && counters) atomicAdd(counters + 2, rr);
         if (st.final_level) {
@@ -2569,7 +3044,7 @@ __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan(DevIndexVie
     __shared__ float distk;
     ScanTally tl;
     init_pool(sm, topk, pool_size, distk);
-    scan_probes(ix, probe + (size_t)qi * qsh.np_max, 0, np, qrot_all + (size_t)qi * ix.Dtot,
+    scan_probes(ix, probe + (size_t)qi * qsh.np_max, np, qrot_all + (size_t)qi * ix.Dtot,
                 prune_all + (size_t)qi * ix.S, topk, sm, pool_size, distk, tl,
                 prep.has(qi) ? prep.lut_of(qi, 0, ix.Dtot) : nullptr, prep.has(qi) ? prep.scal_of(qi, 0, ix.S) : nullptr);
     flush_tally(tl, counters);
@@ -2828,8 +3303,8 @@ struct Bump {
 // kPrepCap holds (nprobe pairs each), at most nq; 0 below kPrepMinQueries
 // queries, where the scan CTAs build each cluster's state in the shorter latency
 // (256 threads per LUT).  12 GB holds every query of a 4,096-query batch at
-// nprobe 256 with D = 1024 (8.8 GB; the CTA scan's copy is as large again), a
-// few percent of the device beside the index.
+// nprobe 256 with D = 1024 (8.8 GB; one segment: the CTA scan's copy is as large
+// again), a few percent of the device beside the index.
 constexpr size_t kPrepCap = (size_t)12 << 30;
 constexpr int64_t kPrepMinQueries = 64;
 size_t prep_pair_bytes(const Index &I) { return 8 * (size_t)I.view.Dtot + sizeof(SegScal) * I.view.S; }
@@ -2860,7 +3335,7 @@ size_t search_scratch_bytes(const Index &I, int64_t nq, int64_t topk, int64_t np
     add(64);                                   // flags
     add(64);                                   // counters
     add(prep_bytes(I, nq, nprobe));            // prepared LUTs of the split list
-    if (prep_slots(I, nq, nprobe) == nq) add(prep_bytes(I, nq, nprobe));  // ... and of the CTA scan's queries
+    if (prep_slots(I, nq, nprobe) == nq && I.view.S == 1) add(prep_bytes(I, nq, nprobe));  // ... and of the CTA scan's
     (void)host_io;
     return b + 256;
 }
@@ -3250,7 +3725,7 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
     const int64_t pslots = prep_slots(I, nq, nprobe);
     uint16_t *prep_lut = pslots ? bp.take<uint16_t>((size_t)pslots * nprobe * 4 * ix.Dtot) : nullptr;
     SegScal *prep_scal = pslots ? bp.take<SegScal>((size_t)pslots * nprobe * ix.S) : nullptr;
-    const bool scan_prep_fits = pslots > 0 && pslots == nq;
+    const bool scan_prep_fits = pslots > 0 && pslots == nq && ix.S == 1;
     uint16_t *scan_lut = scan_prep_fits ? bp.take<uint16_t>((size_t)nq * nprobe * 4 * ix.Dtot) : nullptr;
     SegScal *scan_scal = scan_prep_fits ? bp.take<SegScal>((size_t)nq * nprobe * ix.S) : nullptr;
     cudaEvent_t ev[7] = {};
@@ -3320,10 +3795,10 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
         unsigned long long *cnt = stats ? counters : nullptr;
         const int mode0 = scan_mode(nq, topk, tune);
         const int mode = (qsh.np || qsh.k) && mode0 == 2 ? 0 : mode0;
-        // The CTA scan's queries get batched LUTs too (by query; on the caller's stream,
-        // after the split pass has forked, so it overlaps the split pass's start) when
-        // the budget holds every query's: one batched kernel builds them for less than
-        // the scan CTAs do (10M / 4,096 queries: 3.70 against 3.81 ms per batch).
+        // One segment: the CTA scan's queries get batched LUTs too (by query; on the
+        // caller's stream, after the split pass has forked, so it overlaps the split
+        // pass's start) when the budget holds every query's.  Several segments: the
+        // scan needs the LUT of one probe in four (10M / 4,096 queries) and builds those.
         const std::function<Prepared(const uint8_t *)> scan_prep = [&](const uint8_t *skip) {  // skip: queries left out
             Prepared pp;
             if (!scan_lut || scan_ws(tune)) return pp;
@@ -3423,7 +3898,10 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
             SAQG_REQUIRE(smem_r <= 220 * 1024, "dimension / topk too large for the replay kernel's shared memory");
             ensure_smem((const void *)k_scan_first, (size_t)smem);
             ensure_smem((const void *)k_scan_spec, (size_t)smem1);
-            ensure_smem((const void *)k_scan_replay, (size_t)smem_r);
+            // counters need every record's count, and a longer pool shared memory
+            const auto replay = cnt || topk > kRegPool || ix.S > kRegSegs ? k_scan_replay<0> : topk <= 32 ? k_scan_replay<1>
+                                                                               : k_scan_replay<kRegPool / 32>;
+            ensure_smem((const void *)replay, (size_t)smem_r);
             Prepared prep;  // the listed queries' LUTs, one batched kernel ahead of the split pass
             if (prep_lut) {
                 const size_t lsm = 4 * (size_t)kLutWarps * ix.Dtot;
@@ -3463,7 +3941,7 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
                 k_scan_spec<<<grid, kScanThreads, smem1, sp>>>(ix, probe, (int)nprobe, qrot, prune, sl, cnt, xs, prep);
                 check_launch("k_scan_spec");
                 if (stats && sl.final_level) SAQG_CUDA_TRY(cudaEventRecord(ev[6], sp));
-                k_scan_replay<<<slot_grid, kScanThreads, smem_r, sp>>>(ix, sl, ids_out, d_out, cnt, xs);
+                replay<<<slot_grid, kScanThreads, smem_r, sp>>>(ix, sl, ids_out, d_out, cnt, xs);
                 check_launch("k_scan_replay");
             }
             if (stats) SAQG_CUDA_TRY(cudaEventRecord(ev[4], sp));
@@ -3735,15 +4213,11 @@ __device__ float searched_dist(const DevIndexView &ix, const ScanSmem &sm, int64
         v[s] = __shfl_sync(kFull, v[s], ln);
         f[s] = __shfl_sync(kFull, f[s], ln);
     }
-    // ex-code inner products by the 16 lanes of CodeHelper::compute_ip (each
-    // half-warp computes them; lane 0 holds the result)
+    // ex-code inner products (both half-warps compute them; lane 0 holds the result)
     float ex[kMaxSeg];
-    const unsigned half = lane < 16 ? 0x0000ffffu : 0xffff0000u;
     for (int s = 0; s < S; ++s) {
         const SegDev &g = ix.seg[s];
-        ex[s] = g.bits > 1 ? excode_ip_half(sm.qres + g.qoff, g.lcode + (size_t)gv * g.lstride, g.dim, g.bits - 1,
-                                            lane & 15, half)
-                           : 0.0f;
+        ex[s] = g.bits > 1 ? excode_ip16(sm.qres + g.qoff, g.lcode + (size_t)gv * g.lstride, g.dim, g.bits - 1) : 0.0f;
     }
     float d = 0.0f;
     if (lane == 0) {
