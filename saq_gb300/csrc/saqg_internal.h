@@ -233,8 +233,7 @@ void tc_rank_rotate(const Index &idx, SearchCtx &ctx, const float *q, int64_t nq
 size_t tc_probe_work_bytes(const Index &idx, int64_t nq);
 void tc_rerank(const Index &idx, const uint32_t *probe, int64_t nq, int64_t nprobe, const float *qrot,
                const float *prune, const int *lp, const int *sl_pos, const float *sl_apx, const int *sl_cnt, int L,
-               int64_t topk, const int *qk, int *grp, int *gj, int *ng, float *sl_dist, uint32_t *ids, float *dists,
-               float *apx, cudaStream_t st);
+               int64_t topk, const int *qk, float *sl_dist, uint32_t *ids, float *dists, float *apx, cudaStream_t st);
 // Options of the tensor-core form beyond its arguments.
 struct TcOpts {
     const TcTune *tune = nullptr;  // null: the index's tuned choice for the shape, else built-in

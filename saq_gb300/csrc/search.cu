@@ -48,22 +48,25 @@ constexpr int kScanMinCtas = 4;  // resident scan CTAs per SM the register budge
 
 struct SegScal {
     float delta, vl, sum_vl, sum_q, q_l2sqr, q_l2norm, c1, c2, vfac;
-    float rdelta;  // RN(1 / delta): the LUT quantizer's fast path
+    float rdelta;  // RN(1 / delta), for the LUT quantizer
 };
 
 // A u16 LUT entry (uint16_t)(int)(x / d), x >= 0, with the division rounded to
-// nearest, mostly without dividing: y = RN(x * r), r = RN(1 / d), lies within
-// 3.02 * 2^-24 * y of RN(x / d), so when no integer lies within 2^-21 * y of y
-// both truncate to the same integer.  Otherwise (and for NaN / inf) `ok` is
-// false and the caller divides.  The floors come from adding 2^23 rounded
-// down (2^23 + floor(v) for 0 <= v < 2^23, the integer in the low mantissa
-// bits), so the check and the result take FP32 adds, not conversions.
-__device__ __forceinline__ uint32_t lut_quant_fast(float x, float r, bool &ok) {
-    const float y = __fmul_rn(x, r);
-    const float e = __fmul_rn(y, 4.76837158203125e-07f);  // 2^-21
-    const float lo = __fadd_rd(__fsub_rn(y, e), 8388608.0f), hi = __fadd_rd(__fadd_rn(y, e), 8388608.0f);
-    ok = lo == hi && y < 4194304.0f;  // y < 2^22 keeps both sums in the binade of 2^23
-    return __float_as_uint(lo) & 0xffffu;  // (uint16_t)(int)y: y >= 0, trunc = floor
+// nearest, without dividing.  n, the integer nearest to x * RN(1 / d), is within 0.52
+// of x / d (x / d stays below 65,536), so the entry is n or n - 1: n when x / d rounds
+// to n or above, i.e. when n - x / d is at most half the spacing u of the floats below n
+// (n is the even neighbour of that tie).  x - n d, one FMA, decides: its sign is
+// right, and where it is near -d u / 2 (below 2^-9 d) it is exact, a multiple of d's
+// last place of less than 24 bits.  d must be a normal float with room below
+// (lut_quant_ok); 16 entries take 11 operations each, where a check of the product
+// and a division for 3% of the entries took 7 and a loop.
+__device__ __forceinline__ bool lut_quant_ok(float d) { return d > 1e-30f && d < 1e30f; }
+__device__ __forceinline__ uint32_t lut_quant(float x, float d, float r) {
+    const float m = __fadd_rn(__fmul_rn(x, r), 8388608.0f);  // 2^23 + n: n in the low mantissa bits
+    const float n = __fsub_rn(m, 8388608.0f);
+    const float half_u = __uint_as_float(((__float_as_uint(n) - 1u) & 0x7f800000u) - (24u << 23));  // n = 0: huge
+    const float rem = __fmaf_rn(-n, d, x);
+    return (__float_as_uint(m) - (rem < -__fmul_rn(d, half_u) ? 1u : 0u)) & 0xffffu;
 }
 
 __device__ __forceinline__ uint32_t fkey(float f) {
@@ -644,10 +647,20 @@ __device__ __forceinline__ void lut_entries(const float *__restrict__ qq, float 
     }
 }
 
+// Lut::compFastIP's float epilogue and the L2 form of CaqCluEstimator::compFastDist
+// (caq_estimator.hpp:148-179) for a FastScan sum.
+__device__ __forceinline__ float fast_of_sum(const SegScal &sc, int sum, float onorm, float &ipx) {
+    float t = __fmul_rn((float)sum, sc.delta);
+    t = __fadd_rn(t, sc.sum_vl);
+    ipx = t;
+    float f = __fmul_rn(__fsub_rn(t, sc.c1), sc.c2);
+    f = __fmul_rn(f, onorm);
+    return maxps(0.0f, __fadd_rn(__fmul_rn(onorm, onorm), __fsub_rn(sc.q_l2sqr, f)));
+}
+
 // FastScan sum of one vector (this lane) of block gb: sum over codebooks of
 // LUT_u16[cb][nibble] (accumulate_hacc, fastscan_highacc.hpp:66-139, exact
-// for dim <= 2048), then Lut::compFastIP's float epilogue and the L2 form of
-// CaqCluEstimator::compFastDist (caq_estimator.hpp:148-179).
+// for dim <= 2048), then fast_of_sum.
 __device__ __forceinline__ float fast_est(const SegDev &g, const uint16_t *__restrict__ lut, const SegScal &sc,
                                           int64_t gb, int lane, float onorm, float &ipx) {
     const int nc = g.dim / 64;
@@ -670,12 +683,7 @@ __device__ __forceinline__ float fast_est(const SegDev &g, const uint16_t *__res
             sum += *reinterpret_cast<const uint16_t *>(L + (8 + 2 * j) * 32 + __byte_perm(hy, 0u, 0x4440u | j)) +
                    *reinterpret_cast<const uint16_t *>(L + (8 + 2 * j + 1) * 32 + __byte_perm(ly, 0u, 0x4440u | j));
     }
-    float t = __fmul_rn((float)sum, sc.delta);
-    t = __fadd_rn(t, sc.sum_vl);
-    ipx = t;
-    float f = __fmul_rn(__fsub_rn(t, sc.c1), sc.c2);
-    f = __fmul_rn(f, onorm);
-    return maxps(0.0f, __fadd_rn(__fmul_rn(onorm, onorm), __fsub_rn(sc.q_l2sqr, f)));
+    return fast_of_sum(sc, sum, onorm, ipx);
 }
 
 __device__ __forceinline__ float vars_est(const SegScal &sc, float onorm) {
@@ -929,54 +937,42 @@ __device__ __forceinline__ void seg_epilogue_scalars(const SegDev &g, float prun
     sc.vfac = __fsub_rn(sc.q_l2sqr, __fmul_rn(2.0f, prune_s));
 }
 
-// Float entry j of one codebook in lut_entries' order: entry j = entry[j -
-// lowbit(j)] + q[kPos[lowbit(j)]], so the dims of j's bits are added from the
-// highest bit down (kPos of bit b is 3 - b).
-__device__ __forceinline__ float lut_entry_at(const float *qq, int j) {
-    float t = 0.0f;
-    for (int b = 3; b >= 0; --b)
-        if ((j >> b) & 1) t = __fadd_rn(t, qq[3 - b]);
-    return t;
-}
-
 // The 16 u16 entries of one codebook (4 residual dims at qq), 32 bytes at dst.
-// Every entry takes the multiply first; the few that it cannot settle (about 3%)
-// are divided afterwards and stored over it, in a loop whose trip count is the
-// lane's own number of such entries, so a warp runs a handful of divisions per
-// codebook instead of one per entry that any lane needs.
 __device__ __forceinline__ void quant_codebook(const float *qq, float vl, float delta, float rd, uint16_t *dst) {
     float t[16];
     lut_entries(qq, t);
     uint32_t packed[8];
-    uint32_t slow = 0;
+    if (lut_quant_ok(delta)) {  // the segment's: uniform over most of a warp
 #pragma unroll
-    for (int j = 0; j < 16; j += 2) {
-        bool oa, ob;
-        const uint32_t a = lut_quant_fast(__fsub_rn(t[j], vl), rd, oa);
-        const uint32_t b = lut_quant_fast(__fsub_rn(t[j + 1], vl), rd, ob);
-        slow |= (oa ? 0u : 1u << j) | (ob ? 0u : 2u << j);
-        packed[j / 2] = a | (b << 16);
+        for (int j = 0; j < 16; j += 2)
+            packed[j / 2] = lut_quant(__fsub_rn(t[j], vl), delta, rd) | lut_quant(__fsub_rn(t[j + 1], vl), delta, rd) << 16;
+    } else {
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) {
+            const uint32_t a = (uint16_t)(int)__fdiv_rn(__fsub_rn(t[j], vl), delta);
+            const uint32_t b = (uint16_t)(int)__fdiv_rn(__fsub_rn(t[j + 1], vl), delta);
+            packed[j / 2] = a | (b << 16);
+        }
     }
     uint4 *d = reinterpret_cast<uint4 *>(dst);
     d[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
     d[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-    while (slow) {  // same thread, same address: the later store wins
-        const int j = __ffs(slow) - 1;
-        slow &= slow - 1;
-        dst[j] = (uint16_t)(int)__fdiv_rn(__fsub_rn(lut_entry_at(qq, j), vl), delta);
-    }
 }
 
-// Min and max keys of one codebook's float entries.
-__device__ __forceinline__ void codebook_keys(const float *qq, uint32_t &kmin, uint32_t &kmax) {
-    float t[16];
-    lut_entries(qq, t);
-    float lo = t[0], hi = t[0];
-#pragma unroll
-    for (int j = 1; j < 16; ++j) {
-        lo = fminf(lo, t[j]);
-        hi = fmaxf(hi, t[j]);
-    }
+// Min and max keys of one codebook's float entries.  An entry adds its dims in a
+// fixed order (lut_entries), and rounding is monotone: leaving out a dim that is not
+// negative never raises the sum, adding a negative one never does either, so the
+// smallest entry is the one of the negative dims and the largest that of the positive.
+__device__ __forceinline__ void codebook_keys(const float4 &q, uint32_t &kmin, uint32_t &kmax) {
+    float lo = 0.0f, hi = 0.0f;
+    lo = __fadd_rn(lo, fminf(q.x, 0.0f));
+    hi = __fadd_rn(hi, fmaxf(q.x, 0.0f));
+    lo = __fadd_rn(lo, fminf(q.y, 0.0f));
+    hi = __fadd_rn(hi, fmaxf(q.y, 0.0f));
+    lo = __fadd_rn(lo, fminf(q.z, 0.0f));
+    hi = __fadd_rn(hi, fmaxf(q.z, 0.0f));
+    lo = __fadd_rn(lo, fminf(q.w, 0.0f));
+    hi = __fadd_rn(hi, fmaxf(q.w, 0.0f));
     kmin = fkey(lo);
     kmax = fkey(hi);
 }
@@ -991,21 +987,21 @@ __device__ __forceinline__ void ex_reorder(float *x) {
     __syncwarp();
 }
 
-// Lut::prepare (lut.hpp:60-87) for every segment of cluster c, spread over the
-// whole CTA: residual query, its Eigen-order sum and squared norm, the float
-// LUT's min / max, delta = (max-min)/(65536-0.01) in double, the u16 LUT
-// trunc((entry-min)/delta), and the epilogue constants of compFastIP.
-// Leaves the residual query in ex order (see excode_ip16).
+// The first part of Lut::prepare (lut.hpp:60-87) for every segment of cluster c,
+// spread over the whole CTA: the residual query (natural order, sm.qres), its
+// Eigen-order sum and squared norm, the float LUT's min / max, and from them delta =
+// (max-min)/(65536-0.01) in double and the epilogue constants of compFastIP (these
+// are in place after the caller's next barrier).
 // t_first > 0: only threads [t_first, blockDim.x) take part (whole warps),
 // synchronising on named barrier `bar` instead of __syncthreads.
-__device__ void prepare_cluster(const DevIndexView &ix, const float *__restrict__ qrot, const float *__restrict__ prune,
+__device__ __forceinline__ void cta_sync(int bar, int nt) {
+    if (bar) asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(nt) : "memory");
+    else __syncthreads();
+}
+__device__ void prepare_scalars(const DevIndexView &ix, const float *__restrict__ qrot, const float *__restrict__ prune,
                                 int c, ScanSmem &sm, int t_first = 0, int bar = 0) {
     const int tid = (int)threadIdx.x - t_first, nt = (int)blockDim.x - t_first, warp = tid >> 5, lane = tid & 31;
     const int S = ix.S;
-    auto sync = [&]() {
-        if (bar) asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(nt) : "memory");
-        else __syncthreads();
-    };
     for (int i = tid; i < ix.Dtot; i += nt) {
         int s = 0;
         while (s + 1 < S && i >= ix.seg[s + 1].qoff) ++s;
@@ -1016,7 +1012,7 @@ __device__ void prepare_cluster(const DevIndexView &ix, const float *__restrict_
         sm.mm[2 * tid] = 0xffffffffu;  // min key
         sm.mm[2 * tid + 1] = 0u;       // max key
     }
-    sync();
+    cta_sync(bar, nt);
     for (int t = warp; t < 2 * S; t += nt / 32) {
         const int s = t >> 1;
         const float *qr = sm.qres + ix.seg[s].qoff;
@@ -1035,7 +1031,7 @@ __device__ void prepare_cluster(const DevIndexView &ix, const float *__restrict_
         if (cb < ncb_all) {
             s = 0;
             while (s + 1 < S && cb * 4 >= ix.seg[s + 1].qoff) ++s;
-            codebook_keys(sm.qres + cb * 4, kmin, kmax);
+            codebook_keys(*reinterpret_cast<const float4 *>(sm.qres + cb * 4), kmin, kmax);
         }
         // one shared atomic per segment present in the warp
         const unsigned grp = __match_any_sync(kFull, s);
@@ -1046,22 +1042,31 @@ __device__ void prepare_cluster(const DevIndexView &ix, const float *__restrict_
             atomicMax(&sm.mm[2 * s + 1], kmax);
         }
     }
-    sync();
+    cta_sync(bar, nt);
     if (tid < S) seg_quant_scalars(sm.mm[2 * tid], sm.mm[2 * tid + 1], sm.scal[tid]);  // what the quantizer needs
-    sync();
-    if (tid >= nt - S) {  // the epilogue constants, beside the quantization (the last warp's last lanes)
+    cta_sync(bar, nt);
+    if (tid >= nt - S) {  // the epilogue constants, beside what follows (the last warp's last lanes)
         const int s = tid - (nt - S);
         seg_epilogue_scalars(ix.seg[s], prune[s], sm.scal[s]);
     }
+}
+
+// Lut::prepare: prepare_scalars, then the u16 LUT trunc((entry-min)/delta); leaves the
+// residual query in ex order (see excode_ip16).
+__device__ void prepare_cluster(const DevIndexView &ix, const float *__restrict__ qrot, const float *__restrict__ prune,
+                                int c, ScanSmem &sm, int t_first = 0, int bar = 0) {
+    const int tid = (int)threadIdx.x - t_first, nt = (int)blockDim.x - t_first, warp = tid >> 5;
+    const int S = ix.S, ncb_all = ix.Dtot / 4;
+    prepare_scalars(ix, qrot, prune, c, sm, t_first, bar);
     for (int cb = tid; cb < ncb_all; cb += nt) {
         int s = 0;
         while (s + 1 < S && cb * 4 >= ix.seg[s + 1].qoff) ++s;
         const SegScal &sc = sm.scal[s];
         quant_codebook(sm.qres + cb * 4, sc.vl, sc.delta, sc.rdelta, sm.lut + cb * 16);
     }
-    sync();
+    cta_sync(bar, nt);
     for (int g = warp; g < ix.Dtot / 64; g += nt / 32) ex_reorder(sm.qres + 64 * g);
-    sync();
+    cta_sync(bar, nt);
 }
 
 // Output of the batched preparation (k_lut) for the first `slots` entries of the
@@ -1128,7 +1133,7 @@ __global__ void __launch_bounds__(kLutWarps * 32) k_lut(DevIndexView ix, const u
         uint32_t kmin = 0xffffffffu, kmax = 0u;
         for (int k = lane; k < ncb; k += 32) {
             uint32_t a, b;
-            codebook_keys(qres + (cb0 + k) * 4, a, b);
+            codebook_keys(*reinterpret_cast<const float4 *>(qres + (cb0 + k) * 4), a, b);
             kmin = min(kmin, a);
             kmax = max(kmax, b);
         }
@@ -4195,101 +4200,204 @@ void run_search_static(const Index &I, const float *q, int64_t nq, int64_t topk,
 // ------------------------------------------ tensor-core form: probes and re-rank
 namespace {
 
+// A cluster's residual query (ex order, x) and the scalars of Lut::prepare, by one
+// warp; lanes s and 16 + s return with segment s's scalars.
+__device__ __forceinline__ SegScal warp_scalars(const DevIndexView &ix, const float *__restrict__ qrot,
+                                                const float *__restrict__ prune, int c, float *x) {
+    const int lane = threadIdx.x & 31, at0 = ex_order(lane), at1 = ex_order(lane + 32);
+    SegScal sc;
+    uint32_t my_min = 0xffffffffu, my_max = 0u;
+    for (int s = 0; s < ix.S; ++s) {
+        const SegDev &g = ix.seg[s];
+        const float *cent = g.cent + (size_t)c * g.dim + lane, *q = qrot + g.qoff + lane;
+        float *xs = x + g.qoff;
+        // Eigen's sums (warp_eigen_sum): lane i of the two 16-lane accumulators takes the
+        // dims i, i + 32, ...
+        float sum = 0.0f, sq = 0.0f;
+#pragma unroll 4
+        for (int d = 0; d < g.dim; d += 64) {
+            const float a = __fsub_rn(q[d], cent[d]), b = __fsub_rn(q[d + 32], cent[d + 32]);
+            xs[d + at0] = a;
+            xs[d + at1] = b;
+            sum = d == 0 ? a : __fadd_rn(sum, a);
+            sq = d == 0 ? __fmul_rn(a, a) : __fadd_rn(sq, __fmul_rn(a, a));
+            sum = __fadd_rn(sum, b);
+            sq = __fadd_rn(sq, __fmul_rn(b, b));
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            sum = __fadd_rn(sum, __shfl_down_sync(kFull, sum, o));
+            sq = __fadd_rn(sq, __shfl_down_sync(kFull, sq, o));
+        }
+        sum = __shfl_sync(kFull, sum, 0);
+        sq = __shfl_sync(kFull, sq, 0);
+        __syncwarp();
+        uint32_t kmin = 0xffffffffu, kmax = 0u;
+        for (int k = lane; k < g.dim / 4; k += 32) {
+            const float *p = xs + ex_order(4 * k);  // dims 4k .. 4k + 3 lie four apart
+            uint32_t a, b;
+            codebook_keys(make_float4(p[0], p[4], p[8], p[12]), a, b);
+            kmin = min(kmin, a);
+            kmax = max(kmax, b);
+        }
+        kmin = __reduce_min_sync(kFull, kmin);
+        kmax = __reduce_max_sync(kFull, kmax);
+        if ((lane & 15) == s) {
+            sc.sum_q = sum;
+            sc.q_l2sqr = sq;
+            my_min = kmin;
+            my_max = kmax;
+        }
+    }
+    if ((lane & 15) < ix.S) {
+        seg_quant_scalars(my_min, my_max, sc);
+        seg_epilogue_scalars(ix.seg[lane & 15], prune[lane & 15], sc);
+    }
+    return sc;
+}
+
 // Distance the search inserts for a vector that passes every pruning stage
-// (block_estimates + the accurate pass + replay_block): one segment, the
+// (block_estimates + the accurate pass + the replay): one segment, the
 // accurate distance; several, the running sum of variance bounds, each coded
 // segment's bound replaced by its fast estimate, then every segment's
-// estimate replaced by its accurate distance, in segment order.
-__device__ float searched_dist(const DevIndexView &ix, const ScanSmem &sm, int64_t gb, int64_t gv, int ln, int lane) {
-    const int S = ix.S;
-    float v[kMaxSeg], f[kMaxSeg], ipx[kMaxSeg];
+// estimate replaced by its accurate distance, in segment order.  Two vectors at a
+// time, one per half-warp (gb, gv, ln: the half's own), without a LUT: of each codebook
+// the one entry that the vector's nibble selects is formed and quantized.  x: the
+// residual in ex order; sc: lanes s and 16 + s segment s's scalars.
+__device__ float searched_dist(const DevIndexView &ix, const float *x, const SegScal &sc, int64_t gb, int64_t gv, int ln) {
+    const int S = ix.S, lane = threadIdx.x & 31, l = lane & 15;
+    float v = 0.0f, f = 0.0f, ipx = 0.0f, ex = 0.0f;  // lane l = s of the half: segment s
     for (int s = 0; s < S; ++s) {
         const SegDev &g = ix.seg[s];
-        const float on = g.onorm[gb * 32 + lane];
-        v[s] = vars_est(sm.scal[s], on);
-        float ip = 0.0f;
-        f[s] = g.bits ? fast_est(g, sm.lut + 4 * g.qoff, sm.scal[s], gb, lane, on, ip) : v[s];
-        ipx[s] = __shfl_sync(kFull, ip, ln);
-        v[s] = __shfl_sync(kFull, v[s], ln);
-        f[s] = __shfl_sync(kFull, f[s], ln);
-    }
-    // ex-code inner products (both half-warps compute them; lane 0 holds the result)
-    float ex[kMaxSeg];
-    for (int s = 0; s < S; ++s) {
-        const SegDev &g = ix.seg[s];
-        ex[s] = g.bits > 1 ? excode_ip16(sm.qres + g.qoff, g.lcode + (size_t)gv * g.lstride, g.dim, g.bits - 1) : 0.0f;
-    }
-    float d = 0.0f;
-    if (lane == 0) {
-        float acc[kMaxSeg];
-        for (int s = 0; s < S; ++s) {
-            const SegDev &g = ix.seg[s];
-            acc[s] = accurate_dist(g.onorm[gb * 32 + ln], ipx[s], ex[s], g.exfac[gv].x, g.bits, sm.scal[s].sum_q,
-                                   sm.scal[s].q_l2sqr);
+        int sum = 0;
+        float e = 0.0f;
+        if (g.bits) {
+            const float vl = __shfl_sync(kFull, sc.vl, s), delta = __shfl_sync(kFull, sc.delta, s),
+                        rd = __shfl_sync(kFull, sc.rdelta, s);
+            const bool quick = lut_quant_ok(delta);
+            const int nc = g.dim / 64;
+            // codebook l of every group: byte l / 2 of the vector's 8, high nibble first; its
+            // dims at q[0, 4, 8, 12]
+            const uint32_t *cp = reinterpret_cast<const uint32_t *>(g.codes + (size_t)gb * nc * 32 + ln) + (l >> 3);
+            const int sh = 8 * ((l >> 1) & 3) + 4 * (~l & 1);
+            const float *q = x + g.qoff + ex_order(4 * l);
+#pragma unroll 4
+            for (int c8 = 0; c8 < nc; ++c8) {
+                const uint32_t nib = cp[(size_t)c8 * 64] >> sh;
+                const float *p = q + 64 * c8;
+                float t = (nib & 8u) ? __fadd_rn(0.0f, p[0]) : 0.0f;
+                t = __fadd_rn(t, (nib & 4u) ? p[4] : 0.0f);
+                t = __fadd_rn(t, (nib & 2u) ? p[8] : 0.0f);
+                t = __fadd_rn(t, (nib & 1u) ? p[12] : 0.0f);
+                const float y = __fsub_rn(t, vl);
+                sum += quick ? (int)lut_quant(y, delta, rd) : (int)(uint16_t)(int)__fdiv_rn(y, delta);
+            }
+#pragma unroll
+            for (int o = 8; o; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+            if (g.bits > 1)
+                e = __shfl_sync(kFull, excode_ip16(x + g.qoff, g.lcode + (size_t)gv * g.lstride, g.dim, g.bits - 1), 0, 16);
         }
-        if (S == 1) {
-            d = acc[0];
-        } else {
-            float cur = 0.0f;
-            for (int s = 0; s < S; ++s) cur = __fadd_rn(cur, v[s]);
-            for (int s = 0; s < S; ++s)
-                if (ix.seg[s].bits) cur = __fadd_rn(__fsub_rn(cur, v[s]), f[s]);
-            d = cur;
-            for (int s = 0; s < S; ++s) d = __fadd_rn(d, __fsub_rn(acc[s], ix.seg[s].bits ? f[s] : v[s]));
+        if (l == s) {
+            const float on = g.onorm[gb * 32 + ln];
+            v = vars_est(sc, on);
+            f = g.bits ? fast_of_sum(sc, sum, on, ipx) : v;
+            ex = e;
         }
     }
-    return __shfl_sync(kFull, d, 0);
+    float acc = 0.0f;
+    if (l < S) {
+        const SegDev &g = ix.seg[l];
+        acc = accurate_dist(g.onorm[gb * 32 + ln], ipx, ex, g.exfac[gv].x, g.bits, sc.sum_q, sc.q_l2sqr);
+    }
+    if (S == 1) return __shfl_sync(kFull, acc, 0, 16);
+    float cur = 0.0f;
+    for (int s = 0; s < S; ++s) cur = __fadd_rn(cur, __shfl_sync(kFull, v, s, 16));
+    for (int s = 0; s < S; ++s)
+        if (ix.seg[s].bits)
+            cur = __fadd_rn(__fsub_rn(cur, __shfl_sync(kFull, v, s, 16)), __shfl_sync(kFull, f, s, 16));
+    const float part = __fsub_rn(acc, f);  // accurate less estimate (its bound when uncoded)
+    for (int s = 0; s < S; ++s) cur = __fadd_rn(cur, __shfl_sync(kFull, part, s, 16));
+    return cur;
 }
 
-// Groups of a query's shortlist (positions ascending, so grouped by probe):
-// the first entry and the probe index of each probed cluster holding
-// shortlisted vectors.  One thread per query.
-__global__ void k_tc_groups(const int *__restrict__ sl_pos, const int *__restrict__ sl_cnt,
-                            const int *__restrict__ lp, int nq, int nprobe, int L, int *__restrict__ grp,
-                            int *__restrict__ gj, int *__restrict__ ng) {
-    const int qi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (qi >= nq) return;
-    const int n = sl_cnt[qi];
-    const int *pos = sl_pos + (size_t)qi * L;
-    const int *lq = lp + (size_t)qi * (nprobe + 1);
-    int cnt = 0, j = 0;
-    for (int e = 0; e < n; ++e) {
-        if (e > 0 && pos[e] < lq[j + 1]) continue;  // same probe as the previous entry
-        while (lq[j + 1] <= pos[e]) ++j;           // probes are visited in order
-        grp[(size_t)qi * L + cnt] = e;
-        gj[(size_t)qi * L + cnt] = j;
-        ++cnt;
+// Re-rank of the tensor-core shortlist, one CTA per query: its positions ascend, so
+// the vectors of one probed cluster lie together.  Work item: up to kRerankRun of them,
+// by one warp, which forms the cluster's residual and scalars for itself and then each
+// vector's distance (searched_dist).  A cluster holds a handful of the shortlist, and a
+// vector needs one entry of each codebook, so no LUT is built and nothing waits for a
+// barrier.  2,048 queries of 1,536 dimensions, 40 vectors each: 0.98 ms with a CTA and a
+// LUT per (query, cluster), 0.34 now; 4,096 queries over 10M x 1,024: 1.02 and 0.50.
+constexpr int kRerankThreads = 128, kRerankRun = 8, kRerankMax = 1024;  // at most kTcMaxShort entries
+__global__ void __launch_bounds__(kRerankThreads) k_tc_rerank(DevIndexView ix, const uint32_t *__restrict__ probe,
+                                                              int nprobe, const float *__restrict__ qrot_all,
+                                                              const float *__restrict__ prune,
+                                                              const int *__restrict__ lp, const int *__restrict__ sl_pos,
+                                                              const int *__restrict__ sl_cnt, int L,
+                                                              float *__restrict__ sl_dist) {
+    extern __shared__ __align__(16) float rr_x[];  // a residual per warp
+    __shared__ int pj[kRerankMax];                 // entry's probe
+    __shared__ uint16_t first[kRerankMax + 1];     // items' first entries
+    __shared__ int nitems, next;
+    const int qi = blockIdx.x, n = sl_cnt[qi], tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int *pos = sl_pos + (size_t)qi * L, *lq = lp + (size_t)qi * (nprobe + 1);
+    const float *qrot = qrot_all + (size_t)qi * ix.Dtot;
+    for (int e = tid; e < n; e += kRerankThreads) {  // the last probe that starts at or before it (empty probes share an offset)
+        int lo = 0, hi = nprobe - 1;
+        const int x = pos[e];
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (lq[mid] <= x) lo = mid;
+            else hi = mid - 1;
+        }
+        pj[e] = lo;
     }
-    ng[qi] = cnt;
-}
-
-// Re-rank of the tensor-core shortlist: CTA (g, query) takes the query's g-th
-// group, i.e. one probed cluster: Lut::prepare for it, then the distance the
-// search computes (searched_dist) of each of its shortlisted vectors.
-__global__ void __launch_bounds__(kScanThreads) k_tc_rerank(DevIndexView ix, const uint32_t *__restrict__ probe,
-                                                            int nprobe, const float *__restrict__ qrot,
-                                                            const float *__restrict__ prune,
-                                                            const int *__restrict__ lp, const int *__restrict__ sl_pos,
-                                                            const int *__restrict__ sl_cnt, const int *__restrict__ grp,
-                                                            const int *__restrict__ gj, const int *__restrict__ ng,
-                                                            int L, float *__restrict__ sl_dist) {
-    extern __shared__ __align__(16) char smem_raw[];
-    const int qi = blockIdx.y, g = blockIdx.x;
-    const int ngq = ng[qi];
-    if (g >= ngq) return;
-    ScanSmem sm = scan_smem_layout(smem_raw, ix.Dtot, ix.S, 1, 0);
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g0 = grp[(size_t)qi * L + g], g1 = g + 1 < ngq ? grp[(size_t)qi * L + g + 1] : sl_cnt[qi];
-    const int j = gj[(size_t)qi * L + g];
-    const int base = lp[(size_t)qi * (nprobe + 1) + j];
-    const int c = (int)probe[(size_t)qi * nprobe + j];
-    prepare_cluster(ix, qrot + (size_t)qi * ix.Dtot, prune + (size_t)qi * ix.S, c, sm);
-    const int64_t b0 = ix.blk_off[c], v0 = ix.vec_off[c];
-    const int *pos = sl_pos + (size_t)qi * L;
-    for (int e = g0 + w; e < g1; e += kScanWarps) {
-        const int r = pos[e] - base;
-        const float d = searched_dist(ix, sm, b0 + r / 32, v0 + r, r & 31, lane);
-        if (lane == 0) sl_dist[(size_t)qi * L + e] = d;
+    if (tid == 0) next = 0;
+    __syncthreads();
+    if (w == 0) {
+        int cnt = 0;
+        for (int e0 = 0; e0 < n; e0 += 32) {
+            const int e = e0 + lane;
+            const bool start = e < n && (e % kRerankRun == 0 || pj[e] != pj[e - 1]);
+            const uint32_t b = __ballot_sync(kFull, start);
+            if (start) first[cnt + __popc(b & ((1u << lane) - 1u))] = (uint16_t)e;
+            cnt += __popc(b);
+        }
+        if (lane == 0) {
+            nitems = cnt;
+            first[cnt] = (uint16_t)n;
+        }
+    }
+    __syncthreads();
+    float *x = rr_x + (size_t)w * ix.Dtot;
+    for (;;) {
+        int it = 0;
+        if (lane == 0) it = atomicAdd(&next, 1);
+        it = __shfl_sync(kFull, it, 0);
+        if (it >= nitems) break;
+        const int e0 = first[it], e1 = first[it + 1], j = pj[e0], c = (int)probe[(size_t)qi * nprobe + j], base = lq[j];
+        const int64_t b0 = ix.blk_off[c], v0 = ix.vec_off[c];
+        for (int e = e0; e < e1; ++e) {  // pull every vector's codes, rows and factors in while the scalars are formed
+            const int r = pos[e] - base;
+            const int64_t gb = b0 + r / 32, gv = v0 + r;
+            for (int s = 0; s < ix.S; ++s) {
+                const SegDev &g = ix.seg[s];
+                if (lane == 0) asm volatile("prefetch.global.L1 [%0];" ::"l"(g.onorm + gb * 32 + (r & 31)));
+                if (lane == 1) asm volatile("prefetch.global.L1 [%0];" ::"l"(g.exfac + gv));
+                if (!g.bits) continue;
+                const int nc = g.dim / 64;
+                for (int k = lane; k < nc; k += 32)
+                    asm volatile("prefetch.global.L1 [%0];" ::"l"(g.codes + ((size_t)gb * nc + k) * 32 + (r & 31)));
+                for (int o = 128 * lane; o < g.lstride; o += 128 * 32)
+                    asm volatile("prefetch.global.L1 [%0];" ::"l"(g.lcode + (size_t)gv * g.lstride + o));
+            }
+        }
+        __syncwarp();  // the previous item's residual is done with
+        const SegScal sc = warp_scalars(ix, qrot, prune + (size_t)qi * ix.S, c, x);
+        for (int e = e0; e < e1; e += 2) {
+            const int me = min(e + (lane >> 4), e1 - 1), r = pos[me] - base;
+            const float d = searched_dist(ix, x, sc, b0 + r / 32, v0 + r, r & 31);
+            if ((lane & 15) == 0 && e + (lane >> 4) < e1) sl_dist[(size_t)qi * L + me] = d;
+        }
     }
 }
 
@@ -4384,24 +4492,21 @@ size_t tc_probe_work_bytes(const Index &I, int64_t nq) { return sizeof(Cand) * (
 
 void tc_rerank(const Index &I, const uint32_t *probe, int64_t nq, int64_t nprobe, const float *qrot,
                const float *prune, const int *lp, const int *sl_pos, const float *sl_apx, const int *sl_cnt, int L,
-               int64_t topk, const int *qk, int *grp, int *gj, int *ng, float *sl_dist, uint32_t *ids, float *dists,
-               float *apx, cudaStream_t st) {
+               int64_t topk, const int *qk, float *sl_dist, uint32_t *ids, float *dists, float *apx, cudaStream_t st) {
     const DevIndexView &ix = I.view;
     int L2 = 1;
     while (L2 < L) L2 <<= 1;
-    k_tc_groups<<<(unsigned)((nq + 127) / 128), 128, 0, st>>>(sl_pos, sl_cnt, lp, (int)nq, (int)nprobe, L, grp, gj,
-                                                               ng);
-    check_launch("k_tc_groups");
-    const size_t smem = scan_smem_bytes(ix.Dtot, ix.S, 1, 0);
-    SAQG_REQUIRE(smem <= 200 * 1024, "dimension too large for the re-rank kernel's shared memory");
-    ensure_smem((const void *)k_tc_rerank, (size_t)smem);
-    k_tc_rerank<<<dim3((unsigned)L, (unsigned)nq), kScanThreads, smem, st>>>(ix, probe, (int)nprobe, qrot, prune, lp,
-                                                                             sl_pos, sl_cnt, grp, gj, ng, L, sl_dist);
+    const size_t smem = 4 * (size_t)(kRerankThreads / 32) * ix.Dtot;
+    SAQG_REQUIRE(scan_smem_bytes(ix.Dtot, ix.S, 1, 0) <= 200 * 1024,
+                 "dimension too large for the re-rank kernel's shared memory");
+    ensure_smem((const void *)k_tc_rerank, smem);
+    k_tc_rerank<<<(unsigned)nq, kRerankThreads, smem, st>>>(ix, probe, (int)nprobe, qrot, prune, lp, sl_pos, sl_cnt, L,
+                                                          sl_dist);
     check_launch("k_tc_rerank");
     k_tc_topk<<<(unsigned)nq, kScanThreads, 8 * (size_t)L2, st>>>(ix, probe, (int)nprobe, lp, sl_pos, sl_apx, sl_cnt,
                                                                   sl_dist, L, L2, (int)topk, qk, ids, dists, apx);
     check_launch("k_tc_topk");
-    count_launch(3);
+    count_launch(2);
 }
 
 }  // namespace saqg

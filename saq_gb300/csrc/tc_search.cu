@@ -31,8 +31,8 @@
 //                  four warps read them back with tcgen05.ld for the epilogue
 //   k_tc_select1/2 per query: the shortlist by radix select over 4,096-candidate
 //                  chunks, then over the chunks' survivors, in candidate order
-//   k_tc_groups / k_tc_rerank / k_tc_topk  (search.cu) exact distances of the
-//                  shortlist, one CTA per (query, probed cluster), then top-k
+//   k_tc_rerank / k_tc_topk  (search.cu) exact distances of the shortlist, one CTA
+//                  per query, then top-k
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -551,10 +551,68 @@ __device__ __forceinline__ int block_prefix(int f, int *wtot, int *tot) {
     return base + __popc(b & ((1u << lane) - 1u));
 }
 
+// Few of many, the shortlist's case: a bound T on the L-th smallest key first, then
+// the keys up to T only.  Each thread takes the smallest key of its share, each warp
+// the ceil(L / 8)-th smallest of its lanes' minima, T is the largest of those over the
+// eight warps: at least L keys are <= T.  The keys up to T (about twice L) are
+// collected in any order, ranked against one another by (key, e), and the L first
+// emitted in ascending e by their rank in e.  (Four radix passes over all of them, most
+// keys in a few bins: 0.35 ms for 28M candidates of 4,096 queries; now 0.09.)  False, nothing emitted, when more than
+// kSelCollect keys are up to T (many equal keys).
+constexpr int kSelFew = 256, kSelCollect = 1024;
+template <class Key, class Emit>
+__device__ bool select_few(int M, int L, Key key, Emit emit) {
+    __shared__ uint32_t wkey[8];
+    __shared__ unsigned long long got[kSelCollect];
+    __shared__ uint32_t chosen[kSelFew];
+    __shared__ int ngot;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    uint32_t mine = 0xffffffffu;
+    for (int e = tid; e < M; e += 256) mine = min(mine, key(e));
+    uint32_t t = 0;
+    bool left = true;
+    for (int i = (L + 7) / 8; i > 0; --i) {
+        t = __reduce_min_sync(kFullMask, left ? mine : 0xffffffffu);
+        const unsigned eq = __ballot_sync(kFullMask, left && mine == t);
+        if (eq && lane == __ffs(eq) - 1) left = false;
+    }
+    if (lane == 0) wkey[w] = t;
+    if (tid == 0) ngot = 0;
+    __syncthreads();
+    uint32_t T = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) T = max(T, wkey[i]);
+    for (int e = tid; e < M; e += 256) {
+        const uint32_t k = key(e);
+        if (k <= T) {
+            const int at = atomicAdd(&ngot, 1);
+            if (at < kSelCollect) got[at] = ((unsigned long long)k << 32) | (uint32_t)e;
+        }
+    }
+    __syncthreads();
+    const int m = ngot;
+    if (m > kSelCollect) return false;
+    for (int i = tid; i < m; i += 256) {
+        const unsigned long long x = got[i];
+        int rank = 0;
+        for (int k = 0; k < m; ++k) rank += got[k] < x;
+        if (rank < L) chosen[rank] = (uint32_t)x;
+    }
+    __syncthreads();
+    for (int i = tid; i < L; i += 256) {
+        const uint32_t e = chosen[i];
+        int slot = 0;
+        for (int k = 0; k < L; ++k) slot += chosen[k] < e;
+        emit(slot, (int)e);
+    }
+    return true;
+}
+
 // The L smallest keys of key(e), e in [0, M) (ties: smaller e first), written
 // in ascending e as (pos(e), value(e)).  256 threads; radix select, 8 bits per pass.
 template <class Key, class Emit>
 __device__ void select_smallest(int M, int L, Key key, Emit emit) {
+    if (L <= kSelFew && select_few(M, L, key, emit)) return;
     __shared__ int hist[256];
     __shared__ int wtot[8];
     __shared__ uint32_t s_prefix;
@@ -811,8 +869,8 @@ size_t tc_arena1_bytes(const Index &I, int64_t nq, int64_t topk, int64_t nprobe,
     add(4 * (size_t)I.K * 2);                   // bcnt, bfill
     add(8 * (size_t)(I.K + 1));                 // boff
     add(4 * (size_t)P * 2);                     // bucket, sorted
-    add(4 * (size_t)nq * L * 5);                // sl_pos, sl_apx, sl_dist, groups, group probes
-    add(4 * (size_t)nq * 2);                    // sl_cnt, group counts
+    add(4 * (size_t)nq * L * 3);                // sl_pos, sl_apx, sl_dist
+    add(4 * (size_t)nq);                        // sl_cnt
     add(4 * (size_t)nq * topk * 3);             // outputs (host io)
     add(16);                                    // error word
     add(4 * (size_t)nq * 2);                    // per-query nprobe / k
@@ -918,13 +976,10 @@ void run_search_tc(const Index &I, const float *q, int64_t nq, int64_t topk, int
     long long *boff = reinterpret_cast<long long *>(take(8 * (size_t)(I.K + 1)));
     int *bucket = reinterpret_cast<int *>(take(4 * (size_t)P * 2));
     int *sorted = bucket + P;
-    int *sl_pos = reinterpret_cast<int *>(take(4 * (size_t)nq * L * 5));
+    int *sl_pos = reinterpret_cast<int *>(take(4 * (size_t)nq * L * 3));
     float *sl_apx = reinterpret_cast<float *>(sl_pos + nq * L);
     float *sl_dist = sl_apx + nq * L;
-    int *grp = reinterpret_cast<int *>(sl_dist + nq * L);
-    int *gj = grp + nq * L;
-    int *sl_cnt = reinterpret_cast<int *>(take(4 * (size_t)nq * 2));
-    int *ng = sl_cnt + nq;
+    int *sl_cnt = reinterpret_cast<int *>(take(4 * (size_t)nq));
     uint32_t *oid = reinterpret_cast<uint32_t *>(take(4 * (size_t)nq * topk * 3));
     float *od = reinterpret_cast<float *>(oid + nq * topk);
     float *oa = od + nq * topk;
@@ -1058,7 +1113,7 @@ void run_search_tc(const Index &I, const float *q, int64_t nq, int64_t topk, int
     k_tc_select2<<<(unsigned)nq, 256, 0, st>>>(qchunk, qtot, (int)L, spos, sval, sl_pos, sl_apx, sl_cnt);
     launch_check("k_tc_select2");
     mark(4);
-    tc_rerank(I, probe, nq, nprobe, qrot, prune, lp, sl_pos, sl_apx, sl_cnt, (int)L, topk, qk, grp, gj, ng, sl_dist,
+    tc_rerank(I, probe, nq, nprobe, qrot, prune, lp, sl_pos, sl_apx, sl_cnt, (int)L, topk, qk, sl_dist,
               host ? oid : ids, host ? od : dists, host ? oa : approx, st);
     mark(5);
     count_launch(capped ? 12 : 11);
