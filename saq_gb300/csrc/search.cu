@@ -4473,18 +4473,27 @@ void tc_rank_rotate(const Index &I, SearchCtx &C, const float *q, int64_t nq, in
     const DevIndexView &ix = I.view;
     SAQG_CUDA_TRY(cudaMemsetAsync(flags, 0, 64, st));
     Cand *wk = static_cast<Cand *>(work);
+    // the rotation runs on the context's least-priority stream beside the ranking, as in run_search
+    auto fork_qprep = [&]() {
+        cudaStream_t qs = C.low_stream();
+        SAQG_CUDA_TRY(cudaEventRecord(C.qfork_event(), st));
+        SAQG_CUDA_TRY(cudaStreamWaitEvent(qs, C.qfork_event(), 0));
+        launch_qprep(ix, q, nq, m, qrot, prune, qs);
+        SAQG_CUDA_TRY(cudaEventRecord(C.qjoin_event(), qs));
+    };
     const char *pm = std::getenv("SAQG_PROBE");
     const bool shortlist = nq >= kGemmMinQueries && nprobe <= kShortCap && !(pm && std::string(pm) == "exact");
     if (shortlist) {
-        probe_shortlist(I, C, q, nq, nprobe, qnp, dist, probe, full, fb_list, flags, wk, nullptr, qbf, st);
+        probe_shortlist(I, C, q, nq, nprobe, qnp, dist, probe, full, fb_list, flags, wk, nullptr, qbf, st, fork_qprep);
     } else {
+        fork_qprep();
         k_probe_dist<<<dim3((unsigned)((I.K + 7) / 8), (unsigned)nq), 256, 0, st>>>(ix, q, dist);
         check_launch("k_probe_dist");
         k_probe_select<<<(unsigned)nq, kSelThreads, 0, st>>>(dist, (int)I.K, (int)nprobe, probe, wk, flags, nullptr,
                                                               qnp);
         check_launch("k_probe_select");
     }
-    launch_qprep(ix, q, nq, m, qrot, prune, st);
+    SAQG_CUDA_TRY(cudaStreamWaitEvent(st, C.qjoin_event(), 0));  // the rotated queries
     count_launch(4);
 }
 

@@ -320,6 +320,58 @@ struct TcWork {
     int skip_it;
 };
 
+// A CTA's tiles in its order (every gridDim.x-th), read ahead: the tile after next's
+// entry and the next one's counts and offsets are in flight while the current tile is
+// worked on, so that no role waits for two dependent loads between tiles (a tile's
+// stages take 6 us at HBM's rate, such a pair over 1).  Tiles of clusters without pairs
+// are passed over.
+struct TileWalk {
+    const DevIndexView &ix;
+    const TcWork &w;
+    int ti;           // the current tile's index
+    int2 cur, nxt, nn;
+    int cnt, ncnt;
+    int64_t v0, nv0;  // first vector of the tile's cluster
+    long long rb, nrb;
+    __device__ __forceinline__ int2 entry(int t) const { return t < w.ntiles ? w.tiles[t] : make_int2(-1, 0); }
+    __device__ __forceinline__ void fetch(const int2 &t, int &c, int64_t &v, long long &r) const {
+        c = 0;
+        v = 0;
+        r = 0;
+        if (t.x >= 0) {
+            c = w.bcnt[t.x];
+            v = ix.vec_off[t.x];
+            r = w.boff[t.x];
+        }
+    }
+    __device__ __forceinline__ TileWalk(const DevIndexView &ix_, const TcWork &w_) : ix(ix_), w(w_), ti(blockIdx.x) {
+        cur = entry(ti);
+        nxt = entry(ti + gridDim.x);
+        nn = entry(ti + 2 * gridDim.x);
+        fetch(cur, cnt, v0, rb);
+        fetch(nxt, ncnt, nv0, nrb);
+        settle();
+    }
+    __device__ __forceinline__ void step() {
+        ti += gridDim.x;
+        cur = nxt;
+        cnt = ncnt;
+        v0 = nv0;
+        rb = nrb;
+        nxt = nn;
+        fetch(nxt, ncnt, nv0, nrb);
+        nn = entry(ti + 2 * gridDim.x);
+    }
+    __device__ __forceinline__ void settle() {
+        while (more() && cnt == 0) step();
+    }
+    __device__ __forceinline__ bool more() const { return ti < w.ntiles; }
+    __device__ __forceinline__ void next() {
+        step();
+        settle();
+    }
+};
+
 // Persistent contraction, one CTA per SM, tiles round-robin.  Roles:
 //   warp 0 (one thread)  TMA: per 64-dim stage the 128-row code tile and the
 //                        chunk's query rows (16-row boxes), into a 6-stage ring
@@ -384,13 +436,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_contract(const __grid_cons
         if (lane == 0) {
             int it = 0;
             bool ok = true;
-            for (int ti = blockIdx.x; ti < w.ntiles && ok; ti += gridDim.x) {
-                const int2 tile = w.tiles[ti];
-                const int cnt = w.bcnt[tile.x];
-                const int row0 = (int)(ix.vec_off[tile.x] + (int64_t)tile.y * kTcBM);
+            for (TileWalk t(ix, w); t.more() && ok; t.next()) {
+                const int cnt = t.cnt;
+                const int row0 = (int)(t.v0 + (int64_t)t.cur.y * kTcBM);
                 for (int ch = 0; ch * BN < cnt && ok; ++ch) {
                     const int nh = min(BN, cnt - ch * BN), npad = (nh + 15) & ~15;
-                    const int brow = (int)(w.boff[tile.x] + (long long)ch * BN);
+                    const int brow = (int)(t.rb + (long long)ch * BN);
                     for (int kc = 0; kc < kch; ++kc, ++it) {
                         const int st = it % kTcStages;
                         const uint32_t ph = (uint32_t)(it / kTcStages) & 1u;
@@ -418,8 +469,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_contract(const __grid_cons
         if (lane == 0) {
             int it = 0, g = 0;
             bool ok = true;
-            for (int ti = blockIdx.x; ti < w.ntiles && ok; ti += gridDim.x) {
-                const int cnt = w.bcnt[w.tiles[ti].x];
+            for (TileWalk t(ix, w); t.more() && ok; t.next()) {
+                const int cnt = t.cnt;
                 for (int ch = 0; ch * BN < cnt && ok; ++ch, ++g) {
                     const int nh = min(BN, cnt - ch * BN), npad = (nh + 15) & ~15;
                     const uint32_t idesc = idesc_bf16(npad);
@@ -462,11 +513,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_contract(const __grid_cons
         const int qt = warp & 3, r = qt * 32 + lane;
         int g = 0;
         bool ok = true;
-        for (int ti = blockIdx.x; ti < w.ntiles && ok; ti += gridDim.x) {
-            const int2 tile = w.tiles[ti];
-            const int c = tile.x, cnt = w.bcnt[c];
-            if (cnt == 0) continue;
-            const int64_t v0 = ix.vec_off[c];
+        for (TileWalk t(ix, w); t.more() && ok; t.next()) {
+            const int2 tile = t.cur;
+            const int c = tile.x, cnt = t.cnt;
+            const int64_t v0 = t.v0;
             const int nc = (int)(ix.vec_off[c + 1] - v0);
             const int rl = tile.y * kTcBM + r;
             const bool vrow = rl < nc;
@@ -481,7 +531,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_contract(const __grid_cons
                     ok = false;
                     break;
                 }
-                const long long rb = w.boff[c] + (long long)ch * BN;
+                const long long rb = t.rb + (long long)ch * BN;
                 for (int n0 = 0; n0 < npad; n0 += 16) {
                     float d[16];
 #pragma unroll
