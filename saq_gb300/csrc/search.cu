@@ -2362,7 +2362,12 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) k_scan_warp(DevIndexView ix
 // order.  A final pass per query walks the positions in order and replays the
 // reference's decisions on the records.  Blocks without a record cannot insert
 // anything (none of their lanes is below tau1 >= distk), so the replay is exact.
+// Blocks of a speculative tile (one warp's work): 16 for deferred queries, 4 when a few
+// queries have the GPU alone.  One query over 32 probes of 3-4 blocks has 32 tiles
+// either way, but over 32 x 31 blocks 64 tiles of 16 leave half of the SMs idle; tiles of 4
+// and the ids in the records: 131 to 123 us (host call), 37 queries 1.74 to 1.59 ms.
 constexpr int kTileBlocks = 16;
+constexpr int kFewTileBlocks = 4;
 constexpr int kFirstBlocks = 16;  // exact prefix of a deferred query (its distk bounds the first level)
 // Levels of the speculation for deferred queries, in tiles after the split
 // point: [0, 8), [8, 64), [64, end) by default; the autotuner may pick another
@@ -2415,6 +2420,7 @@ struct SplitState {
     // point of each query (distk at the level's start bounds its speculation)
     int t_lo, t_hi;
     int final_level;     // the last level writes the results, the others the pool
+    int tile_blocks;     // blocks of a speculative tile (kFewTileBlocks or kTileBlocks)
 };
 
 // Scan-order position of the first block of tile t after a query's split
@@ -2430,10 +2436,15 @@ __device__ __forceinline__ int tile_pos(const SplitState &st, int slot, int t) {
         else hi = mid;
     }
     const int first = lo == st.split_p[slot] ? st.split_b[slot] : 0;
-    return st.blk_base[(size_t)slot * npm + lo] + first + (t - to[lo]) * kTileBlocks;
+    return st.blk_base[(size_t)slot * npm + lo] + first + (t - to[lo]) * st.tile_blocks;
 }
 
-__host__ __device__ inline int rec_words_of(int S) { return (8 + (S + 1) + 32 + 32 * S + 3) & ~3; }
+// Words of a record: 8 of header, S + 1 stage minima, the 32 estimates, 32 partials per
+// segment, the 32 ids (so that the replay reads nothing but staged records).
+__host__ __device__ inline int rec_words_of(int S) { return (8 + (S + 1) + 32 + 32 * S + 32 + 3) & ~3; }
+__device__ __forceinline__ const uint32_t *rec_ids(const float *rec, int S) {
+    return reinterpret_cast<const uint32_t *>(rec) + 8 + (S + 1) + 32 + 32 * S;
+}
 
 __device__ __forceinline__ int list_len(const SplitState &st) { return min(*st.nlist, st.cap); }
 
@@ -2504,19 +2515,39 @@ __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan_first(DevIn
             st.tau[slot] = distk;
             st.split_p[slot] = sp_p;
             st.split_b[slot] = sp_b;
+        }
+        if (tid < 32) {  // tiles and blocks before each probe: prefix sums over the warp's lanes
             int tiles = 0;
             int64_t pos = 0;
-            for (int p = 0; p < nprobe; ++p) {
-                const int c = (int)pr[p];
-                const int nb = (int)(ix.blk_off[c + 1] - ix.blk_off[c]);
-                st.tile_off[(size_t)slot * (np_max + 1) + p] = tiles;
-                st.blk_base[(size_t)slot * np_max + p] = (int)pos;
-                const int rest = p < sp_p ? 0 : p == sp_p ? nb - sp_b : nb;
-                tiles += (rest + kTileBlocks - 1) / kTileBlocks;
-                pos += nb;
+            for (int p0 = 0; p0 < nprobe; p0 += 32) {
+                const int p = p0 + tid;
+                int nb = 0, nt = 0;
+                if (p < nprobe) {
+                    const int c = (int)pr[p];
+                    nb = (int)(ix.blk_off[c + 1] - ix.blk_off[c]);
+                    const int rest = p < sp_p ? 0 : p == sp_p ? nb - sp_b : nb;
+                    nt = (rest + st.tile_blocks - 1) / st.tile_blocks;
+                }
+                int xt = nt;
+                int64_t xb = nb;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int yt = __shfl_up_sync(kFull, xt, o);
+                    const int64_t yb = __shfl_up_sync(kFull, xb, o);
+                    if (tid >= o) {
+                        xt += yt;
+                        xb += yb;
+                    }
+                }
+                if (p < nprobe) {
+                    st.tile_off[(size_t)slot * (np_max + 1) + p] = tiles + xt - nt;
+                    st.blk_base[(size_t)slot * np_max + p] = (int)(pos + xb - nb);
+                }
+                tiles += __shfl_sync(kFull, xt, 31);
+                pos += __shfl_sync(kFull, xb, 31);
             }
-            for (int p = nprobe; p <= np_max; ++p) st.tile_off[(size_t)slot * (np_max + 1) + p] = tiles;
-            if (pos != st.npos[slot]) *err = 2;
+            for (int p = nprobe + tid; p <= np_max; p += 32) st.tile_off[(size_t)slot * (np_max + 1) + p] = tiles;
+            if (tid == 0 && pos != st.npos[slot]) *err = 2;
         }
         __syncthreads();  // the next slot reuses the shared state
     }
@@ -2629,8 +2660,8 @@ __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan_spec(DevInd
             t.v0 = ix.vec_off[t.c];
             t.nb = (int)(ix.blk_off[t.c + 1] - t.b0);
             t.n = (int)(ix.vec_off[t.c + 1] - t.v0);
-            t.first = (p == st.split_p[slot] ? st.split_b[slot] : 0) + (local - to[p]) * kTileBlocks;
-            t.blocks = min(kTileBlocks, t.nb - t.first);
+            t.first = (p == st.split_p[slot] ? st.split_b[slot] : 0) + (local - to[p]) * st.tile_blocks;
+            t.blocks = min(st.tile_blocks, t.nb - t.first);
             t.tau = st.tau[slot];
             t.pos = st.blk_base[(size_t)slot * nprobe + p];
             t.left = (1u << t.blocks) - 1u;
@@ -2646,7 +2677,7 @@ __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan_spec(DevInd
                 }
                 __syncwarp();
                 uint32_t left = 0;
-                for (int g = 0; g < kTileBlocks / kQuad; g += 2) {
+                for (int g = 0; kQuad * g < t.blocks; g += 2) {
                     const float *const fvs[2] = {fv, fv};
                     const int64_t gb[2] = {t.b0 + t.first + kQuad * g, t.b0 + t.first + kQuad * g + kQuad};
                     const int nv[2] = {t.blocks - kQuad * g, t.blocks - kQuad * g - kQuad};  // past the tile: none
@@ -2726,6 +2757,7 @@ __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan_spec(DevInd
                     if (S > 1 && lane <= S) r[8 + lane] = sm.stage[wslot * (S + 1) + lane];
                     r[8 + (S + 1) + lane] = sm.cur[wslot * 32 + lane];
                     for (int s = 0; s < S; ++s) r[8 + (S + 1) + 32 + s * 32 + lane] = sm.part[(wslot * S + s) * 32 + lane];
+                    ri[8 + (S + 1) + 32 + 32 * S + lane] = in ? ix.ids[t.v0 + (int64_t)b * 32 + lane] : 0u;
                 }
             }
             __syncthreads();
@@ -2927,12 +2959,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
                         int c;
                         const float *rec = buf + (size_t)r * RW;
                         const bool e = record_effect(S, rec, dk, sz, topk, c);
-                        if (lane == 0) {
-                            eff[r] = e;
-                            const uint32_t *ri = reinterpret_cast<const uint32_t *>(rec);
-                            const int64_t v0 = (int64_t)(((uint64_t)ri[6] << 32) | ri[5]);
-                            if (e) asm volatile("prefetch.global.L1 [%0];" ::"l"(ix.ids + v0 + (int64_t)ri[4] * 32));
-                        }
+                        if (lane == 0) eff[r] = e;
                     }
                     __syncthreads();
                     if (w == 0) {
@@ -2940,7 +2967,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
                         for (; live; live &= live - 1) {
                             const float *rec = buf + (size_t)(__ffs(live) - 1) * RW;
                             const uint32_t *ri = reinterpret_cast<const uint32_t *>(rec);
-                            const uint32_t *rid = ix.ids + (int64_t)(((uint64_t)ri[6] << 32) | ri[5]) + (int64_t)ri[4] * 32;
+                            const uint32_t *rid = rec_ids(rec, S);
                             if (!replay_block_regs(S, rec + 8 + (S + 1), __uint_as_float(ri[7]), rec + 8 + (S + 1) + 32,
                                                    ri[1], rid, P, rr)) {  // a NaN: on the pool in shared memory
                                 P.store(sm.pool_id, sm.pool_d);
@@ -2986,12 +3013,10 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
                         if (rs < cn) {
                             const float *rec = buf + (size_t)rs * RW;
                             const uint32_t *ri = reinterpret_cast<const uint32_t *>(rec);
-                            const int64_t v0 = (int64_t)(((uint64_t)ri[6] << 32) | ri[5]);
                             float dkw = dk;
                             int szw = sz;
-                            replay_block_warp(S, (int)ri[4], rec + 8 + (S + 1), __uint_as_float(ri[7]),
-                                              rec + 8 + (S + 1) + 32, ri[1], ix.ids + v0, sm.pool_id, sm.pool_d, szw, topk,
-                                              dkw, rr);
+                            replay_block_warp(S, 0, rec + 8 + (S + 1), __uint_as_float(ri[7]), rec + 8 + (S + 1) + 32, ri[1],
+                                              rec_ids(rec, S), sm.pool_id, sm.pool_d, szw, topk, dkw, rr);
                             if (lane == 0) {
                                 distk = dkw;
                                 pool_size = szw;
@@ -3110,19 +3135,28 @@ __global__ void __launch_bounds__(kOrderThreads) k_order(DevIndexView ix, const 
 constexpr int kDeferThreads = 1024;
 constexpr int kQblocksMinQueries = 256;  // from this batch size the block counts come from k_qblocks
 
-// Blocks of each query's probes, one thread per query (k_defer's input for
-// large batches, where its single CTA would sum them serially).
-__global__ void k_qblocks(DevIndexView ix, const uint32_t *__restrict__ probe, QueryShape qsh, int nq,
-                          int *__restrict__ qblocks) {
-    const int qi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (qi >= nq) return;
-    int64_t total = 0;
-    const int np = qsh.np_of(qi);
-    for (int p = 0; p < np; ++p) {
+// Blocks of a query's probes (at most INT_MAX), by a warp.
+__device__ __forceinline__ int query_blocks(const DevIndexView &ix, const uint32_t *__restrict__ probe,
+                                            const QueryShape &qsh, int qi) {
+    const int lane = threadIdx.x & 31, np = qsh.np_of(qi);
+    long long total = 0;
+    for (int p = lane; p < np; p += 32) {
         const int c = (int)probe[(size_t)qi * qsh.np_max + p];
         total += ix.blk_off[c + 1] - ix.blk_off[c];
     }
-    qblocks[qi] = total < (int64_t)INT_MAX ? (int)total : INT_MAX;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(kFull, total, o);
+    return total < (long long)INT_MAX ? (int)total : INT_MAX;
+}
+
+// Blocks of each query's probes, one warp per query (k_defer's input for
+// large batches, where its single CTA would sum them one after the other).
+__global__ void __launch_bounds__(256) k_qblocks(DevIndexView ix, const uint32_t *__restrict__ probe, QueryShape qsh,
+                                                 int nq, int *__restrict__ qblocks) {
+    const int qi = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (qi >= nq) return;
+    const int total = query_blocks(ix, probe, qsh, qi);
+    if ((threadIdx.x & 31) == 0) qblocks[qi] = total;
 }
 
 __global__ void __launch_bounds__(kDeferThreads) k_defer(DevIndexView ix, const uint32_t *__restrict__ probe, int nq,
@@ -3134,16 +3168,13 @@ __global__ void __launch_bounds__(kDeferThreads) k_defer(DevIndexView ix, const 
     __shared__ int s_slot;        // list entries handed out
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nt = blockDim.x, nw = nt >> 5;
     const int per = (nq + nt - 1) / nt, q0 = min(nq, tid * per), q1 = min(nq, q0 + per);
-    if (!have_qblocks)
-        for (int qi = q0; qi < q1; ++qi) {
-            int64_t total = 0;
-            const int np = st.qsh.np_of(qi);
-            for (int p = 0; p < np; ++p) {
-                const int c = (int)probe[(size_t)qi * st.qsh.np_max + p];
-                total += ix.blk_off[c + 1] - ix.blk_off[c];
-            }
-            qblocks[qi] = total < (int64_t)INT_MAX ? (int)total : INT_MAX;  // read back by this thread only
+    if (!have_qblocks) {
+        for (int qi = w; qi < nq; qi += nw) {
+            const int total = query_blocks(ix, probe, st.qsh, qi);
+            if (lane == 0) qblocks[qi] = total;
         }
+        __syncthreads();
+    }
     auto eligible = [&](int qi) {
         return defer_blocks < 0 || (defer_blocks > 0 && qblocks[qi] > defer_blocks);
     };
@@ -3868,6 +3899,8 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
             // heavy queries beside a batch: a longer prefix for a tighter bound; a
             // few queries alone: the speculative part has the GPU, so only the pool must fill
             ss.first_blocks = tune.first_blocks > 0 ? tune.first_blocks : (mode == 0 ? kFirstBlocks : 1);
+            // few queries: short tiles, so that they spread over the GPU
+            ss.tile_blocks = mode == 1 ? kFewTileBlocks : kTileBlocks;
             ss.t_lo = 0;
             ss.t_hi = INT_MAX;
             ss.final_level = 1;
@@ -3878,10 +3911,10 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
             SAQG_CUDA_TRY(cudaMemsetAsync(ss.nlist, 0, 32, st));
             int defer = -1;  // mode 1: every query
             if (mode == 0) defer = defer_threshold(tune);
-            const int dthreads = (int)std::min<int64_t>(kDeferThreads, (nq + 31) / 32 * 32);
+            const int dthreads = (int)std::min<int64_t>(kDeferThreads, 32 * nq);  // a warp per query while they fit
             const bool par = nq >= kQblocksMinQueries;
             if (par) {
-                k_qblocks<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(ix, probe, qsh, (int)nq, qblocks);
+                k_qblocks<<<(unsigned)((nq + 7) / 8), 256, 0, st>>>(ix, probe, qsh, (int)nq, qblocks);
                 check_launch("k_qblocks");
             }
             k_defer<<<1, dthreads, 0, st>>>(ix, probe, (int)nq, defer, ss, qblocks, par ? 1 : 0, deferred);
