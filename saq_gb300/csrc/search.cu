@@ -1618,144 +1618,131 @@ __device__ __forceinline__ void replay_block_warp(int S, int bb, const float *cu
     }
 }
 
-// ResultPool (utils/pool.hpp:17-49) of at most 32 kRows entries in a warp's
-// registers, entry 32 r + lane in d[r] / u[r].  An insert costs a ballot per 32
-// entries and a few shuffles, where the pool in shared memory (pool_insert_warp)
-// takes a chain of loads, stores and warp barriers.
+// ResultPool (utils/pool.hpp:17-49) of at most 32 kPer entries in a warp's registers,
+// entry kPer lane + r in d[r] / u[r]; past the size FLT_MAX, so that the k-th entry is
+// distk whether the pool is full or not.  An insert is a shift by one entry under a
+// comparison per entry: the two shuffles of the shift do not wait for the value, and
+// the one of the new distk ends it: 240 cycles.  (With ballots for the position, the size as
+// a counter and the entries spread row by row: 37 queries with k = 100 1.66 ms, now
+// 1.54; in shared memory, pool_insert_warp, over a thousand cycles an insert.)
 constexpr int kRegPool = 128;  // largest k whose pool is held so
-template <int kRows>
+template <int kPer>
 struct RegPool {
-    float d[kRows], dk;
-    uint32_t u[kRows];
-    int sz, cap;
-    bool nan;  // an entry is NaN: the order is not total, replay_block_warp takes over
-    __device__ __forceinline__ void load(const uint32_t *pid, const float *pd, int size, int topk, float distk) {
-        const int lane = threadIdx.x & 31;
-        sz = size;
-        cap = topk;
-        dk = distk;
-        bool n = false;
+    float d[kPer], dk;
+    uint32_t u[kPer];
+    int cap;
+    bool odd;  // an entry is not finite: replay_block_warp takes over
+    __device__ __forceinline__ float kth() const {
+        float x = d[0];
 #pragma unroll
-        for (int r = 0; r < kRows; ++r) {
-            const int e = 32 * r + lane;
-            d[r] = e < sz ? pd[e] : 0.0f;
-            u[r] = e < sz ? pid[e] : 0u;
-            n |= d[r] != d[r];
-        }
-        nan = __any_sync(kFull, n);
+        for (int r = 1; r < kPer; ++r)
+            if (r == (cap - 1) % kPer) x = d[r];
+        return __shfl_sync(kFull, x, (cap - 1) / kPer);
     }
-    __device__ __forceinline__ void store(uint32_t *pid, float *pd) const {
+    __device__ __forceinline__ void load(const uint32_t *pid, const float *pd, int size, int topk) {
         const int lane = threadIdx.x & 31;
+        cap = topk;
+        bool bad = false;
 #pragma unroll
-        for (int r = 0; r < kRows; ++r) {
-            const int e = 32 * r + lane;
-            if (e < sz) {
+        for (int r = 0; r < kPer; ++r) {
+            const int e = kPer * lane + r;
+            d[r] = e < size ? pd[e] : FLT_MAX;
+            u[r] = e < size ? pid[e] : 0u;
+            bad |= e < size && !(d[r] < FLT_MAX);
+        }
+        odd = __any_sync(kFull, bad);
+        dk = kth();
+    }
+    __device__ __forceinline__ void store(uint32_t *pid, float *pd, int &size) const {
+        const int lane = threadIdx.x & 31;
+        int n = 0;
+#pragma unroll
+        for (int r = 0; r < kPer; ++r) {
+            const int e = kPer * lane + r;
+            const bool have = e < cap && d[r] < FLT_MAX;
+            if (have) {
                 pd[e] = d[r];
                 pid[e] = u[r];
             }
+            n += __popc(__ballot_sync(kFull, have));
         }
+        size = n;
         __syncwarp();
     }
-    // Inserts `dist` (uniform, no NaN, accepted under dk) and updates dk.
-    __device__ __forceinline__ void insert(uint32_t id, float dist) {
-        const int lane = threadIdx.x & 31;
-        int lo = 0;
+    // Inserts v (uniform, finite, accepted under dk) and updates dk.
+    __device__ __forceinline__ void insert(uint32_t id, float v) {
+        float pv = __shfl_up_sync(kFull, d[kPer - 1], 1);
+        const uint32_t pu = __shfl_up_sync(kFull, u[kPer - 1], 1);
+        if ((threadIdx.x & 31) == 0) pv = __int_as_float(0xff800000);
 #pragma unroll
-        for (int r = 0; r < kRows; ++r)
-            if (r == 0 || 32 * r < sz) lo += __popc(__ballot_sync(kFull, 32 * r + lane < sz && d[r] < dist));
-#pragma unroll
-        for (int r = kRows - 1; r >= 0; --r) {
-            if (r > 0 && (32 * r >= cap || 32 * r + 31 < lo)) continue;
-            float v = __shfl_up_sync(kFull, d[r], 1);
-            uint32_t x = __shfl_up_sync(kFull, u[r], 1);
-            if (r > 0) {
-                const float pv = __shfl_sync(kFull, d[r > 0 ? r - 1 : 0], 31);
-                const uint32_t px = __shfl_sync(kFull, u[r > 0 ? r - 1 : 0], 31);
-                if (lane == 0) {
-                    v = pv;
-                    x = px;
-                }
-            }
-            const int e = 32 * r + lane;
-            d[r] = e > lo ? v : e == lo ? dist : d[r];
-            u[r] = e > lo ? x : e == lo ? id : u[r];
+        for (int r = kPer - 1; r >= 0; --r) {
+            const float prev = r ? d[r > 0 ? r - 1 : 0] : pv;
+            const uint32_t prevu = r ? u[r > 0 ? r - 1 : 0] : pu;
+            const bool keep = d[r] < v, put = prev < v;  // equal entries move up: the later one goes first
+            d[r] = keep ? d[r] : put ? v : prev;
+            u[r] = keep ? u[r] : put ? id : prevu;
         }
-        sz += sz < cap;
-        float last = d[0];
-#pragma unroll
-        for (int r = 1; r < kRows; ++r)
-            if (r == (cap - 1) >> 5) last = d[r];
-        last = __shfl_sync(kFull, last, (cap - 1) & 31);
-        dk = sz == cap ? last : FLT_MAX;
+        dk = kth();
     }
 };
 
 // replay_block_warp on a pool in registers, for at most kRegSegs segments (ids: the
 // block's 32 ids).  A lane's running sums are formed once and stay in registers: while
-// the largest is below dk the reference's loop runs to the last one, which is
-// inserted; otherwise it ends at the first sum >= dk, which is refused under a full
-// pool unless it equals dk.  Returns false, nothing changed, when a NaN is met.
+// the largest is below dk the reference's loop runs to the last one, which is inserted;
+// otherwise it ends at the first sum >= dk, which is refused unless it equals dk.  Returns
+// the lanes not decided: those of a block with a NaN or an infinity, or from the first
+// lane with a sum that equals dk on (for replay_block_warp).  seen(dk): called after each insert.
 constexpr int kRegSegs = 4;
-template <int kRows>
-__device__ __forceinline__ bool replay_block_regs(int S, const float *cur, float smax, const float *part, uint32_t cm,
-                                                  const uint32_t *ids, RegPool<kRows> &P, unsigned long long &c_rr) {
+template <int kPer, class Seen>
+__device__ __forceinline__ uint32_t replay_block_regs(int S, const float *cur, float smax, const float *part, uint32_t cm,
+                                                      const uint32_t *ids, RegPool<kPer> &P, Seen seen) {
     const int lane = threadIdx.x & 31;
-    if (!cm || (S > 1 && smax > P.dk)) return true;
+    if (P.odd) return cm;
+    if (!cm || (S > 1 && smax > P.dk)) return 0u;
     const bool in = (cm >> lane) & 1u;
     const uint32_t id = in ? ids[lane] : 0u;
     const float c = in ? cur[lane] : FLT_MAX;
-    float x[kRegSegs];
-#pragma unroll
-    for (int s = 0; s < kRegSegs; ++s) x[s] = in && s < S ? part[s * 32 + lane] : 0.0f;
-    if (S == 1) {
-        const float a = in ? x[0] : FLT_MAX;
-        if (P.nan || __any_sync(kFull, a != a)) return false;
-        uint32_t rest = __ballot_sync(kFull, in && c < P.dk);  // the mask, at the block's start
-        c_rr += __popc(rest);
-        while (rest) {
-            const uint32_t ok = rest & __ballot_sync(kFull, !(P.sz == P.cap && a > P.dk));
-            if (!ok) break;
-            const int j = __ffs(ok) - 1;
-            P.insert(__shfl_sync(kFull, id, j), __shfl_sync(kFull, a, j));
-            rest &= ~((2u << j) - 1u);
-        }
-        return true;
-    }
-    float sum[kRegSegs], top, last = c;
+    float sum[kRegSegs], top = 0.0f, last = c;
 #pragma unroll
     for (int s = 0; s < kRegSegs; ++s) {
-        if (s < S) last = __fadd_rn(last, x[s]);
+        if (in && s < S) {
+            const float x = part[s * 32 + lane];
+            last = S == 1 ? x : __fadd_rn(last, x);
+        }
         sum[s] = last;  // past the last segment: the last sum again
         top = s == 0 ? last : fmaxf(top, last);
     }
-    bool nan = false;  // a NaN stays one in the later sums
-    nan = last != last;
-    if (P.nan || __any_sync(kFull, in && nan)) return false;
+    const float gate = fmaxf(c, top);
+    // (a NaN stays one in the later sums)
+    if (__any_sync(kFull, in && !(gate < FLT_MAX && last < FLT_MAX))) return cm;
+    if (S == 1) {
+        uint32_t rest = __ballot_sync(kFull, in && c < P.dk);  // the mask, at the block's start
+        while (rest) {
+            const uint32_t ok = rest & __ballot_sync(kFull, last <= P.dk);
+            if (!ok) break;
+            const int j = __ffs(ok) - 1;
+            P.insert(__shfl_sync(kFull, id, j), __shfl_sync(kFull, last, j));
+            seen(P.dk);
+            rest &= ~((2u << j) - 1u);
+        }
+        return 0u;
+    }
     uint32_t rest = cm;
-    do {
+    while (rest) {
         const float dk = P.dk;
-        const bool full = P.sz == P.cap;
-        const uint32_t pass = rest & __ballot_sync(kFull, c < dk);
-        // the value the lane inserts: the last sum, or the first at or above dk
-        float acc = last;
-        bool taken = top < dk;
-        if (!taken) {
+        bool tie = false;
 #pragma unroll
-            for (int s = kRegSegs - 1; s >= 0; --s)
-                if (sum[s] >= dk) acc = sum[s];
-            taken = !(full && acc > dk);
-        }
-        const uint32_t ok = pass & __ballot_sync(kFull, taken);
-        if (!ok) {
-            c_rr += __popc(pass);
-            break;
-        }
-        const int j = __ffs(ok) - 1;
-        c_rr += __popc(pass & ((2u << j) - 1u));
-        P.insert(__shfl_sync(kFull, id, j), __shfl_sync(kFull, acc, j));
+        for (int s = 0; s < kRegSegs; ++s) tie |= sum[s] == dk;
+        const uint32_t less = __ballot_sync(kFull, gate < dk), ties = rest & __ballot_sync(kFull, tie && c < dk);
+        const uint32_t hit = (rest & less) | ties;
+        if (!hit) break;
+        const int j = __ffs(hit) - 1;
+        if ((ties >> j) & 1u) return rest & ~((1u << j) - 1u);
+        P.insert(__shfl_sync(kFull, id, j), __shfl_sync(kFull, last, j));
+        seen(P.dk);
         rest &= ~((2u << j) - 1u);
-    } while (rest);
-    return true;
+    }
+    return 0u;
 }
 
 // The reference's decisions for the nblk (<= 32) blocks of a tile, in order, by
@@ -1768,7 +1755,7 @@ __device__ __forceinline__ bool replay_block_regs(int S, const float *cur, float
 // Returns the tile's candidate lanes (for the tally).
 __device__ __forceinline__ unsigned replay_tile_warp(int S, int t0, const int *sblk, int nblk, const ScanSmem &v,
                                                      const uint32_t *ids_v0, uint32_t *pid, float *pd, int &sz, int topk,
-                                                     float &dk, unsigned long long &c_rr) {
+                                                     float &dk, bool counted, unsigned long long &c_rr) {
     const int lane = threadIdx.x & 31;
     uint32_t cm = 0;
     float smax = 0.0f;
@@ -1778,20 +1765,35 @@ __device__ __forceinline__ unsigned replay_tile_warp(int S, int t0, const int *s
     }
     uint32_t live = __ballot_sync(kFull, cm != 0 && !(S > 1 && smax > dk));
     if (!live) return __reduce_add_sync(kFull, __popc(cm));
-    auto in_regs = [&](auto &P) {
-        P.load(pid, pd, sz, topk, dk);
-        while (live) {
-            const int ww = __ffs(live) - 1, bb = sblk ? sblk[ww] : t0 + ww;
-            if (!replay_block_regs(S, v.cur + ww * 32, __shfl_sync(kFull, smax, ww), v.part + ww * S * 32,
-                                   __shfl_sync(kFull, cm, ww), ids_v0 + (int64_t)bb * 32, P, c_rr))
-                break;
-            live &= live - 1;
-        }
-        P.store(pid, pd);
-        sz = P.sz;
-        dk = P.dk;
+    const int bb = lane < nblk ? (sblk ? sblk[lane] : t0 + lane) : 0;
+    // blocks from the first of live on, lane by lane (m: the lanes of the first one left)
+    const auto one = [&](uint32_t m, float sx) {
+        const int ww = __ffs(live) - 1;
+        replay_block_warp(S, __shfl_sync(kFull, bb, ww), v.cur + ww * 32, sx, v.part + ww * S * 32, m, ids_v0, pid, pd, sz, topk,
+                          dk, c_rr);
+        live &= live - 1;
     };
-    if (S > kRegSegs) {
+    auto in_regs = [&](auto &P) {
+        while (live) {
+            P.load(pid, pd, sz, topk);
+            uint32_t m = 0u, left = 0u;
+            float sx = 0.0f;
+            for (; live; live &= live - 1) {
+                const int ww = __ffs(live) - 1;
+                m = __shfl_sync(kFull, cm, ww);
+                sx = __shfl_sync(kFull, smax, ww);
+                left = replay_block_regs(S, v.cur + ww * 32, sx, v.part + ww * S * 32, m,
+                                         ids_v0 + (int64_t)__shfl_sync(kFull, bb, ww) * 32, P, [](float) {});
+                if (left) break;
+            }
+            if (!P.odd) {
+                P.store(pid, pd, sz);
+                dk = P.dk;
+            }
+            if (left) one(left, left == m ? sx : -FLT_MAX);  // after an insert of the block its stage minima have passed
+        }
+    };
+    if (counted || S > kRegSegs) {
     } else if (topk <= 32) {
         RegPool<1> P;
         in_regs(P);
@@ -1799,16 +1801,13 @@ __device__ __forceinline__ unsigned replay_tile_warp(int S, int t0, const int *s
         RegPool<kRegPool / 32> P;
         in_regs(P);
     }
-    for (; live; live &= live - 1) {  // more segments, a longer pool, or a NaN met
-        const int ww = __ffs(live) - 1;
-        replay_block_warp(S, sblk ? sblk[ww] : t0 + ww, v.cur + ww * 32, __shfl_sync(kFull, smax, ww), v.part + ww * S * 32,
-                          __shfl_sync(kFull, cm, ww), ids_v0, pid, pd, sz, topk, dk, c_rr);
-    }
+    while (live) one(__shfl_sync(kFull, cm, __ffs(live) - 1), __shfl_sync(kFull, smax, __ffs(live) - 1));
     return __reduce_add_sync(kFull, __popc(cm));
 }
 
 struct ScanTally {
     unsigned long long blocks = 0, vecs = 0, rr = 0, spec = 0;
+    bool counted = false;  // counters are kept: every evaluated lane is counted
 };
 
 // Exact sequential scan of the np probes of one query, continuing the pool held
@@ -1937,7 +1936,7 @@ __device__ void scan_probes(const DevIndexView &ix, const uint32_t *__restrict__
                     float dk = distk;
                     int sz = pool_size;
                     const unsigned nc = replay_tile_warp(S, 0, sm.sblk, ng, sm, ix.ids + h.v0, sm.pool_id, sm.pool_d, sz,
-                                                         topk, dk, tl.rr);
+                                                         topk, dk, tl.counted, tl.rr);
                     if (tid == 0) {
                         tl.spec += nc;
                         distk = dk;
@@ -2102,7 +2101,7 @@ __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan_ws(DevIndex
                 const ScanSmem v = ws_view(sm, extra, S, b);
                 const WsTile mt = meta[b];
                 const unsigned nc = replay_tile_warp(S, mt.t0, nullptr, min(kWsSlots, nb - mt.t0), v, ix.ids + mt.v0,
-                                                     sm.pool_id, sm.pool_d, sz, topk, dk, rr);
+                                                     sm.pool_id, sm.pool_d, sz, topk, dk, counters != nullptr, rr);
                 if (tid == 0) {
                     spec += nc;
                     *vdistk = dk;
@@ -2464,6 +2463,7 @@ __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan_first(DevIn
         __shared__ int pool_size;
         __shared__ float distk;
         ScanTally tl;
+        tl.counted = counters != nullptr;
         init_pool(sm, topk, pool_size, distk);
         const uint32_t *pr = probe + (size_t)qi * np_max;
         const float *qrot = qrot_all + (size_t)qi * ix.Dtot, *prune = prune_all + (size_t)qi * S;
@@ -2495,7 +2495,7 @@ __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan_first(DevIn
                     float dk = distk;
                     int sz = pool_size;
                     const unsigned nc = replay_tile_warp(S, t0, nullptr, te - t0, sm, ix.ids + v0, sm.pool_id, sm.pool_d, sz, topk, dk,
-                                                         tl.rr);
+                                                         tl.counted, tl.rr);
                     if (tid == 0) {
                         tl.spec += nc;
                         distk = dk;
@@ -2819,10 +2819,14 @@ constexpr int kReplayPer = 4;    // scan positions per thread in a window
 // every warp evaluates records under the current distk; the first record with
 // an accepted insert is replayed exactly by warp 0 (the records before it
 // change nothing and only add their counts), and evaluation resumes after it.
-// kRows > 0 (no counters kept, k at most 32 kRows, at most kRegSegs segments): warp 0 holds the pool in registers,
-// and a chunk is evaluated once: the records marked under the distk at its start are
-// replayed one after the other, without a barrier per record.
-template <int kRows>
+// kPer > 0 (no counters kept, k at most 32 kPer, at most kRegSegs segments): warp 0 holds
+// the pool in registers, and a chunk is evaluated once: the records marked under the distk at its
+// start are replayed one after the other, without a barrier per record.  A record left
+// unmarked can still matter to the reference where a running sum equals the distk of
+// its turn (the sum is inserted); all warps look for that among the distk values that the
+// chunk's inserts left, and a chunk with such a sum, or with more inserts than kSeen, is replayed again, every record.
+constexpr int kSeen = 64;
+template <int kPer>
 __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, SplitState st,
                                                               uint32_t *__restrict__ out_ids, float *__restrict__ out_d,
                                                               unsigned long long *__restrict__ counters, int xstride) {
@@ -2859,26 +2863,30 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
         const int RW = st.rec_words, R16 = RW / 4;
         unsigned long long rr = 0;
         __syncthreads();
-        RegPool<kRows ? kRows : 1> P;
-        if (kRows && w == 0) P.load(sm.pool_id, sm.pool_d, pool_size, topk, distk);
+        __shared__ float old_d[kPer ? 32 * kPer : 1];  // the pool before a chunk
+        __shared__ uint32_t old_id[kPer ? 32 * kPer : 1];
+        __shared__ float seen[kSeen];  // distk after each insert of the chunk
+        __shared__ int nseen;
         const int pos_end = min(np, s_phi);
-        for (int base = s_plo; base < pos_end; base += kScanThreads * kReplayPer) {
-            // thread t tests positions base + kReplayPer t .. + kReplayPer - 1; a
+        for (int base = s_plo, per; base < pos_end; base += kScanThreads * per) {
+            // the first window is short: its inserts lower the distk that filters the next
+            per = base == s_plo ? 1 : kReplayPer;
+            // thread t tests positions base + per t .. + per - 1; a
             // block-wide prefix of the counts keeps the list in position order
-            const int p0 = base + kReplayPer * tid;
+            const int p0 = base + per * tid;
             const float dk0 = distk;
             // with a full pool a lane is accepted only at a value <= distk: a record whose
             // every such value exceeds distk (summary z) changes nothing and is not staged.
             // With counters kept, the lanes the reference evaluates in such a record are
             // counted after each chunk under the distk at its position (count_dropped).
             const bool zf = pool_size == topk;
-            const int wend = min(pos_end, base + kScanThreads * kReplayPer);
+            const int wend = min(pos_end, base + kScanThreads * per);
             bool f[kReplayPer];
             int mine = 0;
     #pragma unroll
             for (int r = 0; r < kReplayPer; ++r) {
                 f[r] = false;
-                if (p0 + r < pos_end) {
+                if (r < per && p0 + r < pos_end) {
                     const float4 v = su[p0 + r];
                     f[r] = v.x < dk0 && !(v.y > dk0) && !(zf && v.z > dk0);
                 }
@@ -2950,40 +2958,95 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
                 __syncthreads();
                 const float *buf = stage_buf + (size_t)(k & 1) * kReplayRecs * RW;
                 const int c0 = k * kReplayRecs, cn = min(kReplayRecs, total - c0);
-                if (kRows) {
+                if (kPer) {
                     // every warp marks the records with an accepted insert under the distk at the
-                    // chunk's start (a superset of those that have one at their turn)
+                    // chunk's start (but for ties a superset of those that have one at their turn)
                     const float dk = distk;
                     const int sz = pool_size;
                     for (int r = w; r < cn; r += kScanWarps) {
                         int c;
-                        const float *rec = buf + (size_t)r * RW;
-                        const bool e = record_effect(S, rec, dk, sz, topk, c);
+                        const bool e = record_effect(S, buf + (size_t)r * RW, dk, sz, topk, c);
                         if (lane == 0) eff[r] = e;
                     }
+                    if (tid == 0) nseen = 0;
                     __syncthreads();
-                    if (w == 0) {
-                        uint32_t live = __ballot_sync(kFull, lane < cn && eff[lane]);
-                        for (; live; live &= live - 1) {
-                            const float *rec = buf + (size_t)(__ffs(live) - 1) * RW;
-                            const uint32_t *ri = reinterpret_cast<const uint32_t *>(rec);
-                            const uint32_t *rid = rec_ids(rec, S);
-                            if (!replay_block_regs(S, rec + 8 + (S + 1), __uint_as_float(ri[7]), rec + 8 + (S + 1) + 32,
-                                                   ri[1], rid, P, rr)) {  // a NaN: on the pool in shared memory
-                                P.store(sm.pool_id, sm.pool_d);
-                                float dkw = P.dk;
-                                int szw = P.sz;
-                                replay_block_warp(S, 0, rec + 8 + (S + 1), __uint_as_float(ri[7]), rec + 8 + (S + 1) + 32,
-                                                  ri[1], rid, sm.pool_id, sm.pool_d, szw, topk, dkw, rr);
-                                P.load(sm.pool_id, sm.pool_d, szw, topk, dkw);
+                    const uint32_t marked = __ballot_sync(kFull, lane < cn && eff[lane]);
+                    if (!marked) continue;  // uniform
+                    // the records `live` in order, from the pool in shared memory
+                    const auto replay_records = [&](uint32_t live) {
+                        RegPool<kPer ? kPer : 1> P;
+                        int szw = sz, n = 0;
+                        float dkw = dk;
+                        while (live) {
+                            P.load(sm.pool_id, sm.pool_d, szw, topk);
+                            uint32_t left = 0u, m = 0u;
+                            const float *rec = buf;
+                            for (; live; live &= live - 1) {
+                                rec = buf + (size_t)(__ffs(live) - 1) * RW;
+                                m = reinterpret_cast<const uint32_t *>(rec)[1];
+                                left = replay_block_regs(S, rec + 8 + (S + 1), rec[7], rec + 8 + (S + 1) + 32, m,
+                                                         rec_ids(rec, S), P, [&](float x) {
+                                                             if (lane == 0 && n < kSeen) seen[n] = x;
+                                                             ++n;
+                                                         });
+                                if (left) break;
+                            }
+                            if (!P.odd) {
+                                P.store(sm.pool_id, sm.pool_d, szw);
+                                dkw = P.dk;
+                            }
+                            if (left) {  // lane by lane
+                                n = kSeen + 1;
+                                replay_block_warp(S, 0, rec + 8 + (S + 1), left == m ? rec[7] : -FLT_MAX,
+                                                  rec + 8 + (S + 1) + 32, left, rec_ids(rec, S), sm.pool_id, sm.pool_d, szw, topk,
+                                                  dkw, rr);
+                                live &= live - 1;
                             }
                         }
                         if (lane == 0) {
-                            distk = P.dk;
-                            pool_size = P.sz;
+                            distk = dkw;
+                            pool_size = szw;
+                            nseen = n;
                         }
+                        __syncwarp();
+                    };
+                    const uint32_t all = cn == 32 ? kFull : (1u << cn) - 1u;
+                    if (w == 0) {
+                        for (int i = lane; i < sz; i += 32) {
+                            old_d[i] = sm.pool_d[i];
+                            old_id[i] = sm.pool_id[i];
+                        }
+                        replay_records(marked);
                     }
                     __syncthreads();
+                    if (S > 1 && marked != all) {
+                        const int n = nseen;
+                        bool tie = n > kSeen;
+                        if (!tie)
+                            for (int r = w; r < cn; r += kScanWarps) {
+                                if ((marked >> r) & 1u) continue;
+                                const float *rec = buf + (size_t)r * RW;
+                                const bool in = (reinterpret_cast<const uint32_t *>(rec)[1] >> lane) & 1u;
+                                const float *cur = rec + 8 + (S + 1), *part = cur + 32;
+                                float acc = in ? cur[lane] : FLT_MAX;
+                                if (in && acc < dk)
+                                    for (int s = 0; s < S; ++s) {
+                                        acc = __fadd_rn(acc, part[s * 32 + lane]);
+                                        for (int e = 0; e < n; ++e) tie |= acc == seen[e];
+                                    }
+                            }
+                        if (__syncthreads_or(tie)) {
+                            if (w == 0) {
+                                for (int i = lane; i < sz; i += 32) {
+                                    sm.pool_d[i] = old_d[i];
+                                    sm.pool_id[i] = old_id[i];
+                                }
+                                __syncwarp();
+                                replay_records(all);
+                            }
+                            __syncthreads();
+                        }
+                    }
                     continue;
                 }
                 if (tid == 0) {  // read by warp 0 (thread 0 first) and, after the chunk, by count_dropped
@@ -3036,7 +3099,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
                 }
             }
         }
-        if (kRows && w == 0) P.store(sm.pool_id, sm.pool_d);
         __syncthreads();
         if (tid == 0 && counters) atomicAdd(counters + 2, rr);
         if (st.final_level) {
@@ -3073,6 +3135,7 @@ __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan(DevIndexVie
     __shared__ int pool_size;
     __shared__ float distk;
     ScanTally tl;
+    tl.counted = counters != nullptr;
     init_pool(sm, topk, pool_size, distk);
     scan_probes(ix, probe + (size_t)qi * qsh.np_max, np, qrot_all + (size_t)qi * ix.Dtot,
                 prune_all + (size_t)qi * ix.S, topk, sm, pool_size, distk, tl,
