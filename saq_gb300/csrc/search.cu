@@ -3490,7 +3490,9 @@ size_t split_scratch_bytes(const Index &I, int64_t cap, int64_t topk, int64_t np
 // (`want`), bounded by scratch memory.
 int64_t split_positions(const Index &I, int64_t want) {
     const size_t per = 4 * (size_t)rec_words_of(I.view.S) + 16;
-    size_t budget = (size_t)8 << 30;
+    // 12 GB: with 8 GB a batch of 4,096 queries with nprobe up to 256 over 10M vectors leaves
+    // some of its heaviest queries to the CTA scan (43.9 ms a batch, 39.7 from 10 GB on)
+    size_t budget = (size_t)12 << 30;
     if (const char *e = std::getenv("SAQG_SPLIT_RECORD_BYTES"))  // tests: a small budget forces the overflow path
         budget = std::max<size_t>(per, (size_t)std::atoll(e));
     const int64_t by_mem = (int64_t)(budget / per);
