@@ -4064,6 +4064,12 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
             int nlev = 1;
             if (mode == 0)
                 while (nlev < kMaxSpecLevels && levels[nlev] >= 0) ++nlev;
+            // a last level that holds less than half of the tiles (of the largest query: a tile
+            // per kTileBlocks blocks, and one per probe that they do not fill) costs its three
+            // launches for little: the one before it takes them (400 queries of 70 probes over
+            // 146,720 vectors: 710 us, 692 without that level)
+            const int64_t max_tiles = max_pos / kTileBlocks + nprobe;
+            while (nlev > 1 && 2 * (int64_t)levels[nlev - 1] > max_tiles) --nlev;
             for (int L = 0; L < nlev; ++L) {
                 SplitState sl = ss;
                 sl.t_lo = mode == 0 ? levels[L] : 0;
