@@ -3427,7 +3427,7 @@ struct Bump {
 // kPrepCap holds (nprobe pairs each), at most nq; 0 below kPrepMinQueries
 // queries, where the scan CTAs build each cluster's state in the shorter latency
 // (256 threads per LUT).  12 GB holds every query of a 4,096-query batch at
-// nprobe 256 with D = 1024 (8.8 GB; one segment: the CTA scan's copy is as large
+// nprobe 256 with D = 1024 (8.8 GB; the CTA scan's copy is as large
 // again), a few percent of the device beside the index.
 constexpr size_t kPrepCap = (size_t)12 << 30;
 constexpr int64_t kPrepMinQueries = 64;
@@ -3459,7 +3459,7 @@ size_t search_scratch_bytes(const Index &I, int64_t nq, int64_t topk, int64_t np
     add(64);                                   // flags
     add(64);                                   // counters
     add(prep_bytes(I, nq, nprobe));            // prepared LUTs of the split list
-    if (prep_slots(I, nq, nprobe) == nq && I.view.S == 1) add(prep_bytes(I, nq, nprobe));  // ... and of the CTA scan's
+    if (prep_slots(I, nq, nprobe) == nq) add(prep_bytes(I, nq, nprobe));  // ... and of the CTA scan's
     (void)host_io;
     return b + 256;
 }
@@ -3851,7 +3851,7 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
     const int64_t pslots = prep_slots(I, nq, nprobe);
     uint16_t *prep_lut = pslots ? bp.take<uint16_t>((size_t)pslots * nprobe * 4 * ix.Dtot) : nullptr;
     SegScal *prep_scal = pslots ? bp.take<SegScal>((size_t)pslots * nprobe * ix.S) : nullptr;
-    const bool scan_prep_fits = pslots > 0 && pslots == nq && ix.S == 1;
+    const bool scan_prep_fits = pslots > 0 && pslots == nq;
     uint16_t *scan_lut = scan_prep_fits ? bp.take<uint16_t>((size_t)nq * nprobe * 4 * ix.Dtot) : nullptr;
     SegScal *scan_scal = scan_prep_fits ? bp.take<SegScal>((size_t)nq * nprobe * ix.S) : nullptr;
     cudaEvent_t ev[7] = {};
@@ -3921,10 +3921,12 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
         unsigned long long *cnt = stats ? counters : nullptr;
         const int mode0 = scan_mode(nq, topk, tune);
         const int mode = (qsh.np || qsh.k) && mode0 == 2 ? 0 : mode0;
-        // One segment: the CTA scan's queries get batched LUTs too (by query; on the
-        // caller's stream, after the split pass has forked, so it overlaps the split
-        // pass's start) when the budget holds every query's.  Several segments: the
-        // scan needs the LUT of one probe in four (10M / 4,096 queries) and builds those.
+        // The CTA scan's queries get batched LUTs too (by query; on the caller's stream,
+        // after the split pass has forked, so it overlaps the split pass's start) when
+        // the budget holds every query's.  A CTA that builds the LUTs of the probes that
+        // stage 0 leaves does less work where that is one in four (10M / 16,384 Zipf clusters,
+        // 4,096 queries: 1.93 ms against 1.98) but loses where most are left: 647,483
+        // vectors in 6,497 clusters, 1,088 queries, 3.21 ms against 2.85, 600 on an anisotropic set 2.46 against 2.12.
         const std::function<Prepared(const uint8_t *)> scan_prep = [&](const uint8_t *skip) {  // skip: queries left out
             Prepared pp;
             if (!scan_lut || scan_ws(tune)) return pp;
