@@ -43,7 +43,10 @@ constexpr int kScanThreads = kScanWarps * 32;
 constexpr int kBlocksPerWarp = 2;
 constexpr int kTileB = kScanWarps * kBlocksPerWarp;  // blocks per tile
 constexpr int kMaxTopK = 4096;
-constexpr int kItemCands = 16;  // candidates of a tile up to which half-warps take the accurate distances
+// Candidates of a tile up to which half-warps take the accurate distances: the other
+// form's time is the chain over the widest segment, so the line lies lower where that is short.
+constexpr int kItemCands = 16, kItemCandsNarrow = 8;
+constexpr int kNarrowDim = 512;
 constexpr int kScanMinCtas = 4;  // resident scan CTAs per SM the register budget is sized for
 
 struct SegScal {
@@ -1389,7 +1392,9 @@ __device__ __forceinline__ void tile_candidates(const DevIndexView &ix, ScanSmem
     // half the instructions.  The line lies where the two
     // cross: 256 queries of 1,536 dimensions (about 13 candidates a tile) take 1.67 ms
     // with half-warps up to 16 candidates and 2.51 without, 37 queries with k = 100
-    // (about 75) 4.04 ms without and 4.65 with half-warps up to 96.
+    // (about 75) 4.04 ms without and 4.65 with half-warps up to 96.  Segments of 64, 192 and
+    // 320 dimensions, 1,500 queries: 5.23 ms with the line at 8, 5.58 at 16 (one segment of
+    // 768: 4.81 and 4.71; 1,536: 1.33 and 1.19).
     // The FP64 step of the distance (accurate_dist) would cost a warp's issue for two
     // lanes, so lane 2i, 2i + 1 keep the products of the warp's i-th item and up to 32
     // of them take that step together.
@@ -1428,7 +1433,9 @@ __device__ __forceinline__ void tile_candidates(const DevIndexView &ix, ScanSmem
         held = 0;
         __syncwarp();
     };
-    if (ncand > kItemCands) {
+    int widest = 0;
+    for (int s = 0; s < S; ++s) widest = max(widest, ix.seg[s].dim);
+    if (ncand > (widest < kNarrowDim ? kItemCandsNarrow : kItemCands)) {
         const int P = (ncand + 31) >> 5;  // warps' worth of tasks per segment
         for (int t = w; t < S * P; t += nwarps) {
             const int si = t / P, r0 = (t - si * P) * 32, s = S - 1 - si;
