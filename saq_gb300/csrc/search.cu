@@ -2438,6 +2438,7 @@ struct SplitState {
     // each, so k_scan_first fills the list itself and k_defer does not run
     int64_t stride;
     int tile_blocks;     // blocks of a speculative tile (kFewTileBlocks or kTileBlocks)
+    int replay_recs;     // records of a staged chunk of the replay (at most kReplayRecs)
 };
 
 // Scan-order position of the first block of tile t after a query's split
@@ -2458,7 +2459,7 @@ __device__ __forceinline__ int tile_pos(const SplitState &st, int slot, int t) {
 
 // Words of a record: 8 of header, S + 1 stage minima, the 32 estimates, 32 partials per
 // segment, the 32 ids (so that the replay reads nothing but staged records).
-__host__ __device__ inline int rec_words_of(int S) { return (8 + (S + 1) + 32 + 32 * S + 32 + 3) & ~3; }
+__host__ __device__ constexpr int rec_words_of(int S) { return (8 + (S + 1) + 32 + 32 * S + 32 + 3) & ~3; }
 __device__ __forceinline__ const uint32_t *rec_ids(const float *rec, int S) {
     return reinterpret_cast<const uint32_t *>(rec) + 8 + (S + 1) + 32 + 32 * S;
 }
@@ -2833,14 +2834,19 @@ __device__ __forceinline__ bool record_effect(int S, const float *rec, float dk,
     return __any_sync(kFull, pass && !(sz == topk && acc > dk));
 }
 
-constexpr int kReplayRecs = 32;  // records per staged chunk (double-buffered)
+// Records per staged chunk (double-buffered): 32 where they fit beside the scan's own
+// shared memory, fewer for plans of many segments or a large k (16 segments of 64
+// dimensions leave room for 29, and for 22 with k = 4,096), at the least 4.
+constexpr int kReplayRecs = 32;
+constexpr size_t kScanSmem = 200 * 1024, kReplaySmem = 220 * 1024;  // most shared memory of a scan, of a replay
+static_assert(kScanSmem + 2 * 4 * 4 * rec_words_of(kMaxSeg) <= kReplaySmem, "four records always fit");
 constexpr int kReplayPer = 4;    // scan positions per thread in a window
 
 // Per query on the list: walk its scan positions in order, kScanThreads at a
 // time.  A record can matter only if a candidate estimate lies below distk and
 // no stage minimum above it; distk only shrinks, so positions whose summary
 // fails the distk at the window's start are dropped at once.  The rest are
-// staged into shared memory by asynchronous copies, kReplayRecs at a time
+// staged into shared memory by asynchronous copies, replay_recs at a time
 // (the next chunk in flight while the current one is evaluated).  In a chunk,
 // every warp evaluates records under the current distk; the first record with
 // an accepted insert is replayed exactly by warp 0 (the records before it
@@ -2886,7 +2892,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
         const int np = st.npos[slot];
         const float4 *su = st.summ + st.pos_off[slot];
         const float *rq = st.rec + (size_t)st.pos_off[slot] * st.rec_words;
-        const int RW = st.rec_words, R16 = RW / 4;
+        const int RW = st.rec_words, R16 = RW / 4, RC = st.replay_recs;
         unsigned long long rr = 0;
         __syncthreads();
         __shared__ float old_d[kPer ? 32 * kPer : 1];  // the pool before a chunk
@@ -2935,7 +2941,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
             for (int r = 0; r < kReplayPer; ++r)
                 if (f[r]) list[off++] = p0 + r;
             __syncthreads();
-            const int nch = (total + kReplayRecs - 1) / kReplayRecs;
+            const int nch = (total + RC - 1) / RC;
             // lanes with candidate estimate below the distk at their position in the
             // records of [lo, hi) that the accept bound dropped (distk: c_dk0, then after
             // each of the n_eff records replayed in this range, in position order)
@@ -2965,8 +2971,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
                 __syncthreads();
             }
             auto issue = [&](int k) {
-                const int c0 = k * kReplayRecs, cn = min(kReplayRecs, total - c0);
-                float *buf = stage_buf + (size_t)(k & 1) * kReplayRecs * RW;
+                const int c0 = k * RC, cn = min(RC, total - c0);
+                float *buf = stage_buf + (size_t)(k & 1) * RC * RW;
                 for (int i = tid; i < cn * R16; i += kScanThreads) {
                     const int r = i / R16, e = i - r * R16;
                     cp_async16(buf + (size_t)r * RW + 4 * e, rq + (size_t)list[c0 + r] * RW + 4 * e);
@@ -2982,8 +2988,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
                     cp_async_wait<0>();
                 }
                 __syncthreads();
-                const float *buf = stage_buf + (size_t)(k & 1) * kReplayRecs * RW;
-                const int c0 = k * kReplayRecs, cn = min(kReplayRecs, total - c0);
+                const float *buf = stage_buf + (size_t)(k & 1) * RC * RW;
+                const int c0 = k * RC, cn = min(RC, total - c0);
                 if (kPer) {
                     // every warp marks the records with an accepted insert under the distk at the
                     // chunk's start (but for ties a superset of those that have one at their turn)
@@ -3596,7 +3602,7 @@ void launch_cta_scan(bool ws, const DevIndexView &ix, const uint32_t *probe, con
         return;
     }
     const size_t smem = scan_smem_bytes(ix.Dtot, ix.S, qsh.k_max, xs);
-    SAQG_REQUIRE(smem <= 200 * 1024, "dimension / topk too large for the scan kernel's shared memory");
+    SAQG_REQUIRE(smem <= kScanSmem, "dimension / topk too large for the scan kernel's shared memory");
     ensure_smem((const void *)k_scan, smem);
     const Prepared prep = prep_of(deferred);
     k_scan<<<(unsigned)nq, kScanThreads, smem, st>>>(ix, probe, qsh, qrot, prune, ids, d, cnt, xs, deferred, order,
@@ -3922,7 +3928,7 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
         if (stats) SAQG_CUDA_TRY(cudaEventRecord(ev[2], st));
         const int xs = xstride_of(ix);
         const size_t smem = scan_smem_bytes(ix.Dtot, ix.S, (int)topk, xs);
-        SAQG_REQUIRE(smem <= 200 * 1024, "dimension / topk too large for the scan kernel's shared memory");
+        SAQG_REQUIRE(smem <= kScanSmem, "dimension / topk too large for the scan kernel's shared memory");
         uint32_t *ids_out = host ? oid : ids;
         float *d_out = host ? od : dists;
         unsigned long long *cnt = stats ? counters : nullptr;
@@ -4036,8 +4042,9 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
                                 order, qblocks, scan_prep, st);
             }
             const size_t smem1 = scan_smem_bytes(ix.Dtot, ix.S, 1, xs);
-            const size_t smem_r = smem + 2 * 4 * (size_t)kReplayRecs * ss.rec_words;
-            SAQG_REQUIRE(smem_r <= 220 * 1024, "dimension / topk too large for the replay kernel's shared memory");
+            const size_t rec_smem = 2 * 4 * (size_t)ss.rec_words;
+            ss.replay_recs = (int)std::min<size_t>(kReplayRecs, (kReplaySmem - smem) / rec_smem);
+            const size_t smem_r = smem + ss.replay_recs * rec_smem;
             ensure_smem((const void *)k_scan_first, (size_t)smem);
             ensure_smem((const void *)k_scan_spec, (size_t)smem1);
             // counters need every record's count, and a longer pool shared memory
@@ -4314,7 +4321,7 @@ void run_search_static(const Index &I, const float *q, int64_t nq, int64_t topk,
     if (dists) require_device_ptr(dists, "dists");
     const DevIndexView &ix = I.view;
     const size_t smem = scan_smem_bytes(ix.Dtot, ix.S, (int)topk, xstride_of(ix));
-    SAQG_REQUIRE(smem <= 200 * 1024, "dimension / topk too large for the scan kernel's shared memory");
+    SAQG_REQUIRE(smem <= kScanSmem, "dimension / topk too large for the scan kernel's shared memory");
     int prev = 0;
     SAQG_CUDA_TRY(cudaGetDevice(&prev));
     struct DevGuard {
@@ -4348,7 +4355,7 @@ void run_search_static(const Index &I, const float *q, int64_t nq, int64_t topk,
     check_launch("k_probe_select");
     launch_qprep(ix, q, nq, m, qrot, prune, st);
     const size_t smem_k = scan_smem_bytes(ix.Dtot, ix.S, (int)topk, xstride_of(ix));
-    SAQG_REQUIRE(smem_k <= 200 * 1024, "dimension / topk too large for the scan kernel's shared memory");
+    SAQG_REQUIRE(smem_k <= kScanSmem, "dimension / topk too large for the scan kernel's shared memory");
     ensure_smem((const void *)k_scan, (size_t)smem_k);
     QueryShape qsh;
     qsh.np_max = (int)nprobe;
@@ -4668,7 +4675,7 @@ void tc_rerank(const Index &I, const uint32_t *probe, int64_t nq, int64_t nprobe
     int L2 = 1;
     while (L2 < L) L2 <<= 1;
     const size_t smem = 4 * (size_t)(kRerankThreads / 32) * ix.Dtot;
-    SAQG_REQUIRE(scan_smem_bytes(ix.Dtot, ix.S, 1, 0) <= 200 * 1024,
+    SAQG_REQUIRE(scan_smem_bytes(ix.Dtot, ix.S, 1, 0) <= kScanSmem,
                  "dimension too large for the re-rank kernel's shared memory");
     ensure_smem((const void *)k_tc_rerank, smem);
     k_tc_rerank<<<(unsigned)nq, kRerankThreads, smem, st>>>(ix, probe, (int)nprobe, qrot, prune, lp, sl_pos, sl_cnt, L,
