@@ -2838,7 +2838,10 @@ __device__ __forceinline__ bool record_effect(int S, const float *rec, float dk,
 // shared memory, fewer for plans of many segments or a large k (16 segments of 64
 // dimensions leave room for 29, and for 22 with k = 4,096), at the least 4.
 constexpr int kReplayRecs = 32;
-constexpr size_t kScanSmem = 200 * 1024, kReplaySmem = 220 * 1024;  // most shared memory of a scan, of a replay
+// Most shared memory of a scan (200 KB beside the tiles' block numbers, which a tile
+// buffer has 64 bytes of), of the warp-specialised form's two buffers, and of a replay.
+constexpr size_t kScanSmem = 200 * 1024 + sizeof(int) * kTileB;
+constexpr size_t kScanWsSmem = 220 * 1024 + 2 * sizeof(int) * kTileB, kReplaySmem = 220 * 1024;
 static_assert(kScanSmem + 2 * 4 * 4 * rec_words_of(kMaxSeg) <= kReplaySmem, "four records always fit");
 constexpr int kReplayPer = 4;    // scan positions per thread in a window
 
@@ -3594,7 +3597,7 @@ void launch_cta_scan(bool ws, const DevIndexView &ix, const uint32_t *probe, con
     }
     if (ws) {
         const size_t smem = ws_smem_bytes(ix.Dtot, ix.S, qsh.k_max, xs);
-        SAQG_REQUIRE(smem <= 220 * 1024, "dimension / topk too large for the scan kernel's shared memory");
+        SAQG_REQUIRE(smem <= kScanWsSmem, "dimension / topk too large for the scan kernel's shared memory");
         ensure_smem((const void *)k_scan_ws, smem);
         k_scan_ws<<<(unsigned)nq, kScanThreads, smem, st>>>(ix, probe, qsh, qrot, prune, ids, d, cnt, xs, deferred,
                                                              order);
