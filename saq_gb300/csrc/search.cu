@@ -4499,7 +4499,10 @@ __device__ float searched_dist(const DevIndexView &ix, const float *x, const Seg
 // vector needs one entry of each codebook, so no LUT is built and nothing waits for a
 // barrier.  2,048 queries of 1,536 dimensions, 40 vectors each: 0.98 ms with a CTA and a
 // LUT per (query, cluster), 0.34 now; 4,096 queries over 10M x 1,024: 1.02 and 0.50.
+// Up to four warps, as many as their residuals (4 Dtot bytes each) fit beside the
+// kernel's own 6 KB: four up to 14,080 dimensions, three above.
 constexpr int kRerankThreads = 128, kRerankRun = 8, kRerankMax = 1024;  // at most kTcMaxShort entries
+constexpr size_t kRerankSmem = 220 * 1024;
 __global__ void __launch_bounds__(kRerankThreads) k_tc_rerank(DevIndexView ix, const uint32_t *__restrict__ probe,
                                                               int nprobe, const float *__restrict__ qrot_all,
                                                               const float *__restrict__ prune,
@@ -4513,7 +4516,7 @@ __global__ void __launch_bounds__(kRerankThreads) k_tc_rerank(DevIndexView ix, c
     const int qi = blockIdx.x, n = sl_cnt[qi], tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int *pos = sl_pos + (size_t)qi * L, *lq = lp + (size_t)qi * (nprobe + 1);
     const float *qrot = qrot_all + (size_t)qi * ix.Dtot;
-    for (int e = tid; e < n; e += kRerankThreads) {  // the last probe that starts at or before it (empty probes share an offset)
+    for (int e = tid; e < n; e += (int)blockDim.x) {  // the last probe that starts at or before it (empty probes share an offset)
         int lo = 0, hi = nprobe - 1;
         const int x = pos[e];
         while (lo < hi) {
@@ -4677,12 +4680,13 @@ void tc_rerank(const Index &I, const uint32_t *probe, int64_t nq, int64_t nprobe
     const DevIndexView &ix = I.view;
     int L2 = 1;
     while (L2 < L) L2 <<= 1;
-    const size_t smem = 4 * (size_t)(kRerankThreads / 32) * ix.Dtot;
+    const size_t per_warp = 4 * (size_t)ix.Dtot;
     SAQG_REQUIRE(scan_smem_bytes(ix.Dtot, ix.S, 1, 0) <= kScanSmem,
                  "dimension too large for the re-rank kernel's shared memory");
-    ensure_smem((const void *)k_tc_rerank, smem);
-    k_tc_rerank<<<(unsigned)nq, kRerankThreads, smem, st>>>(ix, probe, (int)nprobe, qrot, prune, lp, sl_pos, sl_cnt, L,
-                                                          sl_dist);
+    const int warps = (int)std::min<size_t>(kRerankThreads / 32, kRerankSmem / per_warp);  // (3 at the check's limit)
+    ensure_smem((const void *)k_tc_rerank, warps * per_warp);
+    k_tc_rerank<<<(unsigned)nq, 32 * warps, warps * per_warp, st>>>(ix, probe, (int)nprobe, qrot, prune, lp, sl_pos,
+                                                                   sl_cnt, L, sl_dist);
     check_launch("k_tc_rerank");
     k_tc_topk<<<(unsigned)nq, kScanThreads, 8 * (size_t)L2, st>>>(ix, probe, (int)nprobe, lp, sl_pos, sl_apx, sl_cnt,
                                                                   sl_dist, L, L2, (int)topk, qk, ids, dists, apx);
