@@ -1662,7 +1662,7 @@ struct RegPool {
             const int e = kPer * lane + r;
             d[r] = e < size ? pd[e] : FLT_MAX;
             u[r] = e < size ? pid[e] : 0u;
-            bad |= e < size && !(d[r] < FLT_MAX);
+            bad |= e < size && !(fabsf(d[r]) < FLT_MAX);
         }
         odd = __any_sync(kFull, bad);
         dk = kth();
@@ -1727,8 +1727,8 @@ __device__ __forceinline__ uint32_t replay_block_regs(int S, const float *cur, f
         top = s == 0 ? last : fmaxf(top, last);
     }
     const float gate = fmaxf(c, top);
-    // (a NaN stays one in the later sums)
-    if (__any_sync(kFull, in && !(gate < FLT_MAX && last < FLT_MAX))) return cm;
+    // (a NaN stays one in the later sums, and a -inf stays or becomes one)
+    if (__any_sync(kFull, in && !(gate < FLT_MAX && fabsf(last) < FLT_MAX))) return cm;
     if (S == 1) {
         uint32_t rest = __ballot_sync(kFull, in && c < P.dk);  // the mask, at the block's start
         while (rest) {
