@@ -602,13 +602,15 @@ __device__ __forceinline__ int block_prefix(int f, int *wtot, int *tot) {
 }
 
 // Few of many, the shortlist's case: a bound T on the L-th smallest key first, then
-// the keys up to T only.  Each thread takes the smallest key of its share, each warp
-// the ceil(L / 8)-th smallest of its lanes' minima, T is the largest of those over the
-// eight warps: at least L keys are <= T.  The keys up to T (about twice L) are
-// collected in any order, ranked against one another by (key, e), and the L first
-// emitted in ascending e by their rank in e.  (Four radix passes over all of them, most
-// keys in a few bins: 0.35 ms for 28M candidates of 4,096 queries; now 0.09.)  False, nothing emitted, when more than
-// kSelCollect keys are up to T (many equal keys).
+// the keys up to T only.  Each thread takes the two smallest keys of its share, each
+// warp the ceil(L / 8)-th smallest of its lanes' 64, T is the largest of those over the
+// eight warps: at least L keys are <= T; of 4,096 about 70 at L = 40, 360 at L = 256 (with
+// one minimum a thread T was the largest of all 256 there: 1,300 keys, more than are
+// collected).  They are collected in any order, ranked against one another by (key, e),
+// and the L first emitted in ascending e by their rank in e.  (Four radix passes over
+// all of them, most keys in a few bins: 0.35 ms for 28M candidates of 4,096 queries; now
+// 0.09.)  False, nothing emitted, when more than kSelCollect keys are up to T (many
+// equal keys).
 constexpr int kSelFew = 256, kSelCollect = 1024;
 template <class Key, class Emit>
 __device__ bool select_few(int M, int L, Key key, Emit emit) {
@@ -617,14 +619,20 @@ __device__ bool select_few(int M, int L, Key key, Emit emit) {
     __shared__ uint32_t chosen[kSelFew];
     __shared__ int ngot;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    uint32_t mine = 0xffffffffu;
-    for (int e = tid; e < M; e += 256) mine = min(mine, key(e));
+    uint32_t m1 = 0xffffffffu, m2 = 0xffffffffu;
+    for (int e = tid; e < M; e += 256) {
+        const uint32_t k = key(e);
+        m2 = min(m2, max(m1, k));
+        m1 = min(m1, k);
+    }
     uint32_t t = 0;
-    bool left = true;
     for (int i = (L + 7) / 8; i > 0; --i) {
-        t = __reduce_min_sync(kFullMask, left ? mine : 0xffffffffu);
-        const unsigned eq = __ballot_sync(kFullMask, left && mine == t);
-        if (eq && lane == __ffs(eq) - 1) left = false;
+        t = __reduce_min_sync(kFullMask, m1);
+        const unsigned eq = __ballot_sync(kFullMask, m1 == t);
+        if (lane == __ffs(eq) - 1) {
+            m1 = m2;
+            m2 = 0xffffffffu;
+        }
     }
     if (lane == 0) wkey[w] = t;
     if (tid == 0) ngot = 0;
