@@ -1866,13 +1866,20 @@ __device__ void scan_probes(const DevIndexView &ix, const uint32_t *__restrict__
             tl.vecs += __reduce_add_sync(kFull, (unsigned)h.n);
         }
         __syncthreads();
-        if (S > 1) {  // stage 0's scalars of every probe (Lut::prepare's q_l2sqr, in its order), a warp per probe
-            for (int i = w; i < m; i += kScanWarps)
-                if (hdr[i].nb)
+        if (S > 1) {  // stage 0's scalars of every probe: the batched preparation's, or (Lut::prepare's q_l2sqr, in
+                      // its order) a warp per probe
+            if (scal) {
+                for (int i = tid; i < m * S; i += kScanThreads)
+                    if (hdr[i / S].nb) vf[i] = scal[(size_t)p0 * S + i].vfac;
+            } else {
+                for (int i = w; i < m; i += kScanWarps) {
+                    if (!hdr[i].nb) continue;
                     for (int s = 0; s < S; ++s) {
                         const float v = stage0_scalar(ix, s, hdr[i].c, qrot, prune);
                         if (lane == 0) vf[i * S + s] = v;
                     }
+                }
+            }
             __syncthreads();
         }
         int loaded = -1;  // probe whose LUT is in place
