@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <functional>
 #include <memory>
@@ -162,23 +163,61 @@ void Index::upload(void *dst, const void *src, size_t bytes) {
     if (bytes) SAQG_CUDA_TRY(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
 }
 
-static void *grow(void *&buf, size_t &have, size_t bytes) {
-    if (bytes > have) {
-        // previous work on this buffer may still be in flight on any stream
-        SAQG_CUDA_TRY(cudaDeviceSynchronize());
-        if (buf) SAQG_CUDA_TRY(cudaFree(buf));
-        buf = nullptr;
-        have = 0;
-        const size_t want = bytes + bytes / 4 + (1 << 20);
-        cudaError_t e = cudaMalloc(&buf, want);
-        if (e != cudaSuccess) throw Error{SAQG_ERR_NOMEM, std::string("scratch cudaMalloc failed: ") + cudaGetErrorString(e)};
-        have = want;
-    }
-    return buf;
+// cudaMalloc.  SAQG_TEST_ALLOC_BYTES (tests): larger ones fail as on a full device.
+static cudaError_t scratch_malloc(void **p, size_t bytes) {
+    if (const char *e = std::getenv("SAQG_TEST_ALLOC_BYTES"))
+        if (bytes > (size_t)std::atoll(e)) return cudaErrorMemoryAllocation;
+    return cudaMalloc(p, bytes);
 }
 
-void *SearchCtx::scratch_get(size_t bytes) { return grow(scratch, scratch_bytes, bytes); }
-void *SearchCtx::split_scratch_get(size_t bytes) { return grow(split_scratch, split_scratch_bytes, bytes); }
+// The arena, grown to `bytes` (a quarter to spare where the device has it) when it is
+// smaller; null, and no arena, when the device's memory does not hold it.
+static void *grow(void *&buf, size_t &have, size_t bytes) {
+    if (bytes <= have) return buf;
+    // previous work on this buffer may still be in flight on any stream
+    SAQG_CUDA_TRY(cudaDeviceSynchronize());
+    if (buf) SAQG_CUDA_TRY(cudaFree(buf));
+    buf = nullptr;
+    have = 0;
+    for (const size_t want : {bytes + bytes / 4 + (1 << 20), bytes}) {
+        const cudaError_t e = scratch_malloc(&buf, want);
+        if (e == cudaSuccess) {
+            have = want;
+            return buf;
+        }
+        cudaGetLastError();
+        buf = nullptr;
+        if (e != cudaErrorMemoryAllocation)
+            throw Error{SAQG_ERR_NOMEM, std::string("scratch cudaMalloc failed: ") + cudaGetErrorString(e)};
+    }
+    return nullptr;
+}
+
+static void *or_nomem(void *p) {
+    if (!p)
+        throw Error{SAQG_ERR_NOMEM,
+                    std::string("scratch cudaMalloc failed: ") + cudaGetErrorString(cudaErrorMemoryAllocation)};
+    return p;
+}
+
+void *SearchCtx::scratch_get(size_t bytes) { return or_nomem(grow(scratch, scratch_bytes, bytes)); }
+void *SearchCtx::split_scratch_get(size_t bytes) { return or_nomem(grow(split_scratch, split_scratch_bytes, bytes)); }
+// As split_scratch_get, but null when memory is short.  What the device refused is asked
+// for again only once it has a sixteenth more free, so that calls after a refusal keep
+// the smaller arena they got.
+void *SearchCtx::split_scratch_try(size_t bytes) {
+    if (bytes <= split_scratch_bytes) return split_scratch;
+    size_t room = 0, total = 0;
+    SAQG_CUDA_TRY(cudaMemGetInfo(&room, &total));
+    room += split_scratch_bytes;
+    if (bytes >= refused_bytes && room < refused_room + refused_room / 16) return nullptr;
+    void *p = grow(split_scratch, split_scratch_bytes, bytes);
+    if (!p) {
+        refused_bytes = bytes;
+        refused_room = room;
+    }
+    return p;
+}
 
 // The split pass is a batch's critical path: its stream gets the device's
 // highest priority, so its CTAs go first while the CTA scan beside it fills in.

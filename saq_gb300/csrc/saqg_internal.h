@@ -87,6 +87,7 @@ struct SearchCtx {
     size_t scratch_bytes = 0;
     void *split_scratch = nullptr;
     size_t split_scratch_bytes = 0;
+    size_t refused_bytes = SIZE_MAX, refused_room = 0;  // least that the device refused, and what it had free then
     cudaStream_t aux = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // the query preparation's stream (lowest priority: it has slack beside the
@@ -104,6 +105,7 @@ struct SearchCtx {
     ~SearchCtx();
     void *scratch_get(size_t bytes);
     void *split_scratch_get(size_t bytes);
+    void *split_scratch_try(size_t bytes);
     cudaStream_t aux_stream();
     cudaEvent_t fork_event();
     cudaEvent_t join_event();

@@ -3522,6 +3522,24 @@ int64_t split_positions(const Index &I, int64_t want) {
     return std::max<int64_t>(1, std::min(want, by_mem));
 }
 
+// The split pass's scratch in the context, for as many record positions of `want` (out:
+// pos_cap) as the budget and the device have room for.  Queries that the records do not
+// reach stay with the CTA scan, so a device short of memory answers a call more slowly
+// instead of refusing it.  While `st` is captured, what the context holds is all there is.
+char *split_scratch_take(const Index &I, SearchCtx &C, int64_t cap, int64_t topk, int64_t nprobe, int64_t want,
+                         int64_t &pos_cap, cudaStream_t st) {
+    auto bytes = [&] { return split_scratch_bytes(I, cap, topk, nprobe, pos_cap); };
+    pos_cap = split_positions(I, want);
+    if (bytes() > C.split_scratch_bytes) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
+        const bool fixed = capture != cudaStreamCaptureStatusNone && C.split_scratch;
+        for (; pos_cap > 1; pos_cap /= 2)
+            if (fixed ? bytes() <= C.split_scratch_bytes : C.split_scratch_try(bytes()) != nullptr) break;
+    }
+    return static_cast<char *>(C.split_scratch_get(bytes()));
+}
+
 // Which exact scan serves a call: the split scan for latency-bound calls (few
 // queries), one CTA per query for batches, unless the tuned shape says
 // otherwise.  SAQG_SCAN_MODE=seq|split|warp forces one (tests).
@@ -3776,8 +3794,8 @@ void probe_shortlist(const Index &I, SearchCtx &C, const float *q, int64_t nq, i
 void presize_ctx(const Index &I, SearchCtx &C, int64_t nq, int64_t topk, int64_t nprobe) {
     std::lock_guard<std::mutex> lock(C.mu);
     C.scratch_get(search_scratch_bytes(I, nq, topk, nprobe, false));
-    const int64_t pos_cap = split_positions(I, nq * I.max_blocks_of_probes(nprobe));
-    C.split_scratch_get(split_scratch_bytes(I, nq, topk, nprobe, pos_cap));
+    int64_t pos_cap = 0;
+    split_scratch_take(I, C, nq, topk, nprobe, nq * I.max_blocks_of_probes(nprobe), pos_cap, nullptr);
     C.aux_stream();
     C.fork_event();
     C.join_event();
@@ -3987,8 +4005,8 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
             const int64_t max_pos = I.max_blocks_of_probes(nprobe);
             const int64_t cap = nq;
             const int64_t want = nq * max_pos;
-            const int64_t pos_cap = split_positions(I, want);
-            Bump sb{(char *)C.split_scratch_get(split_scratch_bytes(I, cap, topk, nprobe, pos_cap))};
+            int64_t pos_cap = 0;
+            Bump sb{split_scratch_take(I, C, cap, topk, nprobe, want, pos_cap, st)};
             SplitState ss;
             ss.nlist = sb.take<int>(16);
             ss.pos_used = reinterpret_cast<unsigned long long *>(ss.nlist + 2);
