@@ -87,6 +87,7 @@ struct SearchCtx {
     size_t scratch_bytes = 0;
     void *split_scratch = nullptr;
     size_t split_scratch_bytes = 0;
+    size_t split_limit = SIZE_MAX;  // most bytes of records' scratch a search may grow it to (serving: its budget)
     size_t refused_bytes = SIZE_MAX, refused_room = 0;  // least that the device refused, and what it had free then
     cudaStream_t aux = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -216,8 +217,10 @@ void run_search(const Index &idx, const float *q, int64_t nq, int64_t topk, int6
 // [1, np_max] / [1, k_max], into np_out / k_out (device, nq each).
 void clamp_shape(const int *np, const int *k, int64_t nq, int np_max, int k_max, int *np_out, int *k_out,
                  cudaStream_t st);
-// Scratch bytes a batch of this shape needs (both arenas), for admission by memory.
+// Scratch bytes a batch of this shape needs (both arenas), for admission by memory, and
+// those of the first arena alone.
 size_t search_bytes_estimate(const Index &idx, int64_t nq, int64_t topk, int64_t nprobe);
+size_t search_arena1_bytes(const Index &idx, int64_t nq, int64_t topk, int64_t nprobe);
 // Grows a context's arenas (and creates its stream, events and BLAS handle)
 // for batches up to this shape, so later searches allocate nothing.
 void presize_ctx(const Index &idx, SearchCtx &ctx, int64_t nq, int64_t topk, int64_t nprobe);

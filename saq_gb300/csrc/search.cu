@@ -3509,10 +3509,13 @@ size_t split_scratch_bytes(const Index &I, int64_t cap, int64_t topk, int64_t np
     return b + 256;
 }
 
+// A record and its summary.
+size_t record_bytes(const Index &I) { return 4 * (size_t)rec_words_of(I.view.S) + 16; }
+
 // Record positions of the split pass for a batch: every block of every query
 // (`want`), bounded by scratch memory.
 int64_t split_positions(const Index &I, int64_t want) {
-    const size_t per = 4 * (size_t)rec_words_of(I.view.S) + 16;
+    const size_t per = record_bytes(I);
     // 12 GB: with 8 GB a batch of 4,096 queries with nprobe up to 256 over 10M vectors leaves
     // some of its heaviest queries to the CTA scan (43.9 ms a batch, 39.7 from 10 GB on)
     size_t budget = (size_t)12 << 30;
@@ -3523,9 +3526,10 @@ int64_t split_positions(const Index &I, int64_t want) {
 }
 
 // The split pass's scratch in the context, for as many record positions of `want` (out:
-// pos_cap) as the budget and the device have room for.  Queries that the records do not
-// reach stay with the CTA scan, so a device short of memory answers a call more slowly
-// instead of refusing it.  While `st` is captured, what the context holds is all there is.
+// pos_cap) as the budget, the context's limit and the device have room for.  Queries that
+// the records do not reach stay with the CTA scan, so a device short of memory answers a
+// call more slowly instead of refusing it.  While `st` is captured, what the context holds
+// is all there is.
 char *split_scratch_take(const Index &I, SearchCtx &C, int64_t cap, int64_t topk, int64_t nprobe, int64_t want,
                          int64_t &pos_cap, cudaStream_t st) {
     auto bytes = [&] { return split_scratch_bytes(I, cap, topk, nprobe, pos_cap); };
@@ -3534,11 +3538,18 @@ char *split_scratch_take(const Index &I, SearchCtx &C, int64_t cap, int64_t topk
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
         const bool fixed = capture != cudaStreamCaptureStatusNone && C.split_scratch;
+        const size_t limit = fixed ? C.split_scratch_bytes : std::max(C.split_limit, C.split_scratch_bytes);
+        if (bytes() > limit) {  // as many as fit below it
+            const size_t over = bytes() - limit;
+            pos_cap = std::max<int64_t>(1, pos_cap - (int64_t)(over / record_bytes(I)) - 1);
+        }
         for (; pos_cap > 1; pos_cap /= 2)
-            if (fixed ? bytes() <= C.split_scratch_bytes : C.split_scratch_try(bytes()) != nullptr) break;
+            if (C.split_scratch_try(bytes())) break;
     }
     return static_cast<char *>(C.split_scratch_get(bytes()));
 }
+
+constexpr int64_t kFewQueries = 16;  // calls of up to so many take the split scan
 
 // Which exact scan serves a call: the split scan for latency-bound calls (few
 // queries), one CTA per query for batches, unless the tuned shape says
@@ -3553,7 +3564,7 @@ int scan_mode(int64_t nq, int64_t topk, const ScanTune &t) {
     if (t.mode == 0 || t.mode == 1) return t.mode;
     if (t.mode == 3) return 0;
     if (t.mode == 2) return topk <= 256 ? 2 : 0;
-    if (nq <= 16) return 1;
+    if (nq <= kFewQueries) return 1;
     return 0;
 }
 
@@ -3806,10 +3817,18 @@ void presize_ctx(const Index &I, SearchCtx &C, int64_t nq, int64_t topk, int64_t
 
 
 
+// Records for two thirds of the blocks, and 8 GB at most, are enough to admit a batch (the
+// heaviest queries come first, the CTA scan takes those that are left without); a few
+// queries, which the split pass answers alone, need them all.  The call itself takes up
+// to all of them where its budget has them (split_limit).
 size_t search_bytes_estimate(const Index &I, int64_t nq, int64_t topk, int64_t nprobe) {
-    const int64_t max_pos = I.max_blocks_of_probes(nprobe);
-    const int64_t pos_cap = split_positions(I, nq * max_pos);
-    return search_scratch_bytes(I, nq, topk, nprobe, false) + split_scratch_bytes(I, nq, topk, nprobe, pos_cap);
+    const int64_t all = split_positions(I, nq * I.max_blocks_of_probes(nprobe));
+    const int64_t of_8gb = (int64_t)(((size_t)8 << 30) / record_bytes(I));
+    const int64_t least = nq <= kFewQueries ? all : std::max<int64_t>(1, std::min(2 * all / 3, of_8gb));
+    return search_scratch_bytes(I, nq, topk, nprobe, false) + split_scratch_bytes(I, nq, topk, nprobe, least);
+}
+size_t search_arena1_bytes(const Index &I, int64_t nq, int64_t topk, int64_t nprobe) {
+    return search_scratch_bytes(I, nq, topk, nprobe, false);
 }
 
 void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_t nprobe, float m, uint32_t *ids,

@@ -8,8 +8,9 @@
 // query upload, the batched search (saqg_search_batch's path on the slot's own
 // search context) and the result download.  So a batch is admitted while the
 // previous ones still run, and their work overlaps on the device.  Admission is
-// by memory too: a batch is cut until its scratch (computed from its shape)
-// fits the budget left by the other in-flight slots.  A completer thread waits
+// by memory too: a batch is cut until its scratch (computed from its shape, with
+// records for two thirds of its blocks) fits the budget left by the other in-flight
+// slots, and its records take the rest of it.  A completer thread waits
 // for each batch's event and hands the rows back to their tickets.  Each
 // query's answer is the one the reference returns for it alone.
 #include <algorithm>
@@ -81,6 +82,12 @@ struct Server {
 
     Server(const Index &idx, const saqg_server_config &c) : I(idx), cfg(c) {}
 
+    // Bytes that a batch's second arena may take: what the budget has left beside the
+    // memory `held` by others and its first arena, and no less than it was admitted with.
+    size_t split_share(size_t budget, size_t held, int64_t n, int64_t k, int64_t np) const {
+        const size_t first = search_arena1_bytes(I, n, k, np), least = search_bytes_estimate(I, n, k, np) - first;
+        return std::max(least, budget - std::min(budget, held + first));
+    }
     void run_dispatcher();
     void run_completer();
     void launch(Slot &s);
@@ -147,6 +154,7 @@ void Server::run_dispatcher() {
             n = (n + 1) / 2;
             ++shrinks;
         }
+        s->ctx.split_limit = split_share((size_t)cfg.mem_budget_bytes, held, n, kmax, npmax);
         s->reqs.assign(pending.begin(), pending.begin() + n);
         pending.erase(pending.begin(), pending.begin() + n);
         s->busy = true;
@@ -256,10 +264,13 @@ Server *server_create(const Index &I, const saqg_server_config *c) {
         while (n > 1 && search_bytes_estimate(I, n, cfg.max_topk, cfg.max_nprobe) * cfg.max_inflight >
                             (size_t)cfg.mem_budget_bytes)
             n = (n + 1) / 2;
-        if (cfg.form == SAQG_FORM_TC)  // the candidate arena grows with the batches it meets
+        if (cfg.form == SAQG_FORM_TC) {  // the candidate arena grows with the batches it meets
             presize_tc_ctx(I, s->ctx, n, cfg.max_topk, cfg.max_nprobe, cfg.shortlist, 0);
-        else
+        } else {
+            s->ctx.split_limit = sv->split_share((size_t)cfg.mem_budget_bytes / cfg.max_inflight, 0, n, cfg.max_topk,
+                                                 cfg.max_nprobe);
             presize_ctx(I, s->ctx, n, cfg.max_topk, cfg.max_nprobe);
+        }
         sv->slots.push_back(std::move(s));
     }
     if (prev != I.device) cudaSetDevice(prev);

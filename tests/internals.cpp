@@ -1,0 +1,36 @@
+// What the library's host code decides, printed for tests/test_internals.py (built
+// there against libsaqg.so).  No GPU needed: `estimate`.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+
+#include "saqg_internal.h"
+
+using namespace saqg;
+
+// Bytes that admission counts for a batch over clusters of `blocks` blocks each.
+static void estimate(int S, int64_t blocks, int64_t nq, int64_t k, int64_t np) {
+    Index I;
+    I.D = 64 * S;
+    I.K = 512;
+    for (int s = 0; s < S; ++s) {
+        Index::SegHost h{};
+        h.dim = 64;
+        h.bits = 4;
+        I.segs.push_back(h);
+        I.view.seg[s].dim = 64;
+        I.view.seg[s].bits = 4;
+    }
+    for (int64_t c = 0; c <= I.K; ++c) I.blk_off.push_back(c * blocks);
+    finalize_view(I);
+    std::printf("%zu\n", search_bytes_estimate(I, nq, k, np));
+}
+
+int main(int argc, char **argv) {
+    const char *what = argc > 1 ? argv[1] : "";
+    if (!std::strcmp(what, "estimate") && argc == 7) {
+        estimate(std::atoi(argv[2]), std::atoll(argv[3]), std::atoll(argv[4]), std::atoll(argv[5]), std::atoll(argv[6]));
+        return 0;
+    }
+    return 2;
+}
