@@ -82,18 +82,22 @@ float time_call(F call, cudaStream_t st, Events &ev) {
 
 }  // namespace
 
-TuneReport autotune_exact(const Index &I, const float *q, int64_t nq, int64_t topk, int64_t nprobe, float m,
-                          cudaStream_t st) {
-    SAQG_REQUIRE(nq >= 1, "autotune needs at least one query");
+std::vector<ScanTune> exact_candidates(int64_t topk) {
     std::vector<ScanTune> cands;
-    ScanTune dflt;  // built-in
-    cands.push_back(dflt);
+    cands.push_back(ScanTune{});  // built-in
     for (int defer : {256, 512, 1024, 2048, 4096})
         for (int first : {16, 64}) cands.push_back(ScanTune{0, defer, first, -1});
-    for (int lv = 1; lv < 5; ++lv) cands.push_back(ScanTune{0, 1024, 16, lv});  // the speculation level sets
+    for (int lv = 1; lv < 5; ++lv) cands.push_back(ScanTune{0, -1, 16, lv});  // the speculation level sets, built-in line
     for (int defer : {-1, 4096}) cands.push_back(ScanTune{3, defer, -1, -1});  // warp-specialised CTA scan
     cands.push_back(ScanTune{1, -1, -1, -1});
     if (topk <= 256) cands.push_back(ScanTune{2, -1, -1, -1});
+    return cands;
+}
+
+TuneReport autotune_exact(const Index &I, const float *q, int64_t nq, int64_t topk, int64_t nprobe, float m,
+                          cudaStream_t st) {
+    SAQG_REQUIRE(nq >= 1, "autotune needs at least one query");
+    const std::vector<ScanTune> cands = exact_candidates(topk);
     DevOut ref((size_t)nq * topk), out((size_t)nq * topk);
     Events ev;
     TuneReport rep;

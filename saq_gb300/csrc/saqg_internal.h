@@ -269,6 +269,7 @@ struct TuneReport {
     int candidates = 0;
     float default_ms = 0, tuned_ms = 0;
 };
+std::vector<ScanTune> exact_candidates(int64_t topk);  // the first: the built-in shapes
 TuneReport autotune_exact(const Index &idx, const float *q_dev, int64_t nq, int64_t topk, int64_t nprobe, float m,
                           cudaStream_t st);
 TuneReport autotune_tc(const Index &idx, const float *q_dev, int64_t nq, int64_t topk, int64_t nprobe,

@@ -1,5 +1,5 @@
 // What the library's host code decides, printed for tests/test_internals.py (built
-// there against libsaqg.so).  No GPU needed: `estimate`.
+// there against libsaqg.so).  No GPU needed: `estimate`, `candidates`.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -30,6 +30,11 @@ int main(int argc, char **argv) {
     const char *what = argc > 1 ? argv[1] : "";
     if (!std::strcmp(what, "estimate") && argc == 7) {
         estimate(std::atoi(argv[2]), std::atoll(argv[3]), std::atoll(argv[4]), std::atoll(argv[5]), std::atoll(argv[6]));
+        return 0;
+    }
+    if (!std::strcmp(what, "candidates")) {
+        for (const ScanTune &t : exact_candidates(10))
+            std::printf("%d %d %d %d\n", t.mode, t.defer_blocks, t.first_blocks, t.spec_levels);
         return 0;
     }
     return 2;

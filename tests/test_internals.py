@@ -40,3 +40,10 @@ def test_admission_counts_two_thirds_of_the_records(internals, segs):
     assert most[0] == most[1]  # bounded
     none = internals("estimate", segs, 1, 4096, k, np)[0][0]
     assert most[0] - none <= 8 << 30
+
+
+def test_autotuner_tries_every_level_set_at_the_built_in_line(internals):
+    cands = internals("candidates")
+    assert cands[0] == [-1, -1, -1, -1]
+    for levels in (1, 2, 3, 4):
+        assert any(mode == 0 and defer == -1 and lv == levels for mode, defer, _, lv in cands)
