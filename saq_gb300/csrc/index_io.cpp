@@ -257,6 +257,16 @@ cudaEvent_t SearchCtx::join_event() {
     return ev_join;
 }
 
+// Every stream and event above, so that later searches create none.
+void SearchCtx::create_streams() {
+    aux_stream();
+    low_stream();
+    fork_event();
+    join_event();
+    qfork_event();
+    qjoin_event();
+}
+
 int64_t Index::max_blocks_of_probes(int64_t nprobe) const {
     if (top_blocks_prefix.empty()) return 1;
     return std::max<int64_t>(1, top_blocks_prefix[std::min<int64_t>(nprobe, (int64_t)top_blocks_prefix.size() - 1)]);

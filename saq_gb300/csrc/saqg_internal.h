@@ -113,6 +113,7 @@ struct SearchCtx {
     cudaStream_t low_stream();
     cudaEvent_t qfork_event();
     cudaEvent_t qjoin_event();
+    void create_streams();
     size_t held_bytes() const { return scratch_bytes + split_scratch_bytes; }
 };
 
@@ -221,8 +222,8 @@ void clamp_shape(const int *np, const int *k, int64_t nq, int np_max, int k_max,
 // those of the first arena alone.
 size_t search_bytes_estimate(const Index &idx, int64_t nq, int64_t topk, int64_t nprobe);
 size_t search_arena1_bytes(const Index &idx, int64_t nq, int64_t topk, int64_t nprobe);
-// Grows a context's arenas (and creates its stream, events and BLAS handle)
-// for batches up to this shape, so later searches allocate nothing.
+// Grows a context's arenas (and creates its streams and events) for batches up to
+// this shape, so later searches allocate nothing.
 void presize_ctx(const Index &idx, SearchCtx &ctx, int64_t nq, int64_t topk, int64_t nprobe);
 // saqg_search for device pointers with its scratch in a static device array.
 void run_search_static(const Index &idx, const float *q, int64_t nq, int64_t topk, int64_t nprobe, float m,
@@ -257,7 +258,7 @@ void run_search_tc(const Index &idx, const float *q, int64_t nq, int64_t topk, i
                    float m, uint32_t *ids, float *dists, float *approx, int mem, cudaStream_t st,
                    saqg_tc_stats *stats, const int *np_host = nullptr, const int *k_host = nullptr,
                    const TcOpts *opts = nullptr);
-// Device scratch bytes of a tensor-core call of this shape with a candidate capacity.
+// The same for tensor-core calls of this shape with a candidate capacity.
 void presize_tc_ctx(const Index &idx, SearchCtx &ctx, int64_t nq, int64_t topk, int64_t nprobe, int64_t shortlist,
                     int64_t cand_cap);
 

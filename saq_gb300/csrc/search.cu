@@ -3807,15 +3807,8 @@ void presize_ctx(const Index &I, SearchCtx &C, int64_t nq, int64_t topk, int64_t
     C.scratch_get(search_scratch_bytes(I, nq, topk, nprobe, false));
     int64_t pos_cap = 0;
     split_scratch_take(I, C, nq, topk, nprobe, nq * I.max_blocks_of_probes(nprobe), pos_cap, nullptr);
-    C.aux_stream();
-    C.fork_event();
-    C.join_event();
-    C.low_stream();
-    C.qfork_event();
-    C.qjoin_event();
+    C.create_streams();
 }
-
-
 
 // Records for two thirds of the blocks, and 8 GB at most, are enough to admit a batch (the
 // heaviest queries come first, the CTA scan takes those that are left without); a few

@@ -948,6 +948,7 @@ void presize_tc_ctx(const Index &I, SearchCtx &C, int64_t nq, int64_t topk, int6
     std::lock_guard<std::mutex> lock(C.mu);
     C.scratch_get(tc_arena1_bytes(I, nq, topk, nprobe, L));
     C.split_scratch_get(tc_arena2_bytes(I.view, cand_cap, nq * nprobe, cand_cap / kTcSelChunk + nq, L));
+    C.create_streams();
 }
 
 void run_search_tc(const Index &I, const float *q, int64_t nq, int64_t topk, int64_t nprobe, int64_t L, float m,

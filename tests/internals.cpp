@@ -1,5 +1,5 @@
 // What the library's host code decides, printed for tests/test_internals.py (built
-// there against libsaqg.so).  No GPU needed: `estimate`, `candidates`.
+// there against libsaqg.so).  Without a GPU: `estimate`, `candidates`; with one: `presize`.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -26,6 +26,18 @@ static void estimate(int S, int64_t blocks, int64_t nq, int64_t k, int64_t np) {
     std::printf("%zu\n", search_bytes_estimate(I, nq, k, np));
 }
 
+static int presize(const char *path) {
+    Index *I = load_index_file(path);
+    {
+        SearchCtx c;
+        presize_tc_ctx(*I, c, 64, 10, 4, 40, 100000);
+        std::printf("%d %d %d %d %d %d\n", c.aux != nullptr, c.low != nullptr, c.ev_fork != nullptr,
+                    c.ev_join != nullptr, c.ev_qfork != nullptr, c.ev_qjoin != nullptr);
+    }
+    delete I;
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const char *what = argc > 1 ? argv[1] : "";
     if (!std::strcmp(what, "estimate") && argc == 7) {
@@ -37,5 +49,6 @@ int main(int argc, char **argv) {
             std::printf("%d %d %d %d\n", t.mode, t.defer_blocks, t.first_blocks, t.spec_levels);
         return 0;
     }
+    if (!std::strcmp(what, "presize") && argc == 3) return presize(argv[2]);
     return 2;
 }

@@ -47,3 +47,11 @@ def test_autotuner_tries_every_level_set_at_the_built_in_line(internals):
     assert cands[0] == [-1, -1, -1, -1]
     for levels in (1, 2, 3, 4):
         assert any(mode == 0 and defer == -1 and lv == levels for mode, defer, _, lv in cands)
+
+
+@pytest.mark.gpu
+def test_tensor_core_slot_has_its_streams(internals, golden_case_by_name):
+    """A context sized ahead for the tensor-core form has the streams and events that form
+    forks onto, so its first batch creates none."""
+    from conftest import INDEX_CASES
+    assert internals("presize", golden_case_by_name(INDEX_CASES[0])) == [[1] * 6]
