@@ -3604,6 +3604,7 @@ int xstride_of(const DevIndexView &) { return 0; }  // re-rank reads ex-codes in
 void check_launch(const char *what) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) throw Error{SAQG_ERR_CUDA, std::string(what) + " launch failed: " + cudaGetErrorString(e)};
+    count_launch(1);
 }
 
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per (kernel, device)
@@ -3710,7 +3711,6 @@ void launch_qprep(const DevIndexView &ix, const float *q, int64_t nq, float m, f
     check_launch("k_qprep_tiled");
     k_prune_bounds<<<(unsigned)((nq * ix.S + 7) / 8), 256, 0, st>>>(ix, q, (int)nq, m, prune);
     check_launch("k_prune_bounds");
-    count_launch(1);
 }
 
 }  // namespace
@@ -3726,7 +3726,6 @@ void clamp_shape(const int *np, const int *k, int64_t nq, int np_max, int k_max,
     if (nq <= 0 || (!np && !k)) return;
     k_clamp_shape<<<(unsigned)((nq + 255) / 256), 256, 0, st>>>(np, k, (int)nq, np_max, k_max, np_out, k_out);
     check_launch("k_clamp_shape");
-    count_launch(1);
 }
 
 namespace {
@@ -3990,7 +3989,6 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
             k_lut<<<(unsigned)((items + kLutWarps - 1) / kLutWarps), kLutWarps * 32, lsm, st>>>(
                 ix, probe, qsh, nullptr, nullptr, (int)nq, skip, qrot, prune, scan_lut, scan_scal);
             check_launch("k_lut");
-            count_launch(1);
             pp.lut = scan_lut;
             pp.scal = scan_scal;
             pp.np_max = (int)nprobe;
@@ -4005,13 +4003,11 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
             k_scan_warp<<<(unsigned)((nq + kWarpsPerCta - 1) / kWarpsPerCta), kWarpsPerCta * 32, wsm, st>>>(
                 ix, probe, (int)nprobe, (int)nq, qrot, prune, (int)topk, ids_out, d_out, cnt, per_warp);
             check_launch("k_scan_warp");
-            count_launch(4);
         } else if (mode == 0 && no_deferral(I, nprobe, tune)) {
             // no query of this call can probe more blocks than the deferral
             // threshold: the CTA scan answers every query, no split pass
             launch_cta_scan(scan_ws(tune), ix, probe, qsh, qrot, prune, ids_out, d_out, cnt, xs, nullptr, nq, order,
                             nullptr, scan_prep, st);
-            count_launch(4);
         } else {
             // split-pass state: every query (mode 1), or the deferred giant-cluster queries (mode 0)
             const int64_t max_pos = I.max_blocks_of_probes(nprobe);
@@ -4100,7 +4096,6 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
                 k_lut<<<(unsigned)((items + kLutWarps - 1) / kLutWarps), kLutWarps * 32, lsm, sp>>>(
                     ix, probe, qsh, ss.qlist, ss.nlist, (int)pslots, nullptr, qrot, prune, prep_lut, prep_scal);
                 check_launch("k_lut");
-                count_launch(1);
                 prep.lut = prep_lut;
                 prep.scal = prep_scal;
                 prep.np_max = (int)nprobe;
@@ -4144,7 +4139,6 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
                 SAQG_CUDA_TRY(cudaEventRecord(C.join_event(), sp));
                 SAQG_CUDA_TRY(cudaStreamWaitEvent(st, C.join_event(), 0));
             }
-            count_launch(mode == 0 ? 8 : 8);
         }
         if (stats) SAQG_CUDA_TRY(cudaEventRecord(ev[3], st));
     }
@@ -4273,7 +4267,6 @@ int64_t run_estimate(const Index &I, const float *q_host, int64_t nprobe, float 
         k_estimate<<<(unsigned)tiles.size(), kScanThreads, smem, st>>>(ix, probe, dtiles, doff, qrot, prune, oids, oacc, ofast,
                                                                        ovars, xs);
         check_launch("k_estimate");
-        count_launch(4);
         const int64_t nw = std::min(total, cap);
         SAQG_CUDA_TRY(cudaMemcpy(ids, oids, 4 * nw, cudaMemcpyDeviceToHost));
         SAQG_CUDA_TRY(cudaMemcpy(acc, oacc, 4 * nw, cudaMemcpyDeviceToHost));
@@ -4403,7 +4396,6 @@ void run_search_static(const Index &I, const float *q, int64_t nq, int64_t topk,
     k_scan<<<(unsigned)nq, kScanThreads, smem_k, st>>>(ix, probe, qsh, qrot, prune, ids, dists, nullptr,
                                                       xstride_of(ix), nullptr, nullptr, Prepared{});
     check_launch("k_scan");
-    count_launch(4);
 }
 
 // ------------------------------------------ tensor-core form: probes and re-rank
@@ -4706,7 +4698,6 @@ void tc_rank_rotate(const Index &I, SearchCtx &C, const float *q, int64_t nq, in
         check_launch("k_probe_select");
     }
     SAQG_CUDA_TRY(cudaStreamWaitEvent(st, C.qjoin_event(), 0));  // the rotated queries
-    count_launch(4);
 }
 
 size_t tc_probe_work_bytes(const Index &I, int64_t nq) { return sizeof(Cand) * (size_t)nq * I.K; }
@@ -4728,7 +4719,6 @@ void tc_rerank(const Index &I, const uint32_t *probe, int64_t nq, int64_t nprobe
     k_tc_topk<<<(unsigned)nq, kScanThreads, 8 * (size_t)L2, st>>>(ix, probe, (int)nprobe, lp, sl_pos, sl_apx, sl_cnt,
                                                                   sl_dist, L, L2, (int)topk, qk, ids, dists, apx);
     check_launch("k_tc_topk");
-    count_launch(2);
 }
 
 }  // namespace saqg

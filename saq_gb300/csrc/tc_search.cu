@@ -864,6 +864,7 @@ void ensure_tc_state(const Index &I, cudaStream_t st) {
 void launch_check(const char *what) {
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) throw Error{SAQG_ERR_CUDA, std::string(what) + " launch failed: " + cudaGetErrorString(e)};
+    count_launch(1);
 }
 
 size_t a16(size_t x) { return (x + 15) & ~size_t(15); }
@@ -1175,7 +1176,6 @@ void run_search_tc(const Index &I, const float *q, int64_t nq, int64_t topk, int
     tc_rerank(I, probe, nq, nprobe, qrot, prune, lp, sl_pos, sl_apx, sl_cnt, (int)L, topk, qk, sl_dist,
               host ? oid : ids, host ? od : dists, host ? oa : approx, st);
     mark(5);
-    count_launch(capped ? 12 : 11);
     if (host) {
         SAQG_CUDA_TRY(cudaMemcpyAsync(ids, oid, 4 * (size_t)nq * topk, cudaMemcpyDeviceToHost, st));
         if (dists) SAQG_CUDA_TRY(cudaMemcpyAsync(dists, od, 4 * (size_t)nq * topk, cudaMemcpyDeviceToHost, st));
