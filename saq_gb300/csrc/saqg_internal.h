@@ -222,6 +222,8 @@ void clamp_shape(const int *np, const int *k, int64_t nq, int np_max, int k_max,
 // those of the first arena alone.
 size_t search_bytes_estimate(const Index &idx, int64_t nq, int64_t topk, int64_t nprobe);
 size_t search_arena1_bytes(const Index &idx, int64_t nq, int64_t topk, int64_t nprobe);
+// Blocks of a speculative tile of the split pass in scan mode `mode`.
+int spec_tile_blocks(int mode, int64_t nq);
 // Grows a context's arenas (and creates its streams and events) for batches up to
 // this shape, so later searches allocate nothing.
 void presize_ctx(const Index &idx, SearchCtx &ctx, int64_t nq, int64_t topk, int64_t nprobe);

@@ -1,5 +1,5 @@
 // What the library's host code decides, printed for tests/test_internals.py (built
-// there against libsaqg.so).  Without a GPU: `estimate`, `candidates`; with one: `presize`.
+// there against libsaqg.so).  Without a GPU: `estimate`, `candidates`, `tiles`; with one: `presize`.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -47,6 +47,11 @@ int main(int argc, char **argv) {
     if (!std::strcmp(what, "candidates")) {
         for (const ScanTune &t : exact_candidates(10))
             std::printf("%d %d %d %d\n", t.mode, t.defer_blocks, t.first_blocks, t.spec_levels);
+        return 0;
+    }
+    if (!std::strcmp(what, "tiles")) {
+        for (int mode : {0, 1})
+            for (int64_t nq : {1, 16, 17, 4096}) std::printf("%d %d %d\n", mode, (int)nq, spec_tile_blocks(mode, nq));
         return 0;
     }
     if (!std::strcmp(what, "presize") && argc == 3) return presize(argv[2]);

@@ -55,3 +55,8 @@ def test_tensor_core_slot_has_its_streams(internals, golden_case_by_name):
     forks onto, so its first batch creates none."""
     from conftest import INDEX_CASES
     assert internals("presize", golden_case_by_name(INDEX_CASES[0])) == [[1] * 6]
+
+
+def test_only_a_few_queries_get_short_tiles(internals):
+    for mode, nq, blocks in internals("tiles"):
+        assert blocks == (4 if mode == 1 and nq <= 16 else 16)
