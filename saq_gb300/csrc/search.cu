@@ -1336,16 +1336,6 @@ __device__ __forceinline__ void tile_candidates(const DevIndexView &ix, ScanSmem
         if (barid) asm volatile("bar.sync %0, %1;" ::"r"(barid), "r"(nthr) : "memory");
         else __syncthreads();
     };
-    // pull a block's codes into L1, a line of 128 bytes per lane at a time
-    auto pull_codes = [&](int b) {
-        for (int s = 0; s < S; ++s) {
-            const SegDev &g = ix.seg[s];
-            const int lines = g.bits ? g.dim / 64 * 2 : 0;
-            const char *p = reinterpret_cast<const char *>(g.codes) + (size_t)(b0 + b) * lines * 128;
-            for (int l = lane; l < lines; l += 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(p + l * 128));
-        }
-    };
-    if (w < ng) pull_codes(blk(w));
 #pragma unroll 1
     for (int slot = w; slot < nslots; slot += nwarps) {
         if (slot >= ng) {
@@ -1353,7 +1343,6 @@ __device__ __forceinline__ void tile_candidates(const DevIndexView &ix, ScanSmem
             continue;
         }
         const int b = blk(slot);
-        if (slot + nwarps < ng) pull_codes(blk(slot + nwarps));
         block_estimates(ix, b0 + b, sm, slot, lane, tau);
         // the mask reads only what this warp's estimates wrote (the slot's cd, cur,
         // stage and nstage rows): a warp barrier orders them
