@@ -43,10 +43,9 @@ constexpr int kScanThreads = kScanWarps * 32;
 constexpr int kBlocksPerWarp = 2;
 constexpr int kTileB = kScanWarps * kBlocksPerWarp;  // blocks per tile
 constexpr int kMaxTopK = 4096;
-// Candidates of a tile up to which half-warps take the accurate distances: the other
-// form's time is the chain over the widest segment, so the line lies lower where that is short.
-constexpr int kItemCands = 16, kItemCandsNarrow = 8;
-constexpr int kNarrowDim = 512;
+// Candidates of a tile up to which half-warps take the accurate distances, with one
+// segment and with several (whose tasks spread over the warps by themselves).
+constexpr int kItemCands = 16, kItemCandsSegs = 6;
 constexpr int kScanMinCtas = 4;  // resident scan CTAs per SM the register budget is sized for
 
 struct SegScal {
@@ -1374,16 +1373,16 @@ __device__ __forceinline__ void tile_candidates(const DevIndexView &ix, ScanSmem
         }
     }
     sync();
-    // Accurate distances.  Few candidates (at most kItemCands): work items of two
-    // candidates of one segment, a half-warp each (excode_ip16), the widest segments
-    // first; a warp takes every nwarps-th.  More: one thread per (candidate, segment)
-    // (excode_ip_thread), the tasks of a segment from a warp boundary on, which takes
-    // half the instructions.  The line lies where the two
-    // cross: 256 queries of 1,536 dimensions (about 13 candidates a tile) take 1.67 ms
-    // with half-warps up to 16 candidates and 2.51 without, 37 queries with k = 100
-    // (about 75) 4.04 ms without and 4.65 with half-warps up to 96.  Segments of 64, 192 and
-    // 320 dimensions, 1,500 queries: 5.23 ms with the line at 8, 5.58 at 16 (one segment of
-    // 768: 4.81 and 4.71; 1,536: 1.33 and 1.19).
+    // Accurate distances.  Few candidates (at most kItemCands, or kItemCandsSegs): work
+    // items of two candidates of one segment, a half-warp each (excode_ip16), the widest
+    // segments first; a warp takes every nwarps-th.  More: one thread per (candidate,
+    // segment) (excode_ip_thread), the tasks of a segment from a warp boundary on, which
+    // takes half the instructions.  The lines lie where the two cross.  One segment (a
+    // single warp's tasks, each a chain over every dimension): 256 queries of 1,536
+    // dimensions, about 13 candidates a tile, 1.20 ms with half-warps up to 16 candidates,
+    // 1.34 up to 8, 1.63 without.  Several: 4,000 queries of an anisotropic 400,000 x 1024
+    // index, many candidates, 11.8 / 12.0 / 12.1 / 12.3 / 12.6 ms with half-warps up to 0 /
+    // 4 / 6 / 8 / 12, 1,500 of Zipf clusters of that size, few, 4.13 / 3.97 / 3.96 / 3.89 / 3.85.
     // The FP64 step of the distance (accurate_dist) would cost a warp's issue for two
     // lanes, so lane 2i, 2i + 1 keep the products of the warp's i-th item and up to 32
     // of them take that step together.
@@ -1422,9 +1421,7 @@ __device__ __forceinline__ void tile_candidates(const DevIndexView &ix, ScanSmem
         held = 0;
         __syncwarp();
     };
-    int widest = 0;
-    for (int s = 0; s < S; ++s) widest = max(widest, ix.seg[s].dim);
-    if (ncand > (widest < kNarrowDim ? kItemCandsNarrow : kItemCands)) {
+    if (ncand > (S > 1 ? kItemCandsSegs : kItemCands)) {
         const int P = (ncand + 31) >> 5;  // warps' worth of tasks per segment
         for (int t = w; t < S * P; t += nwarps) {
             const int si = t / P, r0 = (t - si * P) * 32, s = S - 1 - si;
