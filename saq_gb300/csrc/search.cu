@@ -2394,6 +2394,10 @@ constexpr int kNumSpecLevelSets = (int)(sizeof(kSpecLevelSets) / sizeof(kSpecLev
 // CTA scan, so the line lies low: 37 queries of 1,800 blocks 4.23 ms with 1,024
 // and 1.73 with 256, 256 queries of 560 blocks 1.72 and 1.22, 4,096 queries over
 // 10M vectors 2.90 and 2.15 (384: 2.13, 192: 2.21).
+// When most queries lie above the built-in line, all of them take the split pass: the CTA
+// scan of the rest would hold SMs that its short kernels wait for (600 queries of about
+// 340 blocks on an anisotropic 400,000 x 576 index: 2.25 ms at the line, 1.93 without
+// deferral, 1.66 all deferred).
 constexpr int kDeferBlocks = 256;
 
 struct SplitState {
@@ -3251,8 +3255,9 @@ __global__ void __launch_bounds__(256) k_qblocks(DevIndexView ix, const uint32_t
 }
 
 __global__ void __launch_bounds__(kDeferThreads) k_defer(DevIndexView ix, const uint32_t *__restrict__ probe, int nq,
-                                                         int defer_blocks, SplitState st, int *__restrict__ qblocks,
-                                                         int have_qblocks, uint8_t *__restrict__ deferred) {
+                                                         int defer_blocks, int majority, SplitState st,
+                                                         int *__restrict__ qblocks, int have_qblocks,
+                                                         uint8_t *__restrict__ deferred) {
     __shared__ long long wsum_b[kDeferThreads / 32];
     __shared__ int wsum_n[kDeferThreads / 32], hist[32];
     __shared__ long long s_base;  // record positions handed out
@@ -3265,6 +3270,17 @@ __global__ void __launch_bounds__(kDeferThreads) k_defer(DevIndexView ix, const 
             if (lane == 0) qblocks[qi] = total;
         }
         __syncthreads();
+    }
+    if (majority) {  // with most queries above the line, all of them
+        int over = 0;
+        for (int qi = q0; qi < q1; ++qi) over += qblocks[qi] > defer_blocks;
+        over = __reduce_add_sync(0xffffffffu, over);
+        if (lane == 0) wsum_n[w] = over;
+        __syncthreads();
+        over = 0;
+        for (int i = 0; i < nw; ++i) over += wsum_n[i];
+        if (2 * over > nq) defer_blocks = -1;
+        __syncthreads();  // the sums are used again
     }
     auto eligible = [&](int qi) {
         return defer_blocks < 0 || (defer_blocks > 0 && qblocks[qi] > defer_blocks);
@@ -3573,18 +3589,26 @@ bool scan_ws(const ScanTune &t) {
 }
 
 // The deferral threshold of mode 0 (blocks of a query's probes above which it
-// takes the split pass; 0: never).
+// takes the split pass; 0: never), and whether it was given rather than built in.
+bool defer_line_given(const ScanTune &t) { return t.defer_blocks >= 0 || std::getenv("SAQG_DEFER_BLOCKS"); }
 int defer_threshold(const ScanTune &t) {
     int defer = t.defer_blocks >= 0 ? t.defer_blocks : kDeferBlocks;
     if (const char *e = std::getenv("SAQG_DEFER_BLOCKS")) defer = std::max(0, std::atoi(e));
     return defer;
 }
 
-// Whether no query of a mode-0 call can be deferred: its nprobe largest
-// clusters hold no more blocks than the threshold.
-bool no_deferral(const Index &I, int64_t nprobe, const ScanTune &t) {
+// Whether no query of a mode-0 call is deferred: its nprobe largest clusters hold no more
+// blocks than the threshold, or (built-in line, one nprobe for all: `even`) clusters of
+// about one size give equally long queries that fill one wave of the CTA scan, which
+// then ends everywhere at once (600 queries of 923 blocks, 400,000 x 576: 0.85 ms, 0.92
+// with the split pass; 480 queries, three quarters of a wave: 0.88 and 0.85).
+constexpr int kFullWave = 87, kEvenBlocks = 80;  // percent: of the resident CTAs; mean of the longest query
+bool no_deferral(const Index &I, int64_t nq, int64_t nprobe, bool even, int resident, const ScanTune &t) {
     const int defer = defer_threshold(t);
-    return defer == 0 || I.max_blocks_of_probes(nprobe) <= defer;
+    const int64_t most = I.max_blocks_of_probes(nprobe);
+    if (defer == 0 || most <= defer) return true;
+    return even && !defer_line_given(t) && nq <= resident && 100 * nq >= kFullWave * (int64_t)resident &&
+           kEvenBlocks * most * I.K <= 100 * nprobe * I.blk_off[I.K];
 }
 
 // Per-query nprobe / k copies clamped to the call's maxima (graph launches read
@@ -3677,6 +3701,12 @@ int full_grid(const void *fn, int threads, size_t smem) {
     const int g = std::max(1, sms * std::max(1, per_sm));
     have[{fn, dev, smem}] = g;
     return g;
+}
+
+// CTAs of the CTA scan that the GPU holds at once.
+int resident_scans(size_t smem) {
+    ensure_smem((const void *)k_scan, smem);
+    return full_grid((const void *)k_scan, kScanThreads, smem);
 }
 
 // Prune bounds and rotated queries of a call on `st`.  k_qprep_few spreads over the
@@ -4002,7 +4032,7 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
             k_scan_warp<<<(unsigned)((nq + kWarpsPerCta - 1) / kWarpsPerCta), kWarpsPerCta * 32, wsm, st>>>(
                 ix, probe, (int)nprobe, (int)nq, qrot, prune, (int)topk, ids_out, d_out, cnt, per_warp);
             check_launch("k_scan_warp");
-        } else if (mode == 0 && no_deferral(I, nprobe, tune)) {
+        } else if (mode == 0 && no_deferral(I, nq, nprobe, !qsh.np, resident_scans(smem), tune)) {
             // no query of this call can probe more blocks than the deferral
             // threshold: the CTA scan answers every query, no split pass
             launch_cta_scan(scan_ws(tune), ix, probe, qsh, qrot, prune, ids_out, d_out, cnt, xs, nullptr, nq, order,
@@ -4052,15 +4082,18 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
             ss.stride = mode == 1 && pos_cap >= want && max_pos < INT_MAX && !prep_lut ? max_pos : 0;
             if (!ss.stride) {
                 SAQG_CUDA_TRY(cudaMemsetAsync(ss.nlist, 0, 32, st));
-                int defer = -1;  // mode 1: every query
-                if (mode == 0) defer = defer_threshold(tune);
+                int defer = -1, majority = 0;  // mode 1: every query
+                if (mode == 0) {
+                    defer = defer_threshold(tune);
+                    majority = !defer_line_given(tune);
+                }
                 const int dthreads = (int)std::min<int64_t>(kDeferThreads, 32 * nq);  // a warp per query while they fit
                 const bool par = nq >= kQblocksMinQueries;
                 if (par) {
                     k_qblocks<<<(unsigned)((nq + 7) / 8), 256, 0, st>>>(ix, probe, qsh, (int)nq, qblocks);
                     check_launch("k_qblocks");
                 }
-                k_defer<<<1, dthreads, 0, st>>>(ix, probe, (int)nq, defer, ss, qblocks, par ? 1 : 0, deferred);
+                k_defer<<<1, dthreads, 0, st>>>(ix, probe, (int)nq, defer, majority, ss, qblocks, par ? 1 : 0, deferred);
                 check_launch("k_defer");
             }
             cudaStream_t sp = st;  // stream of the split pass

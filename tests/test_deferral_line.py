@@ -1,0 +1,85 @@
+"""The built-in deferral line on whole batches: most queries above it (all take the split
+pass), equally long queries that fill one wave of the CTA scan (none does), and a minority
+above it; answers against the oracle, and a batch with most queries above the line against
+both forms forced."""
+import numpy as np
+import pytest
+
+import oracle as O
+
+
+def _sizes(kind, K, n):
+    if kind == "equal":
+        return np.full(K, n // K)
+    w = (np.arange(1, K + 1) ** -0.5) if kind == "spread" else np.arange(1, K + 1) ** -1.2
+    return np.maximum(1, (w / w.sum() * n).astype(np.int64))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["equal", "spread", "heavy"])
+@pytest.mark.parametrize("nq", [70, 560, 608, 700])
+def test_whole_batches(kind, nq, tmp_path):
+    from saq_gb300 import ivf
+    rng = np.random.default_rng(nq)
+    D, K = 64, 40
+    sizes = _sizes(kind, K, 40000)
+    cids = np.repeat(np.arange(K), sizes).astype(np.uint32)
+    rng.shuffle(cids)
+    cent = rng.standard_normal((K, D)).astype(np.float32)
+    x = (cent[cids] + 0.7 * rng.standard_normal((len(cids), D))).astype(np.float32)
+    q = (cent[rng.integers(0, K, nq)] + 0.7 * rng.standard_normal((nq, D))).astype(np.float32)
+    path = str(tmp_path / "d.index")
+    O.build_index(path, x, cent, cids, 4.0, False, 0, None)
+    ids, d = ivf.IVF.load(path).search(q, 10, 12, return_dists=True)
+    oi, od = O.OracleIndex(path).search(q, 10, 12, threads=16, with_dists=True)
+    assert np.array_equal(ids, oi) and np.array_equal(d.view(np.uint32), od.view(np.uint32))
+
+
+def _spread_index(clusters, n=400000, D=576):
+    """Vectors of a falling spectrum around sampled centroids: lengths of queries vary, little is pruned."""
+    import torch
+    from saq_gb300 import ivf
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    scale = torch.arange(1, D + 1, device="cuda").float().pow(-0.4)
+
+    def draw(m):
+        return torch.nn.functional.normalize(torch.randn(m, D, generator=g, device="cuda") * scale, dim=1)
+    x = draw(n)
+    cent = x[torch.randperm(n, generator=g, device="cuda")[:clusters]].clone()
+    cids = torch.cat([torch.argmin((cent * cent).sum(1)[None] - 2 * x[a:a + 50000] @ cent.T, 1)
+                      for a in range(0, n, 50000)])
+    ix = ivf.IVF(n, D, clusters, ivf.QuantizeConfig(avg_bits=4.0))
+    ix.construct(x, cent.cpu().numpy(), cids.cpu().numpy().astype(np.uint32), seed=2)
+    return ix, draw
+
+
+def _ms(ix, q, nprobe, monkeypatch, **env):
+    """Best time of a search under these settings."""
+    import torch
+    for name in ("SAQG_DEFER_BLOCKS", "SAQG_SCAN_MODE"):
+        if name in env:
+            monkeypatch.setenv(name, env[name])
+        else:
+            monkeypatch.delenv(name, raising=False)
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    best = 1e9
+    for _ in range(6):
+        torch.cuda.synchronize()
+        a.record()
+        ix.search(q, 10, nprobe)
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b))
+    return best
+
+
+@pytest.mark.gpu
+def test_a_batch_above_the_line_is_not_slower_than_either_form(monkeypatch):
+    """600 queries of about 340 blocks, 256 being the line: with part of them on each form
+    the call took 1.5 times the split pass of all."""
+    ix, draw = _spread_index(4000)
+    q = draw(600)
+    built_in, none, every = (_ms(ix, q, 48, monkeypatch, **e)
+                             for e in ({}, {"SAQG_DEFER_BLOCKS": "0"}, {"SAQG_DEFER_BLOCKS": "1"}))
+    assert built_in < 1.15 * min(none, every), (built_in, none, every)
