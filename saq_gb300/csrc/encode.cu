@@ -858,6 +858,28 @@ struct DevBuf {
 
 }  // namespace
 
+// Vectors that the construction's encoder holds at once at this width: kEncCtas warps an
+// SM, fewer where the table of code values takes more shared memory (12 at 6 bits).
+int64_t encoder_vectors(int bits) {
+    int per_sm = 0;
+    by_width(bits, [&](auto w) {
+        SAQG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_caq_encode_clustered<decltype(w)::value>,
+                                                                    kEncThreads, enc_smem_bytes(bits)));
+    });
+    return (int64_t)encoder_sms() * std::max(1, per_sm) * 32;
+}
+
+// Vectors of a chunk of the construction of n vectors: equal chunks of whole 32-vector
+// groups (residuals and codes are warp-interleaved), each no more than the encoder holds
+// at once, since a few warps left for a second wave would take as long as a full one
+// (125,000 x 512 at 6 bits: 9.2 ms with chunks for 21 warps an SM, 8.4 for its 12).
+int64_t encode_chunk(int64_t n, int bits, int64_t maxd) {
+    const int64_t at_once =
+        std::max<int64_t>(32, std::min<int64_t>((int64_t)(1u << 30) / (8 * maxd), encoder_vectors(bits)) / 32 * 32);
+    const int64_t nchunk = std::max<int64_t>(1, (n + at_once - 1) / at_once);
+    return std::max<int64_t>(32, ((n + nchunk - 1) / nchunk + 31) / 32 * 32);
+}
+
 // IVF::construct (index/ivf.hpp:130-184): group by cluster, plan, then per
 // segment rotate / encode / pack on the GPU, in chunks of vectors.
 Index *construct_index(const float *data, int64_t n, int64_t dim, const float *centroids, int64_t k,
@@ -988,14 +1010,9 @@ Index *construct_index(const float *data, int64_t n, int64_t dim, const float *c
     }
     int64_t maxd = 0;
     for (auto &sg : X.segs) maxd = std::max(maxd, sg.dim);
-    // equal chunks of whole 32-vector groups (residuals and codes are
-    // warp-interleaved), each no more than the encoder holds at once: a few warps left
-    // for a second wave would take as long as a full one
-    const int64_t at_once = std::max<int64_t>(
-        32, std::min<int64_t>((int64_t)(1u << 30) / (8 * maxd), (int64_t)encoder_sms() * kEncCtas * 32) / 32 * 32);
-    const int64_t nchunk = std::max<int64_t>(1, (n + at_once - 1) / at_once);
-    const int64_t chunk = std::max<int64_t>(32, ((n + nchunk - 1) / nchunk + 31) / 32 * 32);
-    const int64_t chunk_pad = (std::min(chunk, n) + 31) / 32 * 32;
+    int64_t most = 0;
+    for (auto &sg : X.segs) most = std::max(most, encode_chunk(n, (int)sg.bits, maxd));
+    const int64_t chunk_pad = (std::min(most, n) + 31) / 32 * 32;
     DevBuf resid(4 * (size_t)chunk_pad * maxd), codes(2 * (size_t)chunk_pad * maxd), facs(16 * (size_t)chunk_pad);
     DevBuf cslice(4 * (size_t)k * maxd);
     int off = 0;
@@ -1046,6 +1063,7 @@ Index *construct_index(const float *data, int64_t n, int64_t dim, const float *c
             SAQG_CUDA_TRY(cudaMemcpy(idbuf->p, ident.data(), 4 * d * d, cudaMemcpyHostToDevice));
             idP = idbuf.get();
         }
+        const int64_t chunk = encode_chunk(n, g.bits, maxd);
         for (int64_t v0 = 0; v0 < n; v0 += chunk) {
             const int64_t nv = std::min(chunk, n - v0);
             dim3 grid((unsigned)(d / kRotN), (unsigned)((nv + kRotM - 1) / kRotM));

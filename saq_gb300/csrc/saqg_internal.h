@@ -313,6 +313,9 @@ void server_run_trace(Server *s, const float *queries, int64_t n, const double *
 // encode.cu
 void run_caq_encode(const float *resid, int64_t n, int64_t dim, int bits, const float *cent, int rdlmt, float eps,
                     int32_t *codes, float *facs, int mem, cudaStream_t st);
+// Vectors the construction encodes at a time, and those its encoder holds at once.
+int64_t encode_chunk(int64_t n, int bits, int64_t maxd);
+int64_t encoder_vectors(int bits);
 Index *construct_index(const float *data, int64_t n, int64_t dim, const float *centroids, int64_t k,
                        const uint32_t *cids, const saqg_quantize_config &cfg, const float *variance,
                        const float *rotations, uint64_t seed, int data_mem);

@@ -1,5 +1,5 @@
 // What the library's host code decides, printed for tests/test_internals.py (built
-// there against libsaqg.so).  Without a GPU: `estimate`, `candidates`, `tiles`; with one: `presize`.
+// there against libsaqg.so).  Without a GPU: `estimate`, `candidates`, `tiles`; with one: `presize`, `chunks`.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -52,6 +52,12 @@ int main(int argc, char **argv) {
     if (!std::strcmp(what, "tiles")) {
         for (int mode : {0, 1})
             for (int64_t nq : {1, 16, 17, 4096}) std::printf("%d %d %d\n", mode, (int)nq, spec_tile_blocks(mode, nq));
+        return 0;
+    }
+    if (!std::strcmp(what, "chunks") && argc == 4) {
+        const int64_t n = std::atoll(argv[2]), maxd = std::atoll(argv[3]);
+        for (int bits = 0; bits <= kMaxBits; ++bits)
+            std::printf("%d %lld %lld\n", bits, (long long)encode_chunk(n, bits, maxd), (long long)encoder_vectors(bits));
         return 0;
     }
     if (!std::strcmp(what, "presize") && argc == 3) return presize(argv[2]);

@@ -60,3 +60,14 @@ def test_tensor_core_slot_has_its_streams(internals, golden_case_by_name):
 def test_only_a_few_queries_get_short_tiles(internals):
     for mode, nq, blocks in internals("tiles"):
         assert blocks == (4 if mode == 1 and nq <= 16 else 16)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 60000, 125000, 1000003])
+def test_encoder_chunks_fit_one_wave_at_every_width(internals, n):
+    held = []
+    for bits, chunk, at_once in internals("chunks", n, 512):
+        assert chunk % 32 == 0 and 32 <= chunk <= at_once
+        assert chunk >= min(n, at_once) / 2 - 32  # equal shares, not a full one and a rest
+        held.append(at_once)
+    assert min(held) < max(held)  # 6-bit codes keep their values in a larger table
