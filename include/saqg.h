@@ -133,11 +133,12 @@ typedef struct saqg_search_stats {
     float ms_scan;         /* the cluster scan (FastScan + re-rank + top-k) */
     float ms_total;        /* first to last kernel */
     int64_t probes;        /* (query, cluster) pairs scanned */
-    int64_t blocks;        /* 32-vector blocks scanned */
+    int64_t blocks;        /* 32-vector blocks of the probed clusters */
     int64_t vectors;       /* vectors scanned */
     int64_t reranked;      /* vectors whose accurate distance the reference evaluates */
     int64_t speculative;   /* accurate distances evaluated (a superset of `reranked`) */
-    int64_t fast_bytes;    /* algorithmic bytes of the scan: 1-bit codes, |o| factors, centroids */
+    int64_t fast_bytes;    /* algorithmic bytes of a scan of those blocks: 1-bit codes, |o| factors, centroids
+                              (the codes of blocks that the first pruning stage drops are not read) */
     int64_t rerank_bytes;  /* algorithmic bytes of the re-rank: ex-codes, ex factors, ids */
     float ms_split;        /* the split pass for giant-cluster queries (auxiliary stream; 0 if unused) */
     float ms_split_first;  /* ... its exact prefix scans (the speculation bounds) */

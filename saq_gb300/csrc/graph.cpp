@@ -1,7 +1,7 @@
 // A batched search of a fixed shape captured into a CUDA graph: its own
 // search context is sized once, a warm-up call builds whatever is built lazily
-// (centroid norms, kernel attributes, the BLAS handle and workspace, the
-// tensor-core code matrix), and the next call is captured on a private stream.
+// (centroid norms, kernel attributes, the tensor-core code matrix), and the next
+// call is captured on a private stream.
 // Each launch then replays all of the search's kernels and copies with one
 // call, on the caller's buffers bound at capture time (queries, and per-query
 // nprobe / topk arrays when given, updated in place between launches).

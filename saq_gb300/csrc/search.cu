@@ -3759,7 +3759,7 @@ void clamp_shape(const int *np, const int *k, int64_t nq, int np_max, int k_max,
 namespace {
 
 
-// Centroid ranking of a batch: TF32 GEMM of inner products, the shortlist
+// Centroid ranking of a batch: BF16 GEMM of inner products, the shortlist
 // kernel, and the full exact path for the queries it hands back.
 void probe_shortlist(const Index &I, SearchCtx &C, const float *q, int64_t nq, int64_t nprobe, const int *qnp,
                      float *dist, uint32_t *probe, uint8_t *full, int *fb_list, int *flags, Cand *work,
@@ -4216,9 +4216,10 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
         stats->probe_exact = shortlist ? (int64_t)hc[4] : nq * I.K;
         stats->probe_full = shortlist ? (int64_t)(hc[5] + hc[6]) : nq;
         stats->probe_full_ties = (int64_t)hc[6];
-        // Algorithmic bytes: per scanned block 32 lanes of 1-bit codes of
-        // every coded segment and |o| of every segment; per probe the rotated centroid;
-        // per re-ranked vector its ex-codes, ex factors and id.
+        // Algorithmic bytes: per block of a probed cluster 32 lanes of 1-bit codes of
+        // every coded segment and |o| of every segment (also where the first pruning
+        // stage leaves the codes unread); per probe the rotated centroid; per re-ranked
+        // vector its ex-codes, ex factors and id.
         int64_t per_lane = 0, per_rr = 4;
         for (int s = 0; s < ix.S; ++s) {
             per_lane += 4 + (ix.seg[s].bits ? ix.seg[s].dim / 8 : 0);

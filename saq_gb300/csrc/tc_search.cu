@@ -29,8 +29,9 @@
 //                  thread issues tcgen05.mma (M=128, N=pairs, K=16 per instruction)
 //                  into per-segment TMEM accumulators (two, alternating by chunk),
 //                  four warps read them back with tcgen05.ld for the epilogue
-//   k_tc_select1/2 per query: the shortlist by radix select over 4,096-candidate
-//                  chunks, then over the chunks' survivors, in candidate order
+//   k_tc_select1/2 per query: the shortlist over 4,096-candidate chunks, then over the
+//                  chunks' survivors, in candidate order (candidates under a bound
+//                  collected; long shortlists and many ties by radix select)
 //   k_tc_rerank / k_tc_topk  (search.cu) exact distances of the shortlist, one CTA
 //                  per query, then top-k
 #include <cuda.h>
@@ -667,7 +668,8 @@ __device__ bool select_few(int M, int L, Key key, Emit emit) {
 }
 
 // The L smallest keys of key(e), e in [0, M) (ties: smaller e first), written
-// in ascending e as (pos(e), value(e)).  256 threads; radix select, 8 bits per pass.
+// in ascending e as (pos(e), value(e)).  256 threads; select_few, else radix select,
+// 8 bits per pass.
 template <class Key, class Emit>
 __device__ void select_smallest(int M, int L, Key key, Emit emit) {
     if (L <= kSelFew && select_few(M, L, key, emit)) return;
