@@ -2394,10 +2394,19 @@ constexpr int kNumSpecLevelSets = (int)(sizeof(kSpecLevelSets) / sizeof(kSpecLev
 // CTA scan, so the line lies low: 37 queries of 1,800 blocks 4.23 ms with 1,024
 // and 1.73 with 256, 256 queries of 560 blocks 1.72 and 1.22, 4,096 queries over
 // 10M vectors 2.90 and 2.15 (384: 2.13, 192: 2.21).
-// When most queries lie above the built-in line, all of them take the split pass: the CTA
-// scan of the rest would hold SMs that its short kernels wait for (600 queries of about
-// 340 blocks on an anisotropic 400,000 x 576 index: 2.25 ms at the line, 1.93 without
-// deferral, 1.66 all deferred).
+// With the built-in line the batch as a whole decides first, since the CTA scan of the
+// queries below it holds SMs that the split pass's short kernels wait for:
+//   * most queries above it: all of them take the split pass (600 queries of about 340
+//     blocks, anisotropic 400,000 x 576: 2.42 ms at the line, 1.95 without deferral, 1.72
+//     all deferred);
+//   * else, where no query is longer than 1.25 times a resident CTA's share of the batch,
+//     none does (4,000 queries of about 230 blocks, a third above the line, anisotropic
+//     400,000 x 576 in 600-vector clusters: 5.33 / 4.78 / 5.19 ms);
+//   * else, with three in ten above it, all (1,500 uneven queries of about 250 blocks,
+//     anisotropic 647,483 x 576: 3.72 / 3.32 / 3.17 ms; 600 of about 275, Zipf 400,000 x
+//     1024: 2.34 / 2.86 / 1.72; worst found, 4,000 of 281, Zipf: 2.49 / 3.49 / 2.72);
+//   * else those above it (a tenth to a quarter: the batch of 4,096 over 10M vectors 1.84 /
+//     8.76 / 2.32 ms).
 constexpr int kDeferBlocks = 256;
 
 struct SplitState {
@@ -3255,11 +3264,11 @@ __global__ void __launch_bounds__(256) k_qblocks(DevIndexView ix, const uint32_t
 }
 
 __global__ void __launch_bounds__(kDeferThreads) k_defer(DevIndexView ix, const uint32_t *__restrict__ probe, int nq,
-                                                         int defer_blocks, int majority, SplitState st,
+                                                         int defer_blocks, int resident, SplitState st,
                                                          int *__restrict__ qblocks, int have_qblocks,
                                                          uint8_t *__restrict__ deferred) {
     __shared__ long long wsum_b[kDeferThreads / 32];
-    __shared__ int wsum_n[kDeferThreads / 32], hist[32];
+    __shared__ int wsum_n[kDeferThreads / 32], wmost[kDeferThreads / 32], hist[32];
     __shared__ long long s_base;  // record positions handed out
     __shared__ int s_slot;        // list entries handed out
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nt = blockDim.x, nw = nt >> 5;
@@ -3271,15 +3280,33 @@ __global__ void __launch_bounds__(kDeferThreads) k_defer(DevIndexView ix, const 
         }
         __syncthreads();
     }
-    if (majority) {  // with most queries above the line, all of them
-        int over = 0;
-        for (int qi = q0; qi < q1; ++qi) over += qblocks[qi] > defer_blocks;
+    if (resident > 0) {  // the built-in line: the batch as a whole decides first (kDeferBlocks)
+        long long sum = 0;
+        int most = 0, over = 0;
+        for (int qi = q0; qi < q1; ++qi) {
+            sum += qblocks[qi];
+            most = max(most, qblocks[qi]);
+            over += qblocks[qi] > defer_blocks;
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        most = __reduce_max_sync(0xffffffffu, most);
         over = __reduce_add_sync(0xffffffffu, over);
-        if (lane == 0) wsum_n[w] = over;
+        if (lane == 0) {
+            wsum_b[w] = sum;
+            wsum_n[w] = over;
+            wmost[w] = most;
+        }
         __syncthreads();
-        over = 0;
-        for (int i = 0; i < nw; ++i) over += wsum_n[i];
-        if (2 * over > nq) defer_blocks = -1;
+        sum = over = 0;
+        for (int i = 0; i < nw; ++i) {
+            sum += wsum_b[i];
+            over += wsum_n[i];
+            most = max(most, wmost[i]);
+        }
+        const bool even = 4LL * most * resident <= 5 * sum;  // no query is much longer than a CTA's share
+        if (2 * over > nq || (!even && 10LL * over >= 3LL * nq)) defer_blocks = -1;
+        else if (even) defer_blocks = 0;
         __syncthreads();  // the sums are used again
     }
     auto eligible = [&](int qi) {
@@ -4082,10 +4109,10 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
             ss.stride = mode == 1 && pos_cap >= want && max_pos < INT_MAX && !prep_lut ? max_pos : 0;
             if (!ss.stride) {
                 SAQG_CUDA_TRY(cudaMemsetAsync(ss.nlist, 0, 32, st));
-                int defer = -1, majority = 0;  // mode 1: every query
+                int defer = -1, resident = 0;  // mode 1: every query
                 if (mode == 0) {
                     defer = defer_threshold(tune);
-                    majority = !defer_line_given(tune);
+                    resident = defer_line_given(tune) ? 0 : resident_scans(smem);
                 }
                 const int dthreads = (int)std::min<int64_t>(kDeferThreads, 32 * nq);  // a warp per query while they fit
                 const bool par = nq >= kQblocksMinQueries;
@@ -4093,7 +4120,7 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
                     k_qblocks<<<(unsigned)((nq + 7) / 8), 256, 0, st>>>(ix, probe, qsh, (int)nq, qblocks);
                     check_launch("k_qblocks");
                 }
-                k_defer<<<1, dthreads, 0, st>>>(ix, probe, (int)nq, defer, majority, ss, qblocks, par ? 1 : 0, deferred);
+                k_defer<<<1, dthreads, 0, st>>>(ix, probe, (int)nq, defer, resident, ss, qblocks, par ? 1 : 0, deferred);
                 check_launch("k_defer");
             }
             cudaStream_t sp = st;  // stream of the split pass

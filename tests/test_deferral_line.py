@@ -1,7 +1,7 @@
-"""The built-in deferral line on whole batches: most queries above it (all take the split
-pass), equally long queries that fill one wave of the CTA scan (none does), and a minority
-above it; answers against the oracle, and a batch with most queries above the line against
-both forms forced."""
+"""The built-in deferral line on whole batches: many queries above it (all take the split
+pass), equally long queries that fill one wave of the CTA scan or are short beside a long
+batch (none does), and a few above it; answers against the oracle, and batches with many
+queries above the line against both forms forced."""
 import numpy as np
 import pytest
 
@@ -17,7 +17,7 @@ def _sizes(kind, K, n):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["equal", "spread", "heavy"])
-@pytest.mark.parametrize("nq", [70, 560, 608, 700])
+@pytest.mark.parametrize("nq", [70, 560, 608, 700, 3000])
 def test_whole_batches(kind, nq, tmp_path):
     from saq_gb300 import ivf
     rng = np.random.default_rng(nq)
@@ -30,9 +30,11 @@ def test_whole_batches(kind, nq, tmp_path):
     q = (cent[rng.integers(0, K, nq)] + 0.7 * rng.standard_normal((nq, D))).astype(np.float32)
     path = str(tmp_path / "d.index")
     O.build_index(path, x, cent, cids, 4.0, False, 0, None)
-    ids, d = ivf.IVF.load(path).search(q, 10, 12, return_dists=True)
-    oi, od = O.OracleIndex(path).search(q, 10, 12, threads=16, with_dists=True)
-    assert np.array_equal(ids, oi) and np.array_equal(d.view(np.uint32), od.view(np.uint32))
+    ix, ref = ivf.IVF.load(path), O.OracleIndex(path)
+    for nprobe in (6, 12) if nq > 1000 else (12,):  # 6: some 200 blocks each
+        ids, d = ix.search(q, 10, nprobe, return_dists=True)
+        oi, od = ref.search(q, 10, nprobe, threads=16, with_dists=True)
+        assert np.array_equal(ids, oi) and np.array_equal(d.view(np.uint32), od.view(np.uint32)), nprobe
 
 
 def _spread_index(clusters, n=400000, D=576):
@@ -75,11 +77,13 @@ def _ms(ix, q, nprobe, monkeypatch, **env):
 
 
 @pytest.mark.gpu
-def test_a_batch_above_the_line_is_not_slower_than_either_form(monkeypatch):
+@pytest.mark.parametrize("nprobe,nq", [(48, 600), (22, 128)])
+def test_a_batch_above_the_line_is_not_slower_than_either_form(nprobe, nq, monkeypatch):
     """600 queries of about 340 blocks, 256 being the line: with part of them on each form
-    the call took 1.5 times the split pass of all."""
+    the call took 1.5 times the split pass of all; 128 with a third to a half above it: 1.3
+    times."""
     ix, draw = _spread_index(4000)
-    q = draw(600)
-    built_in, none, every = (_ms(ix, q, 48, monkeypatch, **e)
+    q = draw(nq)
+    built_in, none, every = (_ms(ix, q, nprobe, monkeypatch, **e)
                              for e in ({}, {"SAQG_DEFER_BLOCKS": "0"}, {"SAQG_DEFER_BLOCKS": "1"}))
     assert built_in < 1.15 * min(none, every), (built_in, none, every)
