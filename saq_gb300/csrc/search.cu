@@ -46,6 +46,7 @@ constexpr int kMaxTopK = 4096;
 // Candidates of a tile up to which half-warps take the accurate distances, with one
 // segment and with several (whose tasks spread over the warps by themselves).
 constexpr int kItemCands = 16, kItemCandsSegs = 6;
+constexpr int kPullDim = 1024;  // one segment from this width on: codes prefetched (tile_candidates)
 constexpr int kScanMinCtas = 4;  // resident scan CTAs per SM the register budget is sized for
 
 struct SegScal {
@@ -1326,15 +1327,29 @@ __device__ __forceinline__ bool stages_pass(const float *st, int n, float tau) {
 // The threads [tbase, tbase + nthr) take part (whole warps; a tile then has at
 // most nthr / 32 * kBlocksPerWarp slots); they synchronise on __syncthreads when
 // barid is 0, else on the named barrier barid.
-template <class Blk>
+// kOne: the index has one segment (a form of its own, so that neither holds the other's
+// registers).
+template <bool kOne = false, class Blk>
 __device__ __forceinline__ void tile_candidates(const DevIndexView &ix, ScanSmem &sm, int64_t b0, int64_t v0, int nb, int n, int ng,
                                 Blk blk, float tau, int tbase = 0, int nthr = kScanThreads, int barid = 0) {
-    const int S = ix.S, tid = (int)threadIdx.x - tbase, w = tid >> 5, lane = tid & 31;
+    const int S = kOne ? 1 : ix.S, tid = (int)threadIdx.x - tbase, w = tid >> 5, lane = tid & 31;
     const int nwarps = nthr >> 5, nslots = nwarps * kBlocksPerWarp;
     auto sync = [&]() {
         if (barid) asm volatile("bar.sync %0, %1;" ::"r"(barid), "r"(nthr) : "memory");
         else __syncthreads();
     };
+    // One wide segment: the next block's codes into L1 ahead of their use, a line of 128
+    // bytes per lane (256 queries of 1,536 dimensions over equal clusters, L2 cold: 0.597 ms,
+    // 0.622 without this and without the form of its own; 768 dimensions would lose 1-3% by
+    // it, several segments up to 8%).
+    const bool pull = kOne && ix.seg[0].dim >= kPullDim;
+    auto pull_codes = [&](int b) {
+        const SegDev &g = ix.seg[0];
+        const int lines = g.bits ? g.dim / 64 * 2 : 0;
+        const char *p = reinterpret_cast<const char *>(g.codes) + (size_t)(b0 + b) * lines * 128;
+        for (int l = lane; l < lines; l += 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(p + l * 128));
+    };
+    if (pull && w < ng) pull_codes(blk(w));
 #pragma unroll 1
     for (int slot = w; slot < nslots; slot += nwarps) {
         if (slot >= ng) {
@@ -1342,6 +1357,7 @@ __device__ __forceinline__ void tile_candidates(const DevIndexView &ix, ScanSmem
             continue;
         }
         const int b = blk(slot);
+        if (pull && slot + nwarps < ng) pull_codes(blk(slot + nwarps));
         block_estimates(ix, b0 + b, sm, slot, lane, tau);
         // the mask reads only what this warp's estimates wrote (the slot's cd, cur,
         // stage and nstage rows): a warp barrier orders them
@@ -1825,14 +1841,15 @@ struct ProbeHdr {
     int c, nb, n, quads;
     int64_t b0, v0;
 };
-__device__ void scan_probes(const DevIndexView &ix, const uint32_t *__restrict__ probe, int np,
+template <bool kOne>
+__device__ __forceinline__ void scan_probes(const DevIndexView &ix, const uint32_t *__restrict__ probe, int np,
                             const float *__restrict__ qrot, const float *__restrict__ prune, int topk, ScanSmem &sm,
                             int &pool_size, float &distk, ScanTally &tl, const uint16_t *__restrict__ lut,
                             const SegScal *__restrict__ scal) {
     __shared__ ProbeHdr hdr[kHdrProbes];
     __shared__ float vf[kHdrProbes * kMaxSeg];
     __shared__ uint8_t nib[2][kPassQuads];  // blocks of each group left by the filter (two passes' worth)
-    const int S = ix.S, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int S = kOne ? 1 : ix.S, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     int par = 0;
     for (int p0 = 0; p0 < np; p0 += kHdrProbes) {
         const int m = min(kHdrProbes, np - p0);
@@ -1938,7 +1955,7 @@ __device__ void scan_probes(const DevIndexView &ix, const uint32_t *__restrict__
                     const uint32_t gm = __shfl_sync(kFull, mine, g);
                     return kQuad * (first + g) + nth_bit(gm, r - (__shfl_sync(kFull, sincl, g) - __popc(gm)));
                 };
-                tile_candidates(ix, sm, h.b0, h.v0, h.nb, h.n, ng, blk, distk);
+                tile_candidates<kOne>(ix, sm, h.b0, h.v0, h.nb, h.n, ng, blk, distk);
                 if (tid < 32) {
                     float dk = distk;
                     int sz = pool_size;
@@ -3161,6 +3178,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_replay(DevIndexView ix, S
 
 // One CTA per query: the whole probe list sequentially (queries deferred to
 // the split pass are skipped).
+template <bool kOne>
 __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan(DevIndexView ix, const uint32_t *__restrict__ probe,
                                                        QueryShape qsh, const float *__restrict__ qrot_all,
                                                        const float *__restrict__ prune_all,
@@ -3178,9 +3196,10 @@ __global__ void __launch_bounds__(kScanThreads, kScanMinCtas) k_scan(DevIndexVie
     ScanTally tl;
     tl.counted = counters != nullptr;
     init_pool(sm, topk, pool_size, distk);
-    scan_probes(ix, probe + (size_t)qi * qsh.np_max, np, qrot_all + (size_t)qi * ix.Dtot,
-                prune_all + (size_t)qi * ix.S, topk, sm, pool_size, distk, tl,
-                prep.has(qi) ? prep.lut_of(qi, 0, ix.Dtot) : nullptr, prep.has(qi) ? prep.scal_of(qi, 0, ix.S) : nullptr);
+    scan_probes<kOne>(ix, probe + (size_t)qi * qsh.np_max, np, qrot_all + (size_t)qi * ix.Dtot,
+                      prune_all + (size_t)qi * ix.S, topk, sm, pool_size, distk, tl,
+                      prep.has(qi) ? prep.lut_of(qi, 0, ix.Dtot) : nullptr,
+                      prep.has(qi) ? prep.scal_of(qi, 0, ix.S) : nullptr);
     flush_tally(tl, counters);
     write_results(sm, pool_size, topk, qsh.k_max, out_ids + (size_t)qi * qsh.k_max,
                   out_d ? out_d + (size_t)qi * qsh.k_max : nullptr);
@@ -3670,6 +3689,9 @@ void ensure_smem(const void *fn, size_t bytes) {
     h = bytes;
 }
 
+// The CTA scan for an index of S segments.
+auto scan_kernel(int S) { return S == 1 ? k_scan<true> : k_scan<false>; }
+
 // The CTA-per-query scan of `nq` queries (deferred ones skipped): k_scan, with
 // the batched LUTs that prep_of(deferred) launches and returns (or none), or its
 // warp-specialised form k_scan_ws, which gives the same answers.
@@ -3692,9 +3714,10 @@ void launch_cta_scan(bool ws, const DevIndexView &ix, const uint32_t *probe, con
     }
     const size_t smem = scan_smem_bytes(ix.Dtot, ix.S, qsh.k_max, xs);
     SAQG_REQUIRE(smem <= kScanSmem, "dimension / topk too large for the scan kernel's shared memory");
-    ensure_smem((const void *)k_scan, smem);
+    const auto scan = scan_kernel(ix.S);
+    ensure_smem((const void *)scan, smem);
     const Prepared prep = prep_of(deferred);
-    k_scan<<<(unsigned)nq, kScanThreads, smem, st>>>(ix, probe, qsh, qrot, prune, ids, d, cnt, xs, deferred, order,
+    scan<<<(unsigned)nq, kScanThreads, smem, st>>>(ix, probe, qsh, qrot, prune, ids, d, cnt, xs, deferred, order,
                                                       prep);
     check_launch("k_scan");
 }
@@ -3731,9 +3754,10 @@ int full_grid(const void *fn, int threads, size_t smem) {
 }
 
 // CTAs of the CTA scan that the GPU holds at once.
-int resident_scans(size_t smem) {
-    ensure_smem((const void *)k_scan, smem);
-    return full_grid((const void *)k_scan, kScanThreads, smem);
+int resident_scans(int S, size_t smem) {
+    const auto scan = scan_kernel(S);
+    ensure_smem((const void *)scan, smem);
+    return full_grid((const void *)scan, kScanThreads, smem);
 }
 
 // Prune bounds and rotated queries of a call on `st`.  k_qprep_few spreads over the
@@ -4062,7 +4086,7 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
             k_scan_warp<<<(unsigned)((nq + kWarpsPerCta - 1) / kWarpsPerCta), kWarpsPerCta * 32, wsm, st>>>(
                 ix, probe, (int)nprobe, (int)nq, qrot, prune, (int)topk, ids_out, d_out, cnt, per_warp);
             check_launch("k_scan_warp");
-        } else if (mode == 0 && no_deferral(I, nq, nprobe, !qsh.np, resident_scans(smem), tune)) {
+        } else if (mode == 0 && no_deferral(I, nq, nprobe, !qsh.np, resident_scans(ix.S, smem), tune)) {
             // no query of this call can probe more blocks than the deferral
             // threshold: the CTA scan answers every query, no split pass
             launch_cta_scan(scan_ws(tune), ix, probe, qsh, qrot, prune, ids_out, d_out, cnt, xs, nullptr, nq, order,
@@ -4115,7 +4139,7 @@ void run_search(const Index &I, const float *q, int64_t nq, int64_t topk, int64_
                 int defer = -1, resident = 0;  // mode 1: every query
                 if (mode == 0) {
                     defer = defer_threshold(tune);
-                    resident = defer_line_given(tune) ? 0 : resident_scans(smem);
+                    resident = defer_line_given(tune) ? 0 : resident_scans(ix.S, smem);
                 }
                 const int dthreads = (int)std::min<int64_t>(kDeferThreads, 32 * nq);  // a warp per query while they fit
                 const bool par = nq >= kQblocksMinQueries;
@@ -4451,11 +4475,12 @@ void run_search_static(const Index &I, const float *q, int64_t nq, int64_t topk,
     launch_qprep(ix, q, nq, m, qrot, prune, st);
     const size_t smem_k = scan_smem_bytes(ix.Dtot, ix.S, (int)topk, xstride_of(ix));
     SAQG_REQUIRE(smem_k <= kScanSmem, "dimension / topk too large for the scan kernel's shared memory");
-    ensure_smem((const void *)k_scan, (size_t)smem_k);
+    const auto scan = scan_kernel(ix.S);
+    ensure_smem((const void *)scan, smem_k);
     QueryShape qsh;
     qsh.np_max = (int)nprobe;
     qsh.k_max = (int)topk;
-    k_scan<<<(unsigned)nq, kScanThreads, smem_k, st>>>(ix, probe, qsh, qrot, prune, ids, dists, nullptr,
+    scan<<<(unsigned)nq, kScanThreads, smem_k, st>>>(ix, probe, qsh, qrot, prune, ids, dists, nullptr,
                                                       xstride_of(ix), nullptr, nullptr, Prepared{});
     check_launch("k_scan");
 }
